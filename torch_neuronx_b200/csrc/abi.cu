@@ -141,6 +141,16 @@ int choose(const B200SdpaParams* a, const Problem& p, int* path) {
   return B200_SDPA_OK;
 }
 
+// A request is on the generic path when it has not one of the tensor-core kernels' own shapes.  Within that path
+// the zero-filled tensor-core tiles serve what they can, unless the caller asked for the fp32 arithmetic of the
+// CUDA-core kernel (force_path).  Plans keep the name of the path; their geometry fields describe the kernel.
+bool served_padded(const B200SdpaParams* a, const Problem& p) {
+  return a->force_path != B200_SDPA_PATH_GENERIC && prefill_padded_eligible(p, a->dtype);
+}
+bool served_padded(const B200SdpaBwdParams* a, const BwdProblem& bp) {
+  return a->force_path != B200_SDPA_PATH_GENERIC && bwd_padded_eligible(bp, a->dtype);
+}
+
 // Makes the requested device current for the duration of one entry point and puts the caller's
 // device back afterwards (a library call must not change which device the host thread is on).
 // Also the one place that checks the compute capability: every kernel here is sm_100a code.
@@ -329,8 +339,14 @@ int b200_sdpa_query_plan(const B200SdpaParams* params, B200SdpaPlan* plan) {
   switch (path) {
     case B200_SDPA_PATH_DECODE: return plan_decode(p, params->dtype, params->kv_chunk, plan);
     case B200_SDPA_PATH_PREFILL: return plan_prefill(p, params->dtype, plan);
-    default: return plan_generic(p, params->dtype, plan);
+    default: break;
   }
+  if (served_padded(params, p)) {
+    rc = plan_prefill_padded(p, plan);
+    plan->path = B200_SDPA_PATH_GENERIC;
+    return rc;
+  }
+  return plan_generic(p, params->dtype, plan);
 }
 
 int b200_sdpa_fwd(const B200SdpaParams* params, void* stream) {
@@ -355,6 +371,7 @@ int b200_sdpa_fwd(const B200SdpaParams* params, void* stream) {
     path = prefill_eligible(p, params->dtype, &unused) ? B200_SDPA_PATH_PREFILL : B200_SDPA_PATH_GENERIC;
   }
   if (path == B200_SDPA_PATH_PREFILL) return launch_prefill(p, params->dtype, params->workspace, params->workspace_bytes, st);
+  if (served_padded(params, p)) return launch_prefill_padded(p, params->dtype, st);
   return launch_generic(p, params->dtype, st);
 }
 
@@ -388,7 +405,13 @@ int b200_sdpa_bwd_query_plan(const B200SdpaBwdParams* a, B200SdpaPlan* plan) {
   int path = 0;
   rc = choose_bwd(a, bp, &path);
   if (rc != B200_SDPA_OK) return rc;
-  return path == B200_SDPA_PATH_PREFILL ? plan_bwd_tc(bp, a->dtype, plan) : plan_bwd_generic(bp, a->dtype, plan);
+  if (path == B200_SDPA_PATH_PREFILL) return plan_bwd_tc(bp, a->dtype, plan);
+  if (served_padded(a, bp)) {
+    rc = plan_bwd_tc(bp, a->dtype, plan);
+    plan->path = B200_SDPA_PATH_GENERIC;
+    return rc;
+  }
+  return plan_bwd_generic(bp, a->dtype, plan);
 }
 
 int b200_sdpa_bwd(const B200SdpaBwdParams* a, void* stream) {
@@ -401,7 +424,7 @@ int b200_sdpa_bwd(const B200SdpaBwdParams* a, void* stream) {
   DeviceScope scope(a->device);
   if (scope.status() != B200_SDPA_OK) return scope.status();
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (path == B200_SDPA_PATH_PREFILL) {
+  if (path == B200_SDPA_PATH_PREFILL || served_padded(a, bp)) {
     rc = launch_bwd_tc(bp, a->dtype, a->workspace, a->workspace_bytes, st);
     // without scratch an automatic choice falls through to the kernels that need none
     if (rc != B200_SDPA_ERR_WORKSPACE || a->force_path == B200_SDPA_PATH_PREFILL) return rc;

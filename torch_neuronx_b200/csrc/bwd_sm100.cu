@@ -139,12 +139,16 @@ __device__ __forceinline__ uint64_t mnmajor_desc(uint32_t tile) { return smem_de
 __device__ __forceinline__ uint64_t mnmajor_step(int kk) { return static_cast<uint64_t>(kk * (2048 >> 4)); }
 
 // acc[tmem d, 128 x 64] = A[smem tile, K-major] * B[rows 64 hh .. 64 hh + 63 of a smem tile, K-major]^T over D
-template <int D>
-__device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint32_t a_tile, uint32_t b_tile, int hh, uint32_t idesc) {
+// (PAD: only the first `steps` of the D / 16 k-steps, the columns beyond hold zeros)
+template <int D, bool PAD>
+__device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint32_t a_tile, uint32_t b_tile, int hh, uint32_t idesc, int steps) {
   const uint64_t ad = kmajor_desc(a_tile), bd = kmajor_desc(b_tile + static_cast<uint32_t>(hh) * (kU * 128));
   if (elect_one()) {
 #pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk) mma_ss(d_tmem, ad + kmajor_step(kk), bd + kmajor_step(kk), idesc, kk > 0 ? 1u : 0u);
+    for (int kk = 0; kk < D / 16; ++kk) {
+      if (PAD && kk >= steps) break;
+      mma_ss(d_tmem, ad + kmajor_step(kk), bd + kmajor_step(kk), idesc, kk > 0 ? 1u : 0u);
+    }
   }
 }
 // acc[tmem d] (+)= A[tmem] * B[rows 64 hh .. 64 hh + 63 of a smem tile, MN-major].  The 16-bit A
@@ -253,7 +257,9 @@ __device__ __forceinline__ float bias_to_f32(const uint32_t bits16) {
 
 static_assert(sizeof(ASync) <= 272, "barrier block must fit its reserve (272 bytes + up to 1008 of alignment <= 1280)");
 
-template <int D, bool BF16, bool BIAS>
+// PAD: head dimensions E, Dv (multiples of 8) that do not fill the D = 128 tile; the tensor maps carry the real
+// extents (loads fill with zeros, stores clip) and the products skip the k-steps and output columns beyond them.
+template <int D, bool BF16, bool BIAS, bool PAD>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -382,7 +388,8 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     __syncwarp();
   } else if (warp == kMmaWarp) {
     constexpr uint32_t idesc_score = make_idesc(BF16, false, kT, kT);
-    constexpr uint32_t idesc_acc = make_idesc(BF16, true, kT, D);
+    const uint32_t idesc_acc = make_idesc(BF16, true, kT, PAD ? (p.E + 15) / 16 * 16 : D);
+    const int steps_e = PAD ? (p.E + 15) / 16 : D / 16, steps_v = PAD ? (p.Dv + 15) / 16 : D / 16;
     bool alive = n_tiles > 0;
     if (alive) {
       alive = wait_clocked(smem_u32(&sync->fixed_full), 0, abort_flag, wait_limit);
@@ -401,11 +408,15 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const uint64_t od = kmajor_desc(do_tile), vd = kmajor_desc(v_ring + vs * C::kTileBytes);
       if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
+        for (int kk = 0; kk < D / 16; ++kk) {
+          if (PAD && kk >= steps_e) break;
           mma_ss(tmem_base + kColS, qd + kmajor_step(kk), kd + kmajor_step(kk), idesc_score, kk > 0 ? 1u : 0u);
+        }
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk)
+        for (int kk = 0; kk < D / 16; ++kk) {
+          if (PAD && kk >= steps_v) break;
           mma_ss(tmem_base + kColDP, od + kmajor_step(kk), vd + kmajor_step(kk), idesc_score, kk > 0 ? 1u : 0u);
+        }
         mma_commit(smem_u32(&sync->sp_full));
         mma_commit(smem_u32(&sync->v_empty[vs]));   // V_j has no reader after dP_j
       }
@@ -560,7 +571,10 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       fence_proxy_async_smem();
       mbar_arrive(smem_u32(&sync->staged));
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {
-        for (int bx = 0; bx < C::kBoxes; ++bx) tma_store_4d(&tm_dq, q_tile + bx * kBoxBytes, bx * 64, row0, h, b);
+        for (int bx = 0; bx < C::kBoxes; ++bx) {
+          if (PAD && bx * 64 >= p.E) break;
+          tma_store_4d(&tm_dq, q_tile + bx * kBoxBytes, bx * 64, row0, h, b);
+        }
         tma_store_commit();
         tma_store_wait_read();
       }
@@ -582,7 +596,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
 // --------------------------------------------------------------- dK/dV kernel --
 
-template <int D, bool BF16, bool BIAS>
+template <int D, bool BF16, bool BIAS, bool PAD>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -713,7 +727,9 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     __syncwarp();
   } else if (warp == kMmaWarp) {
     constexpr uint32_t idesc_score = make_idesc(BF16, false, kT, kU);
-    constexpr uint32_t idesc_acc = make_idesc(BF16, true, kT, D);
+    const uint32_t idesc_dk = make_idesc(BF16, true, kT, PAD ? (p.E + 15) / 16 * 16 : D);
+    const uint32_t idesc_dv = make_idesc(BF16, true, kT, PAD ? (p.Dv + 15) / 16 * 16 : D);
+    const int steps_e = PAD ? (p.E + 15) / 16 : D / 16, steps_v = PAD ? (p.Dv + 15) / 16 : D / 16;
     bool alive = n_items > 0;
     if (alive) {
       alive = wait_clocked(smem_u32(&sync->fixed_full), 0, abort_flag, wait_limit);
@@ -732,8 +748,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         tc_fence_after_sync();
       }
       const uint32_t q_tile = ring + stage * 2 * C::kTileBytes, do_tile = q_tile + C::kTileBytes;
-      issue_ss<D>(tmem_base + kColS + buf * kU, k_tile, q_tile, hh, idesc_score);
-      issue_ss<D>(tmem_base + kColDP + buf * kU, v_tile, do_tile, hh, idesc_score);
+      issue_ss<D, PAD>(tmem_base + kColS + buf * kU, k_tile, q_tile, hh, idesc_score, steps_e);
+      issue_ss<D, PAD>(tmem_base + kColDP + buf * kU, v_tile, do_tile, hh, idesc_score, steps_v);
       if (elect_one()) mma_commit(smem_u32(&sync->sp_full[buf]));
       return true;
     };
@@ -749,8 +765,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
       tc_fence_after_sync();
       const uint32_t q_tile = ring + stage * 2 * C::kTileBytes, do_tile = q_tile + C::kTileBytes;
-      issue_ts(tmem_base + kColDV, tmem_base + kColS + buf * kU, do_tile, hh, idesc_acc, u > 0);   // dV += P^T_u dO_u
-      issue_ts(tmem_base + kColDK, tmem_base + kColDP + buf * kU, q_tile, hh, idesc_acc, u > 0);   // dK += dS^T_u Q_u
+      issue_ts(tmem_base + kColDV, tmem_base + kColS + buf * kU, do_tile, hh, idesc_dv, u > 0);   // dV += P^T_u dO_u
+      issue_ts(tmem_base + kColDK, tmem_base + kColDP + buf * kU, q_tile, hh, idesc_dk, u > 0);   // dK += dS^T_u Q_u
       if (elect_one()) {
         if (hh == 1) mma_commit(smem_u32(&sync->ring_empty[stage]));
         if (u + 1 == n_units) mma_commit(smem_u32(&sync->acc_done));
@@ -872,8 +888,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       mbar_arrive(smem_u32(&sync->staged));
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {
         for (int bx = 0; bx < C::kBoxes; ++bx) {
-          tma_store_4d(&tm_dk, ring + bx * kBoxBytes, bx * 64, j0, hk, b);
-          tma_store_4d(&tm_dv, ring + C::kTileBytes + bx * kBoxBytes, bx * 64, j0, hk, b);
+          if (!PAD || bx * 64 < p.E) tma_store_4d(&tm_dk, ring + bx * kBoxBytes, bx * 64, j0, hk, b);
+          if (!PAD || bx * 64 < p.Dv) tma_store_4d(&tm_dv, ring + C::kTileBytes + bx * kBoxBytes, bx * 64, j0, hk, b);
         }
         tma_store_commit();
         tma_store_wait_read();
@@ -893,19 +909,19 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
 int padded_rows(const Problem& p) { return (p.L + kT - 1) / kT * kT; }
 
-template <int D, bool BF16, bool BIAS>
+template <int D, bool BF16, bool BIAS, bool PAD = false>
 int launch_tc(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t stream) {
   using C = BCfg<D>;
   const Problem& p = bp.f;
   CUtensorMap tq, tk, tv, tdo, tdq, tdk, tdv;
-  if (!make_map(&tq, p.q, BF16, D, p.L, p.Hq, p.B, p.qs) || !make_map(&tk, p.k, BF16, D, p.S, p.Hkv, p.B, p.ks) ||
-      !make_map(&tv, p.v, BF16, D, p.S, p.Hkv, p.B, p.vs) || !make_map(&tdo, bp.dout, BF16, D, p.L, p.Hq, p.B, bp.dos) ||
-      !make_map(&tdq, bp.dq, BF16, D, p.L, p.Hq, p.B, bp.dqs) ||
-      !make_map(&tdk, bp.dk, BF16, D, p.S, p.Hkv, p.B, bp.dks) ||
-      !make_map(&tdv, bp.dv, BF16, D, p.S, p.Hkv, p.B, bp.dvs))
+  if (!make_map(&tq, p.q, BF16, p.E, p.L, p.Hq, p.B, p.qs) || !make_map(&tk, p.k, BF16, p.E, p.S, p.Hkv, p.B, p.ks) ||
+      !make_map(&tv, p.v, BF16, p.Dv, p.S, p.Hkv, p.B, p.vs) || !make_map(&tdo, bp.dout, BF16, p.Dv, p.L, p.Hq, p.B, bp.dos) ||
+      !make_map(&tdq, bp.dq, BF16, p.E, p.L, p.Hq, p.B, bp.dqs) ||
+      !make_map(&tdk, bp.dk, BF16, p.E, p.S, p.Hkv, p.B, bp.dks) ||
+      !make_map(&tdv, bp.dv, BF16, p.Dv, p.S, p.Hkv, p.B, bp.dvs))
     return B200_SDPA_ERR_CUDA;
-  auto kq = bwd_dq_tc_kernel<D, BF16, BIAS>;
-  auto kkv = bwd_dkv_tc_kernel<D, BF16, BIAS>;
+  auto kq = bwd_dq_tc_kernel<D, BF16, BIAS, PAD>;
+  auto kkv = bwd_dkv_tc_kernel<D, BF16, BIAS, PAD>;
   if (cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, ACfg<D>::kSmemBytes) != cudaSuccess ||
       cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) {
     cudaGetLastError();
@@ -939,8 +955,8 @@ int launch_tc(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t stre
   const long long limit = wait_limit_cycles();
   const long long n_streams = static_cast<long long>(p.Hkv) * p.B;
   // the dQ kernel streams keys and values; the dK/dV kernel the queries, dO and row statistics of a group
-  const int wave_q = kv_streams_per_wave(static_cast<long long>(p.S) * 2 * D * 2, n_streams);
-  const int wave_kv = kv_streams_per_wave(static_cast<long long>(p.L) * p.group * (2 * D * 2 + 8), n_streams);
+  const int wave_q = kv_streams_per_wave(static_cast<long long>(p.S) * (p.E + p.Dv) * 2, n_streams);
+  const int wave_kv = kv_streams_per_wave(static_cast<long long>(p.L) * p.group * ((p.E + p.Dv) * 2 + 8), n_streams);
   // The two kernels are independent of each other (both read the row statistics of the kernel before them).
   // The dK/dV kernel, whose CTAs are long, goes first and releases its dependents as soon as its last CTA is
   // resident; the dQ kernel is a programmatic dependent launch, so its CTAs take the SMs the first kernel's
@@ -973,11 +989,12 @@ int launch_tc(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t stre
 }  // namespace
 
 
-bool bwd_tc_eligible(const BwdProblem& bp, int dtype, bool* alignment_only_failure) {
+namespace {
+
+// What every head dimension needs.
+bool operands_eligible(const BwdProblem& bp, int dtype, bool* alignment_only_failure) {
   const Problem& p = bp.f;
-  if (alignment_only_failure) *alignment_only_failure = false;
   if (dtype != B200_SDPA_F16 && dtype != B200_SDPA_BF16) return false;
-  if (p.E != p.Dv || (p.E != 64 && p.E != 128)) return false;
   if (bp.dbias != nullptr) return false;   // the logit gradient is written by the CUDA-core kernels only
   if (!(p.scale > 0.f) || !(p.scale < 1e30f)) return false;
   if (p.L < 1 || p.S < 1) return false;
@@ -990,6 +1007,26 @@ bool bwd_tc_eligible(const BwdProblem& bp, int dtype, bool* alignment_only_failu
                   strides_ok(bp.dv, bp.dvs, p.S, p.Hkv, p.B);
   if (!ok && alignment_only_failure) *alignment_only_failure = true;
   return ok;
+}
+
+}  // namespace
+
+bool bwd_tc_eligible(const BwdProblem& bp, int dtype, bool* alignment_only_failure) {
+  const Problem& p = bp.f;
+  if (alignment_only_failure) *alignment_only_failure = false;
+  if (p.E != p.Dv || (p.E != 64 && p.E != 128)) return false;
+  return operands_eligible(bp, dtype, alignment_only_failure);
+}
+
+// Head dimensions between 64 and 128 (multiples of 8) on zero-filled 128-wide tiles, as in the forward.  Fewer
+// than 64 rows or keys leave more than half of every tile empty and the CUDA-core kernels, one launch fewer, are
+// not slower there.
+bool bwd_padded_eligible(const BwdProblem& bp, int dtype) {
+  const Problem& p = bp.f;
+  if (p.L < 64 || p.S < 64) return false;
+  const int hi = p.E > p.Dv ? p.E : p.Dv;
+  if (hi <= 64 || hi > 128 || p.E % 8 != 0 || p.Dv % 8 != 0 || (p.E == 128 && p.Dv == 128)) return false;
+  return operands_eligible(bp, dtype, nullptr);
 }
 
 uint64_t bwd_tc_workspace_bytes(const BwdProblem& bp) {
@@ -1006,7 +1043,7 @@ int plan_bwd_tc(const BwdProblem& bp, int dtype, B200SdpaPlan* plan) {
   plan->grid_y = static_cast<int32_t>(static_cast<long long>((p.S + kT - 1) / kT) * p.Hkv * p.B);
   plan->grid_z = 1;
   plan->threads = kThreads;
-  plan->smem_bytes = p.E == 128 ? BCfg<128>::kSmemBytes : BCfg<64>::kSmemBytes;
+  plan->smem_bytes = p.E == 64 && p.Dv == 64 ? BCfg<64>::kSmemBytes : BCfg<128>::kSmemBytes;
   plan->kv_splits = 1;
   plan->launches = 3;
   plan->workspace_bytes = bwd_tc_workspace_bytes(bp);
@@ -1014,13 +1051,19 @@ int plan_bwd_tc(const BwdProblem& bp, int dtype, B200SdpaPlan* plan) {
 }
 
 int launch_bwd_tc(const BwdProblem& bp, int dtype, void* workspace, uint64_t workspace_bytes, cudaStream_t stream) {
-  if (!bwd_tc_eligible(bp, dtype, nullptr)) return B200_SDPA_ERR_UNSUPPORTED;
+  const bool padded = bwd_padded_eligible(bp, dtype);
+  if (!padded && !bwd_tc_eligible(bp, dtype, nullptr)) return B200_SDPA_ERR_UNSUPPORTED;
   const uint64_t need = bwd_tc_workspace_bytes(bp);
   if (workspace == nullptr || workspace_bytes < need || reinterpret_cast<uintptr_t>(workspace) % 16)
     return B200_SDPA_ERR_WORKSPACE;
   float* lse2 = reinterpret_cast<float*>(workspace);
   float* delta = lse2 + need / (2 * sizeof(float));
   const bool bf16 = dtype == B200_SDPA_BF16;
+  if (padded) {
+    if (bp.f.bias != nullptr)
+      return bf16 ? launch_tc<128, true, true, true>(bp, lse2, delta, stream) : launch_tc<128, false, true, true>(bp, lse2, delta, stream);
+    return bf16 ? launch_tc<128, true, false, true>(bp, lse2, delta, stream) : launch_tc<128, false, false, true>(bp, lse2, delta, stream);
+  }
   if (bp.f.bias != nullptr) {
     if (bp.f.E == 128)
       return bf16 ? launch_tc<128, true, true>(bp, lse2, delta, stream) : launch_tc<128, false, true>(bp, lse2, delta, stream);

@@ -103,6 +103,10 @@ int launch_decode_static(const Problem& p, int dtype, int kv_chunk, cudaStream_t
 int launch_prefill(const Problem& p, int dtype, void* workspace, uint64_t workspace_bytes, cudaStream_t stream);
 int plan_prefill(const Problem& p, int dtype, B200SdpaPlan* plan);
 bool prefill_eligible(const Problem& p, int dtype, bool* alignment_only_failure);
+// head dimensions between 64 and 128 on zero-filled 128-wide tiles
+bool prefill_padded_eligible(const Problem& p, int dtype);
+int plan_prefill_padded(const Problem& p, B200SdpaPlan* plan);
+int launch_prefill_padded(const Problem& p, int dtype, cudaStream_t stream);
 // persistent form of the prefill kernel (prefill_persistent_sm100.cu): head dimension 128, large problems
 bool prefill_persistent_wanted(const Problem& p);
 bool prefill_accumulate_eligible(const Problem& p);   // accumulating form: layout rules of (acc, acc_lse)
@@ -118,6 +122,7 @@ int launch_merge(const B200SdpaMergeParams& m, cudaStream_t stream);
 int launch_bwd_generic(const BwdProblem& bp, int dtype, cudaStream_t stream);
 int plan_bwd_generic(const BwdProblem& bp, int dtype, B200SdpaPlan* plan);
 bool bwd_tc_eligible(const BwdProblem& bp, int dtype, bool* alignment_only_failure);
+bool bwd_padded_eligible(const BwdProblem& bp, int dtype);
 uint64_t bwd_tc_workspace_bytes(const BwdProblem& bp);
 int plan_bwd_tc(const BwdProblem& bp, int dtype, B200SdpaPlan* plan);
 int launch_bwd_tc(const BwdProblem& bp, int dtype, void* workspace, uint64_t workspace_bytes, cudaStream_t stream);

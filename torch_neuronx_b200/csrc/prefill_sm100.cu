@@ -107,7 +107,10 @@ __device__ __forceinline__ TileGeom tile_geometry(const Problem& p, int row0, in
   return g;
 }
 
-template <int D, bool BF16, bool BIAS, bool ACC>
+// PAD: head dimensions E, Dv (multiples of 8) that do not fill the D = 128 tile.  The tensor maps carry the
+// real extents, so the copies fill the tile's remaining columns with zeros and the output store clips them;
+// the products run over ceil(E / 16) k-steps and ceil(Dv / 16) * 16 output columns only.
+template <int D, bool BF16, bool BIAS, bool ACC, bool PAD>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const Problem p,
@@ -247,7 +250,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // index is a compile-time constant everywhere for the same reason.
     {
       constexpr uint32_t idesc_qk = make_idesc(BF16, false, kBlockM, kBlockN);
-      constexpr uint32_t idesc_pv = make_idesc(BF16, true, kBlockM, D);
+      const uint32_t idesc_pv = make_idesc(BF16, true, kBlockM, PAD ? (p.Dv + 15) / 16 * 16 : D);
+      const int qk_steps = PAD ? (p.E + 15) / 16 : D / 16;
       bool alive = n_iter > 0;
 
       // descriptors: fixed fields once, then only the 16-byte-unit start address moves
@@ -262,6 +266,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (elect_one() && dbg_tmem(p.status, DBG_PREFILL * 100 + 1, d_addr, tmem_base, 128, 512)) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
+            if (PAD && kk >= qk_steps) break;
             const uint64_t off = static_cast<uint64_t>(((kk >> 2) * kBoxBytes + (kk & 3) * 32) >> 4);
             mma_ss(d_addr, qd + off, kd + off, idesc_qk, kk > 0 ? 1u : 0u);
           }
@@ -641,7 +646,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         fence_proxy_async_smem();
         mbar_arrive(smem_u32(&sync->o_staged[t]));
         if (r == 0 && wait_clocked(smem_u32(&sync->o_staged[t]), 0, abort_flag, wait_limit)) {
-          for (int bx = 0; bx < C::kBoxes; ++bx) tma_store_4d(&tm_o, q_smem[t] + bx * kBoxBytes, bx * 64, tg.row0, head_of_tile[t], b);
+          for (int bx = 0; bx < C::kBoxes; ++bx) {
+            if (PAD && bx * 64 >= p.Dv) break;
+            tma_store_4d(&tm_o, q_smem[t] + bx * kBoxBytes, bx * 64, tg.row0, head_of_tile[t], b);
+          }
           tma_store_commit();
           tma_store_wait_read();
         }
@@ -687,19 +695,19 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
 // mask is causal (that is where the row-block layout leaves one tile idle at the end).
 int pair_heads_mode(const Problem& p) { return (p.causal && p.group % 2 == 0) ? 1 : 0; }
 
-template <int D, bool BF16, bool BIAS, bool ACC = false>
+template <int D, bool BF16, bool BIAS, bool ACC = false, bool PAD = false>
 int launch_variant(const Problem& p, cudaStream_t stream) {
   using C = Cfg<D>;
   CUtensorMap tq, tk, tv, to;
-  if (!make_map(&tq, p.q, BF16, D, p.L, p.Hq, p.B, p.qs) || !make_map(&tk, p.k, BF16, D, p.S, p.Hkv, p.B, p.ks) ||
-      !make_map(&tv, p.v, BF16, D, p.S, p.Hkv, p.B, p.vs))
+  if (!make_map(&tq, p.q, BF16, p.E, p.L, p.Hq, p.B, p.qs) || !make_map(&tk, p.k, BF16, p.E, p.S, p.Hkv, p.B, p.ks) ||
+      !make_map(&tv, p.v, BF16, p.Dv, p.S, p.Hkv, p.B, p.vs))
     return B200_SDPA_ERR_CUDA;
   if (ACC) {
     to = tq;   // the accumulating form stores through plain pointers; the map is never used
-  } else if (!make_map(&to, p.out, BF16, D, p.L, p.Hq, p.B, p.os)) {
+  } else if (!make_map(&to, p.out, BF16, p.Dv, p.L, p.Hq, p.B, p.os)) {
     return B200_SDPA_ERR_CUDA;
   }
-  auto kern = prefill_kernel<D, BF16, BIAS, ACC>;
+  auto kern = prefill_kernel<D, BF16, BIAS, ACC, PAD>;
   // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute: set on every
   // launch (a cheap host-side call), so a process that drives several GPUs gets it on each of them
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) {
@@ -711,7 +719,7 @@ int launch_variant(const Problem& p, cudaStream_t stream) {
   const int n_qblk = (p.L + rows - 1) / rows;
   const long long grid = static_cast<long long>(n_qblk) * (p.Hq / (pair_heads ? 2 : 1)) * p.B;
   if (grid <= 0 || grid > 0x7fffffffLL) return B200_SDPA_ERR_UNSUPPORTED;
-  const int per_wave = kv_streams_per_wave(static_cast<long long>(p.S) * 2 * D * 2, static_cast<long long>(p.Hkv) * p.B);
+  const int per_wave = kv_streams_per_wave(static_cast<long long>(p.S) * (p.E + p.Dv) * 2, static_cast<long long>(p.Hkv) * p.B);
   kern<<<static_cast<unsigned>(grid), kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, to, p, n_qblk, pair_heads,
                                                                          per_wave, wait_limit_cycles());
   if (cudaGetLastError() != cudaSuccess) return B200_SDPA_ERR_CUDA;
@@ -721,11 +729,11 @@ int launch_variant(const Problem& p, cudaStream_t stream) {
 
 }  // namespace
 
-bool prefill_eligible(const Problem& p, int dtype, bool* alignment_only_failure) {
-  if (p.E > 128) return prefill_wide_eligible(p, dtype, alignment_only_failure);
-  if (alignment_only_failure) *alignment_only_failure = false;
+namespace {
+
+// What every head dimension needs: 16-bit types, a positive finite scale, TMA-legal bases and strides.
+bool operands_eligible(const Problem& p, int dtype, bool* alignment_only_failure) {
   if (dtype != B200_SDPA_F16 && dtype != B200_SDPA_BF16) return false;
-  if (p.E != p.Dv || (p.E != 64 && p.E != 128)) return false;
   if (!(p.scale > 0.f) || !(p.scale < 1e30f)) return false;
   if (p.L < 1 || p.S < 1) return false;
   if (p.bias != nullptr) {
@@ -735,6 +743,40 @@ bool prefill_eligible(const Problem& p, int dtype, bool* alignment_only_failure)
                   strides_ok(p.v, p.vs, p.S, p.Hkv, p.B) && strides_ok(p.out, p.os, p.L, p.Hq, p.B);
   if (!ok && alignment_only_failure) *alignment_only_failure = true;
   return ok;
+}
+
+void plan_per_cta(const Problem& p, long long grid, int rows, B200SdpaPlan* plan) {
+  plan->path = B200_SDPA_PATH_PREFILL;
+  plan->block_m = rows;
+  plan->block_n = kBlockN;
+  plan->grid_x = static_cast<int32_t>(grid);
+  plan->grid_y = plan->grid_z = 1;
+  plan->threads = kThreads;
+  plan->smem_bytes = p.E == 64 && p.Dv == 64 ? Cfg<64>::kSmemBytes : Cfg<128>::kSmemBytes;
+  plan->kv_splits = 1;
+  plan->launches = 1;
+  plan->workspace_bytes = 0;
+}
+
+}  // namespace
+
+bool prefill_eligible(const Problem& p, int dtype, bool* alignment_only_failure) {
+  if (p.E > 128) return prefill_wide_eligible(p, dtype, alignment_only_failure);
+  if (alignment_only_failure) *alignment_only_failure = false;
+  if (p.E != p.Dv || (p.E != 64 && p.E != 128)) return false;
+  return operands_eligible(p, dtype, alignment_only_failure);
+}
+
+// Head dimensions between 64 and 128 (multiples of 8, so that rows stay on the 16-byte grid of a tensor copy):
+// 128-wide tiles with zero-filled columns.  Below 64 the exponentials bound a tile whatever its head dimension
+// and the requests are small; those keep the CUDA-core kernel.  Measured (fp16, 16 x 16 heads x 577 x 577, head
+// dimension 80): CUDA-core kernel 2463 us, these tiles 86 us.
+bool prefill_padded_eligible(const Problem& p, int dtype) {
+  const int hi = p.E > p.Dv ? p.E : p.Dv;
+  if (hi <= 64 || hi > 128 || p.E % 8 != 0 || p.Dv % 8 != 0) return false;
+  if (p.E == p.Dv && p.E == 128) return false;
+  if (p.block_table != nullptr || p.k_new != nullptr || p.acc_mode != 0) return false;
+  return operands_eligible(p, dtype, nullptr);
 }
 
 int plan_prefill(const Problem& p, int dtype, B200SdpaPlan* plan) {
@@ -749,17 +791,27 @@ int plan_prefill(const Problem& p, int dtype, B200SdpaPlan* plan) {
   const int n_qblk = (p.L + rows - 1) / rows;
   const long long grid = static_cast<long long>(n_qblk) * (p.Hq / (pair_heads ? 2 : 1)) * p.B;
   if (grid > 0x7fffffffLL) return B200_SDPA_ERR_UNSUPPORTED;
-  plan->path = B200_SDPA_PATH_PREFILL;
-  plan->block_m = rows;
-  plan->block_n = kBlockN;
-  plan->grid_x = static_cast<int32_t>(grid);
-  plan->grid_y = plan->grid_z = 1;
-  plan->threads = kThreads;
-  plan->smem_bytes = p.E == 128 ? Cfg<128>::kSmemBytes : Cfg<64>::kSmemBytes;
-  plan->kv_splits = 1;
-  plan->launches = 1;
-  plan->workspace_bytes = 0;
+  plan_per_cta(p, grid, rows, plan);
   return B200_SDPA_OK;
+}
+
+int plan_prefill_padded(const Problem& p, B200SdpaPlan* plan) {
+  const int pair_heads = pair_heads_mode(p);
+  const int rows = pair_heads ? kBlockM : kRowsPerCta;
+  const long long grid = static_cast<long long>((p.L + rows - 1) / rows) * (p.Hq / (pair_heads ? 2 : 1)) * p.B;
+  if (grid > 0x7fffffffLL) return B200_SDPA_ERR_UNSUPPORTED;
+  plan_per_cta(p, grid, rows, plan);
+  return B200_SDPA_OK;
+}
+
+// The caller has checked prefill_padded_eligible().
+int launch_prefill_padded(const Problem& p, int dtype, cudaStream_t stream) {
+  const bool bf16 = dtype == B200_SDPA_BF16;
+  if (p.bias != nullptr)
+    return bf16 ? launch_variant<128, true, true, false, true>(p, stream)
+                : launch_variant<128, false, true, false, true>(p, stream);
+  return bf16 ? launch_variant<128, true, false, false, true>(p, stream)
+              : launch_variant<128, false, false, false, true>(p, stream);
 }
 
 int launch_prefill(const Problem& p, int dtype, void* workspace, uint64_t workspace_bytes, cudaStream_t stream) {
