@@ -32,8 +32,7 @@
 // Its tensor memory is full with that; the dQ kernel has one accumulator less and works on
 // whole 128-column tiles instead (layout and pipeline described at the kernel).
 // Every wait is bounded (see tc_common.cuh).
-#include "tc_common.cuh"
-#include "debug.cuh"
+#include "bwd_common.cuh"
 
 namespace b200 {
 
@@ -42,7 +41,6 @@ namespace {
 using namespace ptx;
 using namespace tc;
 
-constexpr int kT = 128;                 // tile edge: query rows, keys, TMEM lanes
 constexpr int kThreads = 320;
 constexpr int kEThreads = 256;            // elementwise role: two column halves x 128 lanes
 constexpr int kU = 64;                    // score columns per unit
@@ -126,18 +124,6 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const BwdProblem bp, floa
   }
 }
 
-// --------------------------------------------------------------- shared bits --
-
-// K-major operand descriptor of a 128-row tile; k-step kk covers 16 elements of D.
-__device__ __forceinline__ uint64_t kmajor_desc(uint32_t tile) { return smem_desc_sw128(tile, 16, 1024); }
-__device__ __forceinline__ uint64_t kmajor_step(int kk) {
-  return static_cast<uint64_t>(((kk >> 2) * kBoxBytes + (kk & 3) * 32) >> 4);
-}
-// MN-major B operand descriptor of the same tile (rows are the contraction axis);
-// k-step kk covers 16 rows.
-__device__ __forceinline__ uint64_t mnmajor_desc(uint32_t tile) { return smem_desc_sw128(tile, kBoxBytes, 1024); }
-__device__ __forceinline__ uint64_t mnmajor_step(int kk) { return static_cast<uint64_t>(kk * (2048 >> 4)); }
-
 // acc[tmem d, 128 x 64] = A[smem tile, K-major] * B[rows 64 hh .. 64 hh + 63 of a smem tile, K-major]^T over D
 // (PAD: only the first `steps` of the D / 16 k-steps, the columns beyond hold zeros)
 template <int D, bool PAD>
@@ -162,36 +148,6 @@ __device__ __forceinline__ void issue_ts(uint32_t d_tmem, uint32_t a_tmem, uint3
     for (int kk = 0; kk < kU / 16; ++kk)
       mma_ts(d_tmem, a_tmem + static_cast<uint32_t>((kk >> 1) * 32 + (kk & 1) * 8), bd + mnmajor_step(kk), idesc,
              (kk > 0 || accumulate) ? 1u : 0u);
-  }
-}
-
-// One thread's accumulator row (TMEM lane) -> 16-bit -> the 128-byte-swizzled staging
-// tile a TMA store expects.
-template <int D, bool BF16>
-__device__ __forceinline__ void stage_row(uint32_t acc_addr, bool have_acc, float mul, uint8_t* stage, int r,
-                                          int half) {
-  // the two threads of a lane share the row: D/64 chunks of 32 columns each
-#pragma unroll
-  for (int cc = 0; cc < D / 64; ++cc) {
-    const int c = half * (D / 64) + cc;
-    uint32_t v[32];
-    if (have_acc) {
-      tmem_ld_32x32(acc_addr + c * 32, v);
-      tmem_ld_wait();
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = 0u;
-    }
-    uint32_t pk[16];
-#pragma unroll
-    for (int i = 0; i < 32; i += 2)
-      pk[i >> 1] = pack2<BF16>(__uint_as_float(v[i]) * mul, __uint_as_float(v[i + 1]) * mul);
-    uint8_t* box = stage + (c >> 1) * kBoxBytes + r * 128;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int unit = ((c & 1) * 4 + u) ^ (r & 7);
-      *reinterpret_cast<uint4*>(box + unit * 16) = make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
-    }
   }
 }
 
@@ -907,7 +863,33 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
 // ------------------------------------------------------------------ host side --
 
-int padded_rows(const Problem& p) { return (p.L + kT - 1) / kT * kT; }
+}  // namespace
+
+int launch_bwd_prep(const BwdProblem& bp, bool bf16, float* lse2, float* delta, cudaStream_t stream) {
+  const Problem& p = bp.f;
+  const int l_pad = padded_rows(p);
+  const long long rows = static_cast<long long>(p.B) * p.Hq * l_pad;
+  auto rows_aligned = [](const void* base, const int64_t* st) {
+    return st[3] == 1 && reinterpret_cast<uintptr_t>(base) % 16 == 0 && st[0] % 8 == 0 && st[1] % 8 == 0 && st[2] % 8 == 0;
+  };
+  const bool vec = p.Dv % 8 == 0 && rows_aligned(bp.dout, bp.dos) && rows_aligned(p.out, p.os);
+  const long long warps = vec ? (rows + 3) / 4 : rows;
+  const long long blocks = (warps * 32 + 255) / 256;
+  if (blocks > 0x7fffffffLL) return B200_SDPA_ERR_UNSUPPORTED;
+  const unsigned grid = static_cast<unsigned>(blocks);
+  if (bf16) {
+    if (vec) bwd_prep_kernel<__nv_bfloat16, true><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
+    else bwd_prep_kernel<__nv_bfloat16, false><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
+  } else {
+    if (vec) bwd_prep_kernel<__half, true><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
+    else bwd_prep_kernel<__half, false><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
+  }
+  if (cudaGetLastError() != cudaSuccess) return B200_SDPA_ERR_CUDA;
+  count_launch(KID_BWD_PREP);
+  return B200_SDPA_OK;
+}
+
+namespace {
 
 template <int D, bool BF16, bool BIAS, bool PAD = false>
 int launch_tc(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t stream) {
@@ -928,26 +910,8 @@ int launch_tc(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t stre
     return B200_SDPA_ERR_CUDA;
   }
   const int l_pad = padded_rows(p);
-  {
-    const long long rows = static_cast<long long>(p.B) * p.Hq * l_pad;
-    auto rows_aligned = [](const void* base, const int64_t* st) {
-      return st[3] == 1 && reinterpret_cast<uintptr_t>(base) % 16 == 0 && st[0] % 8 == 0 && st[1] % 8 == 0 && st[2] % 8 == 0;
-    };
-    const bool vec = p.Dv % 8 == 0 && rows_aligned(bp.dout, bp.dos) && rows_aligned(p.out, p.os);
-    const long long warps = vec ? (rows + 3) / 4 : rows;
-    const long long blocks = (warps * 32 + 255) / 256;
-    if (blocks > 0x7fffffffLL) return B200_SDPA_ERR_UNSUPPORTED;
-    const unsigned grid = static_cast<unsigned>(blocks);
-    if (BF16) {
-      if (vec) bwd_prep_kernel<__nv_bfloat16, true><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
-      else bwd_prep_kernel<__nv_bfloat16, false><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
-    } else {
-      if (vec) bwd_prep_kernel<__half, true><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
-      else bwd_prep_kernel<__half, false><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
-    }
-    if (cudaGetLastError() != cudaSuccess) return B200_SDPA_ERR_CUDA;
-    count_launch(KID_BWD_PREP);
-  }
+  const int prep = launch_bwd_prep(bp, BF16, lse2, delta, stream);
+  if (prep != B200_SDPA_OK) return prep;
   const int n_qblk = (p.L + kT - 1) / kT, n_kblk = (p.S + kT - 1) / kT;
   const long long grid_q = static_cast<long long>(n_qblk) * p.Hq * p.B;
   const long long grid_kv = static_cast<long long>(n_kblk) * p.Hkv * p.B;
@@ -1014,7 +978,7 @@ bool operands_eligible(const BwdProblem& bp, int dtype, bool* alignment_only_fai
 bool bwd_tc_eligible(const BwdProblem& bp, int dtype, bool* alignment_only_failure) {
   const Problem& p = bp.f;
   if (alignment_only_failure) *alignment_only_failure = false;
-  if (p.E != p.Dv || (p.E != 64 && p.E != 128)) return false;
+  if (!bwd_wide_dims(p) && (p.E != p.Dv || (p.E != 64 && p.E != 128))) return false;
   return operands_eligible(bp, dtype, alignment_only_failure);
 }
 
@@ -1059,6 +1023,7 @@ int launch_bwd_tc(const BwdProblem& bp, int dtype, void* workspace, uint64_t wor
   float* lse2 = reinterpret_cast<float*>(workspace);
   float* delta = lse2 + need / (2 * sizeof(float));
   const bool bf16 = dtype == B200_SDPA_BF16;
+  if (bwd_wide_dims(bp.f)) return launch_bwd_wide(bp, bf16, lse2, delta, stream);
   if (padded) {
     if (bp.f.bias != nullptr)
       return bf16 ? launch_tc<128, true, true, true>(bp, lse2, delta, stream) : launch_tc<128, false, true, true>(bp, lse2, delta, stream);

@@ -122,6 +122,9 @@ int launch_merge(const B200SdpaMergeParams& m, cudaStream_t stream);
 int launch_bwd_generic(const BwdProblem& bp, int dtype, cudaStream_t stream);
 int plan_bwd_generic(const BwdProblem& bp, int dtype, B200SdpaPlan* plan);
 bool bwd_tc_eligible(const BwdProblem& bp, int dtype, bool* alignment_only_failure);
+// head dimensions 192/128 and 256 (bwd_wide_sm100.cu)
+bool bwd_wide_dims(const Problem& p);
+int launch_bwd_wide(const BwdProblem& bp, bool bf16, float* lse2, float* delta, cudaStream_t stream);
 bool bwd_padded_eligible(const BwdProblem& bp, int dtype);
 uint64_t bwd_tc_workspace_bytes(const BwdProblem& bp);
 int plan_bwd_tc(const BwdProblem& bp, int dtype, B200SdpaPlan* plan);

@@ -28,7 +28,8 @@ enum DebugFile {
   DBG_PREFILL = 5,
   DBG_PREFILL_PERSISTENT = 6,
   DBG_PREFILL_WIDE = 7,
-  DBG_BWD_TC = 8
+  DBG_BWD_TC = 8,
+  DBG_BWD_WIDE = 9
 };
 
 __device__ __forceinline__ bool dbg_fail(int* status, int site, long long index, long long limit) {
