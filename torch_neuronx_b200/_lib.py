@@ -19,9 +19,10 @@ import threading
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libb200_sdpa.so")
 OPS_LIB_PATH = os.path.join(HERE, "libb200_sdpa_ops.so")   # C++ operator layer (dispatcher kernels of the ATen ops)
+NATIVE_PATH = os.path.join(HERE, "_native.so")             # direct Python entry points over both
 # B200_SDPA_CHECKED=1 runs everything on the bounds-checking build of the library (csrc/debug.cuh;
 # `python -m torch_neuronx_b200.build --checked`); the C++ operator layer is linked against the normal library, so
-# the ATen ops then go through the Python implementations and the same checked kernels.
+# the ATen ops then go through the Python implementations and the same checked kernels (no direct entry points).
 CHECKED = os.environ.get("B200_SDPA_CHECKED", "0") not in ("", "0")
 if CHECKED:
     LIB_PATH = os.path.join(HERE, "libb200_sdpa_checked.so")
@@ -248,6 +249,7 @@ def load():
 
 
 _ops_loaded = None
+native = None   # the extension module with the direct entry points (csrc_ops/py_calls.cpp), once loaded
 
 
 def load_ops() -> bool:
@@ -255,7 +257,7 @@ def load_ops() -> bool:
     ATen ops with the dispatcher, as upstream's native dispatcher does
     (``torch_neuronx/csrc/core/dispatch/NeuronDispatcher.cpp:2370-2582``).  Returns False when the
     library has not been built; the same kernels are then reached through the ctypes binding."""
-    global _ops_loaded
+    global _ops_loaded, native
     if _ops_loaded is not None:
         return _ops_loaded
     with _lock:
@@ -268,7 +270,11 @@ def load_ops() -> bool:
                     C.CDLL(LIB_PATH, mode=C.RTLD_GLOBAL)   # the layer links against it by name
                     torch.ops.load_library(OPS_LIB_PATH)
                     _ops_loaded = True
-                except OSError as exc:
+                    if os.path.exists(NATIVE_PATH):
+                        from . import _native as module
+
+                        native = module
+                except (OSError, ImportError) as exc:
                     # a library from an interrupted or outdated build: importing the package must still work
                     # (the build itself runs as a module of it); any compute call will report the real problem
                     import warnings

@@ -27,6 +27,10 @@ OBJ_DIR = os.path.join(CSRC, "build")
 LIB_PATH = os.path.join(HERE, "libb200_sdpa.so")
 OPS_SRC = os.path.join(HERE, "csrc_ops", "aten_ops.cpp")
 OPS_LIB_PATH = os.path.join(HERE, "libb200_sdpa_ops.so")
+OPS_HEADER = os.path.join(HERE, "csrc_ops", "ops_common.h")
+# the direct Python entry points (an extension module over the two libraries)
+NATIVE_SRC = os.path.join(HERE, "csrc_ops", "py_calls.cpp")
+NATIVE_PATH = os.path.join(HERE, "_native.so")
 # the checked build: the same sources with -DB200_SDPA_DEBUG (index, scratch-slot and tensor-memory column
 # checks that report through the status word; csrc/debug.cuh)
 CHECKED_OBJ_DIR = os.path.join(CSRC, "build_checked")
@@ -121,7 +125,10 @@ def _build(verbose: bool, force: bool, OBJ_DIR: str, LIB_PATH: str, extra_flags,
 
 
 def build_ops(stamps: dict, force: bool = False, verbose: bool = False) -> str:
-    """Build (if needed) the C++ operator layer against the installed torch; returns its path."""
+    """Build (if needed) the C++ operator layer and the extension module over it against the installed torch;
+    returns the layer's path."""
+    import sysconfig
+
     import torch
     from torch.utils import cpp_extension
 
@@ -134,17 +141,22 @@ def build_ops(stamps: dict, force: bool = False, verbose: bool = False) -> str:
              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     for inc in cpp_extension.include_paths() + [os.path.join(cuda_home, "include")]:
         flags += ["-isystem", inc]
-    key = _digest([OPS_SRC, os.path.join(HERE, "..", "include", "b200_sdpa.h")], " ".join(flags) + torch.__version__)
-    if not force and stamps.get("aten_ops.cpp") == key and os.path.exists(OPS_LIB_PATH):
-        return OPS_LIB_PATH
-    cmd = [gxx] + flags + [OPS_SRC, "-o", OPS_LIB_PATH, f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
-                           f"-L{HERE}", "-lb200_sdpa", "-Wl,-rpath,$ORIGIN"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        raise RuntimeError(f"g++ failed for aten_ops.cpp:\n{res.stdout}\n{res.stderr}")
-    if verbose:
-        sys.stderr.write(f"--- aten_ops.cpp\n{res.stderr}\n")
-    stamps["aten_ops.cpp"] = key
+    headers = [OPS_HEADER, os.path.join(HERE, "..", "include", "b200_sdpa.h")]
+    libs = [f"-L{torch_lib}", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-L{HERE}", "-lb200_sdpa", "-Wl,-rpath,$ORIGIN"]
+    for src, path, more in (
+        (OPS_SRC, OPS_LIB_PATH, []),
+        (NATIVE_SRC, NATIVE_PATH, ["-isystem", sysconfig.get_paths()["include"], "-l:libb200_sdpa_ops.so", "-ltorch_python"]),
+    ):
+        name = os.path.basename(src)
+        key = _digest([src] + headers, " ".join(flags + more) + torch.__version__)
+        if not force and stamps.get(name) == key and os.path.exists(path):
+            continue
+        res = subprocess.run([gxx] + flags + [src, "-o", path] + libs + more, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"g++ failed for {name}:\n{res.stdout}\n{res.stderr}")
+        if verbose:
+            sys.stderr.write(f"--- {name}\n{res.stderr}\n")
+        stamps[name] = key
     return OPS_LIB_PATH
 
 

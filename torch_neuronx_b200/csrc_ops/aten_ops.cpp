@@ -10,7 +10,6 @@
 // query's layout through the caching allocator (:2352, python_ops/scaled_dot_product_fused_attention.py:
 // 357-358), fills the C-ABI parameter block and launches on the current stream.  There is no fallback:
 // non-CUDA tensors are rejected and every launch goes through libb200_sdpa.so.
-#include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/library.h>
@@ -24,20 +23,18 @@
 #include <tuple>
 #include <vector>
 
-#include "../../include/b200_sdpa.h"
+#include "ops_common.h"
+
+namespace b200_ops {
 
 namespace {
 
 constexpr int kMaxDevices = 64;
 
-struct PerDevice {
-  at::Tensor status;        // int32[4]: first device-side error seen by a kernel
-  at::Tensor philox_seed;   // int32 scalar zeros (dropout is off)
-  at::Tensor philox_offset;
-};
-
 std::once_flag g_once[kMaxDevices];
 PerDevice g_dev[kMaxDevices];
+
+}  // namespace
 
 // Created once per device, by whichever thread gets there first (calls arrive without the interpreter
 // lock, so several threads may race here).
@@ -53,21 +50,21 @@ PerDevice& device_state(int dev) {
   return d;
 }
 
-int dtype_code(at::ScalarType t) {
-  switch (t) {
-    case at::kFloat: return B200_SDPA_F32;
-    case at::kHalf: return B200_SDPA_F16;
-    case at::kBFloat16: return B200_SDPA_BF16;
-    default: return -1;
-  }
+// Output buffer laid out like the query: identical strides when the shapes agree, otherwise dense strides
+// in the query's dimension order (the rule of torch's own meta kernel for this op).
+at::Tensor alloc_like_query(const at::Tensor& query, std::array<int64_t, 4> shape) {
+  if (query.sizes() == at::IntArrayRef(shape.data(), 4)) return at::empty_like(query);
+  std::array<int, 4> order = {0, 1, 2, 3};
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return query.stride(a) > query.stride(b); });
+  std::array<int64_t, 4> permuted, back;
+  for (int i = 0; i < 4; ++i) permuted[i] = shape[order[i]];
+  for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 4; ++j)
+      if (order[j] == i) back[i] = j;
+  return at::empty(at::IntArrayRef(permuted.data(), 4), query.options()).permute(at::IntArrayRef(back.data(), 4));
 }
 
-// Scratch for one call: a fresh block from the caching allocator (stream-ordered, so the block can be
-// reused by the next call on the same stream as soon as this one has been queued).
-at::Tensor scratch(int dev, uint64_t bytes) {
-  return at::empty({static_cast<int64_t>(bytes < 16 ? 16 : bytes)},
-                   at::TensorOptions().device(at::kCUDA, dev).dtype(at::kByte));
-}
+namespace {
 
 void validate(const at::Tensor& query, const at::Tensor& key, const at::Tensor& value,
               const c10::optional<at::Tensor>& attn_bias, double dropout_p, bool is_causal, bool return_debug_mask) {
@@ -101,20 +98,6 @@ void validate(const at::Tensor& query, const at::Tensor& key, const at::Tensor& 
               "Expected query, key, and value to be on the same device");
 }
 
-// Output buffer laid out like the query: identical strides when the shapes agree, otherwise dense strides
-// in the query's dimension order (the rule of torch's own meta kernel for this op).
-at::Tensor alloc_like_query(const at::Tensor& query, std::array<int64_t, 4> shape) {
-  if (query.sizes() == at::IntArrayRef(shape.data(), 4)) return at::empty_like(query);
-  std::array<int, 4> order = {0, 1, 2, 3};
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return query.stride(a) > query.stride(b); });
-  std::array<int64_t, 4> permuted, back;
-  for (int i = 0; i < 4; ++i) permuted[i] = shape[order[i]];
-  for (int i = 0; i < 4; ++i)
-    for (int j = 0; j < 4; ++j)
-      if (order[j] == i) back[i] = j;
-  return at::empty(at::IntArrayRef(permuted.data(), 4), query.options()).permute(at::IntArrayRef(back.data(), 4));
-}
-
 // Strides of `bias` viewed as broadcast to (B, Hq, L, S): 0 where broadcast.
 void bias_strides(const at::Tensor& bias, const std::array<int64_t, 4>& target, int64_t* out) {
   TORCH_CHECK(bias.dim() <= 4, "attn_mask must have at most 4 dimensions");
@@ -130,10 +113,6 @@ void bias_strides(const at::Tensor& bias, const std::array<int64_t, 4>& target, 
       out[i] = 0;
     }
   }
-}
-
-template <size_t N> void copy_strides(const at::Tensor& t, int64_t (&dst)[N]) {
-  for (size_t i = 0; i < N; ++i) dst[i] = t.stride(static_cast<int64_t>(i));
 }
 
 // bool mask (true = keep) -> 0 / -inf in the query dtype; float masks as they are; other float widths -> fp32
@@ -327,11 +306,13 @@ at::Tensor status_word(int64_t device) { return device_state(static_cast<int>(de
 
 }  // namespace
 
+}  // namespace b200_ops
+
 TORCH_LIBRARY_IMPL(aten, CUDA, m) {
-  m.impl("_scaled_dot_product_fused_attention_overrideable", &fused_attention_overrideable);
-  m.impl("_scaled_dot_product_fused_attention_overrideable_backward", &fused_attention_overrideable_backward);
+  m.impl("_scaled_dot_product_fused_attention_overrideable", &b200_ops::fused_attention_overrideable);
+  m.impl("_scaled_dot_product_fused_attention_overrideable_backward", &b200_ops::fused_attention_overrideable_backward);
 }
 
 TORCH_LIBRARY(b200_sdpa_native, m) {
-  m.def("status_word(int device) -> Tensor", &status_word);
+  m.def("status_word(int device) -> Tensor", &b200_ops::status_word);
 }

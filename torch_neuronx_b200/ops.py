@@ -26,6 +26,7 @@ fallback: non-CUDA tensors are rejected and a missing library raises.
 
 from __future__ import annotations
 
+import collections.abc
 import ctypes as C
 import math
 from typing import Optional
@@ -45,8 +46,51 @@ _status_words: dict[int, torch.Tensor] = {}
 _zero_scalars: dict[int, tuple] = {}
 _workspaces: dict[tuple[int, int], torch.Tensor] = {}
 _retired_workspaces: list = []
-last_plan: dict = {}
 last_bwd_plan: dict = {}
+
+
+class _LastPlan(collections.abc.MutableMapping):
+    """The plan of the last forward call.  A call made by the direct native entry points leaves its plan there
+    and it is turned into a dict only when somebody looks."""
+
+    def __init__(self):
+        self._d: dict = {}
+
+    def _now(self) -> dict:
+        t = _lib.native.take_plan() if _lib.native is not None else None
+        if t is not None:
+            path, block_m, block_n, gx, gy, gz, threads, smem, splits, launches, workspace = t
+            self._d = dict(
+                path=_lib.PATH_NAMES.get(path, str(path)), block_m=block_m, block_n=block_n, grid=(gx, gy, gz),
+                threads=threads, smem_bytes=smem, kv_splits=splits, launches=launches, workspace_bytes=workspace,
+            )
+        return self._d
+
+    def __getitem__(self, key):
+        return self._now()[key]
+
+    def __setitem__(self, key, value):
+        self._now()[key] = value
+
+    def __delitem__(self, key):
+        del self._now()[key]
+
+    def __iter__(self):
+        return iter(self._now())
+
+    def __len__(self):
+        return len(self._now())
+
+    def clear(self):
+        if _lib.native is not None:
+            _lib.native.take_plan()
+        self._d = {}
+
+    def __repr__(self):
+        return repr(self._now())
+
+
+last_plan = _LastPlan()
 
 
 def _device_index(t: torch.Tensor) -> int:
@@ -226,6 +270,11 @@ def sdpa_forward(
 
     Inputs must already satisfy :func:`_validate`; dtype is fp32/fp16/bf16.
     ``attn_bias`` is additive (bool masks are converted by the callers)."""
+    if attn_bias is None and _lib.native is not None and not torch.compiler.is_compiling():
+        got = _lib.native.forward(query, key, value, is_causal, scale, kv_lens, q_offset, k_offset, need_lse, out, lse,
+                                  force_path, kv_chunk)
+        if got is not None:
+            return got
     lib = _lib.load()
     dev = _device_index(query)
     B, Hq, L, E = query.shape
@@ -395,6 +444,11 @@ def paged_decode(
     kernel reads the pages in place -- no gather into a dense cache.  Upstream's decode
     runs the same op on a dense cache (``torch_mlir/ops/scaled_dot_product_attention.py:64-68``);
     the paged layout is what a serving loop around that op keeps."""
+    if _lib.native is not None and layout in ("NHD", "HND") and not torch.compiler.is_compiling():
+        got = _lib.native.decode(query, k_pages, v_pages, block_table, kv_lens, scale, 1 if layout == "NHD" else 2, out, lse,
+                                 need_lse, kv_chunk, k_new, v_new, rope_cos, rope_sin, rope_interleaved)
+        if got is not None:
+            return got if k_new is not None else got[:2]
     lib = _lib.load()
     if layout not in ("NHD", "HND"):
         raise ValueError("layout must be 'NHD' or 'HND'")
@@ -531,6 +585,11 @@ def decode_append(
     and to the new key inside the same kernel (fp32 arithmetic, one rounding; ``rope_interleaved``
     selects the (2i, 2i+1) pairing instead of (i, i + D/2)) and the key is cached rotated.  (Upstream's loop appends with separate ops
     before the attention op: ``tests/blocks/block_def/llama.py:110-119`` is the caller shape.)"""
+    if _lib.native is not None and k_new is not None and not torch.compiler.is_compiling():
+        got = _lib.native.decode(query, k_cache, v_cache, None, kv_lens, scale, 0, None, None, need_lse, kv_chunk,
+                                 k_new, v_new, rope_cos, rope_sin, rope_interleaved)
+        if got is not None:
+            return got
     lib = _lib.load()
     if query.dim() != 4 or query.shape[2] != 1 or k_cache.dim() != 4 or v_cache.shape != k_cache.shape:
         raise RuntimeError("decode_append: query must be (B, Hq, 1, D) and the caches (B, Hkv, S, D)")
@@ -1036,6 +1095,10 @@ def scaled_dot_product_attention(
     the shapes (``Hq % Hkv == 0``) and never expanded in memory.  ``kv_lens``
     (int32 ``(B,)``) is the one extension: valid keys per batch for right padding or
     a ragged cache, instead of a dense mask."""
+    if attn_mask is None and dropout_p == 0.0 and _lib.native is not None and not torch.compiler.is_compiling():
+        out = _lib.native.attention(query, key, value, is_causal, scale, enable_gqa, kv_lens)
+        if out is not None:
+            return out
     _validate(query, key, value, attn_mask, dropout_p, is_causal, False)
     if not enable_gqa and query.shape[1] != key.shape[1]:
         raise RuntimeError("SDPA: number of heads differ between query and key; pass enable_gqa=True")
