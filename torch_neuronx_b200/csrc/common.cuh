@@ -132,6 +132,32 @@ int launch_bwd_tc(const BwdProblem& bp, int dtype, void* workspace, uint64_t wor
 
 void count_launch(int kernel_id);
 
+// ---- programmatic dependent launch -----------------------------------------
+// A kernel launched with launch_pdl() may be placed as soon as every CTA of the grid before it in the stream has
+// called pdl_launch_dependents() or finished, so its launch and set-up run under that grid's tail.  It calls
+// pdl_wait() before it touches global memory: that returns when the grid before it is complete and its writes are
+// visible (at once where that grid took no part in this).  Between the small calls of a generation loop the gaps
+// are worth 2-4 us each.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+bool launch_pdl(void (*kern)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
+
 // ---- small device helpers -------------------------------------------------
 
 template <typename T> __device__ __forceinline__ float to_f32(T x);

@@ -88,13 +88,13 @@ struct TileGeom {
   bool in_range;  // row0 < L
 };
 
-__device__ __forceinline__ TileGeom tile_geometry(const Problem& p, int row0, int kv_limit) {
+__device__ __forceinline__ TileGeom tile_geometry(const Problem& p, int row0, int kv_limit, int rows = kBlockM) {
   TileGeom g;
   g.row0 = row0;
   g.in_range = row0 < p.L;
   long long end = kv_limit, first = kv_limit;
   if (p.causal) {
-    const int last_row = (row0 + kBlockM < p.L ? row0 + kBlockM : p.L) - 1;
+    const int last_row = (row0 + rows < p.L ? row0 + rows : p.L) - 1;
     const long long e = static_cast<long long>(last_row) + p.causal_shift + 1;
     const long long f = static_cast<long long>(row0) + p.causal_shift + 1;
     end = e < end ? e : end;
@@ -107,14 +107,28 @@ __device__ __forceinline__ TileGeom tile_geometry(const Problem& p, int row0, in
   return g;
 }
 
+// The split form (PACK): few query rows against many keys.  A 128-row tile holds `lb` consecutive rows of every
+// query head of one kv head (heads * lb <= 128), so the group reads its keys once; the key axis is cut into
+// `n_split` ranges, one CTA each, whose unnormalised fp32 results and (maximum, sum) pairs a second launch merges.
+struct PackArgs {
+  int lb;               // rows of one head in a tile
+  int dual;             // one row tile only: the CTA's two tiles are the same rows against even and odd key tiles
+  int n_pairs;          // pairs of row tiles along the queries
+  int n_split;
+  int split_tiles;      // key tiles of one split
+  float* part_o;        // [B][Hq][L][n_split][Dv]
+  float* part_ml;       // [B][Hq][L][n_split][2]: maximum in log2 units, sum
+};
+
 // PAD: head dimensions E, Dv (multiples of 8) that do not fill the D = 128 tile.  The tensor maps carry the
 // real extents, so the copies fill the tile's remaining columns with zeros and the output store clips them;
 // the products run over ceil(E / 16) k-steps and ceil(Dv / 16) * 16 output columns only.
-template <int D, bool BF16, bool BIAS, bool ACC, bool PAD>
+template <int D, bool BF16, bool BIAS, bool ACC, bool PAD, bool PACK>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const Problem p,
-               const int n_qblk, const int pair_heads, const int streams_per_wave, const long long wait_limit) {
+               const int n_qblk, const int pair_heads, const int streams_per_wave, const long long wait_limit,
+               const PackArgs pack) {
   using C = Cfg<D>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -125,45 +139,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
 
-  // Work item: longest (latest) query blocks first, heads of one kv group adjacent.
-  // Two layouts of the CTA's two 128-row tiles:
-  //   pair_heads == 0: rows [256 q, +128) and [256 q + 128, +128) of one query head;
-  //   pair_heads == 1: the same 128 rows of two query heads that share a kv head
-  //     (even group size) -- both tiles then see exactly the same keys, so under a
-  //     causal mask neither waits for the other's extra diagonal tile.
-  // The (batch, kv head) key/value streams are taken `streams_per_wave` at a time, so that what the
-  // CTAs in flight read together fits in L2 (all streams at once when they do).
-  const int heads_per_cta = pair_heads ? 2 : 1;
-  const int ctas_per_stream = p.group / heads_per_cta;            // per query block
-  const int n_streams = p.Hkv * p.B;
-  const int full_wave_ctas = n_qblk * streams_per_wave * ctas_per_stream;
-  const int wave = static_cast<int>(blockIdx.x / full_wave_ctas);
-  const int in_wave = static_cast<int>(blockIdx.x - static_cast<unsigned>(wave) * full_wave_ctas);
-  const int first_stream = wave * streams_per_wave;
-  const int wave_streams = (n_streams - first_stream) < streams_per_wave ? (n_streams - first_stream) : streams_per_wave;
-  const int per_blk = wave_streams * ctas_per_stream;
-  const int qblk = n_qblk - 1 - in_wave / per_blk;
-  const int rem = in_wave % per_blk;
-  const int stream = first_stream + rem / ctas_per_stream;
-  const int hk = stream % p.Hkv;
-  const int b = stream / p.Hkv;
-  const int hq0 = hk * p.group + (rem % ctas_per_stream) * heads_per_cta;
-  const int head_of_tile[2] = {hq0, pair_heads ? hq0 + 1 : hq0};
-  const int kv_limit = valid_keys(p, b);
-  const int rows_per_cta = pair_heads ? kBlockM : kRowsPerCta;
-  const TileGeom tg0 = tile_geometry(p, qblk * rows_per_cta, kv_limit);
-  const TileGeom tg1 = tile_geometry(p, qblk * rows_per_cta + (pair_heads ? 0 : kBlockM), kv_limit);
-  const int n_iter = tg0.n_tiles > tg1.n_tiles ? tg0.n_tiles : tg1.n_tiles;
-
-
-  const uint32_t q_smem[2] = {tiles, tiles + C::kTileBytes};
-  const uint32_t kv_smem = tiles + kTilesPerCta * C::kTileBytes;
-
-  // Set-up is spread over the roles so that the first copies are in flight while
-  // barriers are initialised and tensor memory is allocated: the producer lane owns
-  // the barriers of its own copies and starts Q and the first ring slots at once.
-  int items_issued = 0;   // (producer lane) ring items already issued
-  bool q_armed = false;   // (producer lane) a copy into the Q slots is in flight or has landed
+  // Set-up.  The kernel is launched as a programmatic dependent of whatever precedes it in the stream: barriers,
+  // tensor memory and the tensor maps are made ready while that finishes, and nothing of global memory is touched
+  // before the wait (which returns when the preceding grid is complete and its writes are visible).
   if (warp == kProducerWarp && lane == 0) {
     mbar_init(smem_u32(&sync->q_full), 1);
     for (int s = 0; s < C::kStages; ++s) {
@@ -171,29 +149,10 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       mbar_init(smem_u32(&sync->kv_empty[s]), 1);
     }
     mbar_fence_init();
-    // A tile without visible keys never reads its Q: its shared-memory slot is used
-    // straight away to stage the all-zero output, so nothing may be in flight into it.
-    uint32_t q_bytes = 0;
-    if (tg0.n_tiles > 0) q_bytes += C::kTileBytes;
-    if (tg1.n_tiles > 0) q_bytes += C::kTileBytes;
-    const uint32_t qbar = smem_u32(&sync->q_full);
-    if (q_bytes > 0) mbar_arrive_expect_tx(qbar, q_bytes);
-    q_armed = q_bytes > 0;
-    for (int t = 0; t < 2; ++t) {
-      const TileGeom& tg = t == 0 ? tg0 : tg1;
-      if (tg.n_tiles == 0) continue;
-      for (int bx = 0; bx < C::kBoxes; ++bx)
-        tma_load_4d(q_smem[t] + bx * kBoxBytes, &tm_q, qbar, bx * 64, tg.row0, head_of_tile[t], b);
-    }
-    for (; items_issued < 2 * n_iter && items_issued < C::kStages; ++items_issued) {
-      const uint32_t bar = smem_u32(&sync->kv_full[items_issued]);
-      mbar_arrive_expect_tx(bar, C::kTileBytes);
-      const CUtensorMap* map = (items_issued & 1) ? &tm_v : &tm_k;
-      for (int bx = 0; bx < C::kBoxes; ++bx)
-        tma_load_4d(kv_smem + items_issued * C::kTileBytes + bx * kBoxBytes, map, bar, bx * 64,
-                    (items_issued >> 1) * kBlockN, hk, b);
-    }
-    prefetch_tmap(&tm_o);
+    prefetch_tmap(&tm_q);
+    prefetch_tmap(&tm_k);
+    prefetch_tmap(&tm_v);
+    if (!PACK) prefetch_tmap(&tm_o);
   }
   if (tid < 2) {
     const int t = tid;
@@ -214,6 +173,113 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     tmem_alloc(smem_u32(&sync->tmem_base), kTmemCols);
     tmem_relinquish();
   }
+  pdl_wait();
+  // the next kernel of the stream may be placed where this grid leaves room
+  pdl_launch_dependents();
+
+  // Work item: longest (latest) query blocks first, heads of one kv group adjacent.
+  // Two layouts of the CTA's two 128-row tiles:
+  //   pair_heads == 0: rows [256 q, +128) and [256 q + 128, +128) of one query head;
+  //   pair_heads == 1: the same 128 rows of two query heads that share a kv head
+  //     (even group size) -- both tiles then see exactly the same keys, so under a
+  //     causal mask neither waits for the other's extra diagonal tile.
+  // The (batch, kv head) key/value streams are taken `streams_per_wave` at a time, so that what the
+  // CTAs in flight read together fits in L2 (all streams at once when they do).
+  int hk, b, hq0, key_tile0 = 0;
+  const bool dual = PACK && pack.dual != 0;
+  TileGeom tg0, tg1;
+  int head_of_tile[2];
+  int kv_limit;
+  if constexpr (PACK) {
+    // neighbouring CTAs: the splits of one pair of row tiles (longest first), then the next (batch, kv head)
+    const int n_ranges = dual ? pack.n_split / 2 : pack.n_split;   // CTAs along the keys
+    const int split = static_cast<int>(blockIdx.x) % n_ranges;
+    const int unit = static_cast<int>(blockIdx.x) / n_ranges;
+    const int n_streams = p.Hkv * p.B;
+    const int pair = pack.n_pairs - 1 - unit / n_streams;
+    const int stream = unit % n_streams;
+    hk = stream % p.Hkv;
+    b = stream / p.Hkv;
+    hq0 = hk * p.group;
+    head_of_tile[0] = head_of_tile[1] = hq0;
+    kv_limit = valid_keys(p, b);
+    key_tile0 = split * pack.split_tiles;
+    tg0 = tile_geometry(p, 2 * pair * pack.lb, kv_limit, pack.lb);
+    tg1 = tile_geometry(p, (2 * pair + 1) * pack.lb, kv_limit, pack.lb);
+    auto clip = [&](int n) { n -= key_tile0; return n < 0 ? 0 : (n > pack.split_tiles ? pack.split_tiles : n); };
+    tg0.n_tiles = clip(tg0.n_tiles);
+    tg1.n_tiles = clip(tg1.n_tiles);
+    if (dual) {
+      const int n = tg0.n_tiles;
+      tg1 = tg0;
+      tg0.n_tiles = (n + 1) / 2;
+      tg1.n_tiles = n / 2;
+    }
+  } else {
+    const int heads_per_cta = pair_heads ? 2 : 1;
+    const int ctas_per_stream = p.group / heads_per_cta;            // per query block
+    const int n_streams = p.Hkv * p.B;
+    const int full_wave_ctas = n_qblk * streams_per_wave * ctas_per_stream;
+    const int wave = static_cast<int>(blockIdx.x / full_wave_ctas);
+    const int in_wave = static_cast<int>(blockIdx.x - static_cast<unsigned>(wave) * full_wave_ctas);
+    const int first_stream = wave * streams_per_wave;
+    const int wave_streams = (n_streams - first_stream) < streams_per_wave ? (n_streams - first_stream) : streams_per_wave;
+    const int per_blk = wave_streams * ctas_per_stream;
+    const int qblk = n_qblk - 1 - in_wave / per_blk;
+    const int rem = in_wave % per_blk;
+    const int stream = first_stream + rem / ctas_per_stream;
+    hk = stream % p.Hkv;
+    b = stream / p.Hkv;
+    hq0 = hk * p.group + (rem % ctas_per_stream) * heads_per_cta;
+    head_of_tile[0] = hq0;
+    head_of_tile[1] = pair_heads ? hq0 + 1 : hq0;
+    kv_limit = valid_keys(p, b);
+    const int rows_per_cta = pair_heads ? kBlockM : kRowsPerCta;
+    tg0 = tile_geometry(p, qblk * rows_per_cta, kv_limit);
+    tg1 = tile_geometry(p, qblk * rows_per_cta + (pair_heads ? 0 : kBlockM), kv_limit);
+  }
+  const int n_iter = tg0.n_tiles > tg1.n_tiles ? tg0.n_tiles : tg1.n_tiles;
+
+  // Ring items.  Item i is a K or a V tile; plain order K(0) V(0) K(1) V(1) ..., dual order K(0) K(1) V(0) V(1) K(2)
+  // K(3) V(2) V(3) ... (the last odd pair may be missing).
+  const int n_ring = dual ? 4 * n_iter : 2 * n_iter;
+  auto item_is_v = [&](int i) { return dual ? (i >> 1) & 1 : i & 1; };
+  auto item_tile = [&](int i) { return dual ? (i >> 2) * 2 + (i & 1) : i >> 1; };
+  auto item_exists = [&](int i) { return !dual || item_tile(i) < tg0.n_tiles + tg1.n_tiles; };
+
+  const uint32_t q_smem[2] = {tiles, tiles + C::kTileBytes};
+  const uint32_t kv_smem = tiles + kTilesPerCta * C::kTileBytes;
+
+  // The producer lane, which initialised the barriers of its own copies, starts Q and the first ring slots before
+  // the CTA-wide barrier.
+  int items_issued = 0;   // (producer lane) ring items already issued
+  bool q_armed = false;   // (producer lane) a copy into the Q slots is in flight or has landed
+  if (warp == kProducerWarp && lane == 0) {
+    // A tile without visible keys never reads its Q: its shared-memory slot is used
+    // straight away to stage the all-zero output, so nothing may be in flight into it.
+    const uint32_t q_tile_bytes = PACK ? C::kBoxes * 128 * pack.lb * p.group : C::kTileBytes;
+    uint32_t q_bytes = 0;
+    if (tg0.n_tiles > 0) q_bytes += q_tile_bytes;
+    if (tg1.n_tiles > 0 && !dual) q_bytes += q_tile_bytes;
+    const uint32_t qbar = smem_u32(&sync->q_full);
+    if (q_bytes > 0) mbar_arrive_expect_tx(qbar, q_bytes);
+    q_armed = q_bytes > 0;
+    for (int t = 0; t < 2; ++t) {
+      const TileGeom& tg = t == 0 ? tg0 : tg1;
+      if (tg.n_tiles == 0 || (dual && t == 1)) continue;
+      for (int bx = 0; bx < C::kBoxes; ++bx)
+        tma_load_4d(q_smem[t] + bx * kBoxBytes, &tm_q, qbar, bx * 64, tg.row0, head_of_tile[t], b);
+    }
+    for (; items_issued < n_ring && items_issued < C::kStages; ++items_issued) {
+      if (!item_exists(items_issued)) continue;
+      const uint32_t bar = smem_u32(&sync->kv_full[items_issued]);
+      mbar_arrive_expect_tx(bar, C::kTileBytes);
+      const CUtensorMap* map = item_is_v(items_issued) ? &tm_v : &tm_k;
+      for (int bx = 0; bx < C::kBoxes; ++bx)
+        tma_load_4d(kv_smem + items_issued * C::kTileBytes + bx * kBoxBytes, map, bar, bx * 64,
+                    (key_tile0 + item_tile(items_issued)) * kBlockN, hk, b);
+    }
+  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -223,8 +289,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
       bool alive = true;
-      for (int item = items_issued; item < 2 * n_iter && alive; ++item) {
-        const int j = item >> 1;
+      for (int item = items_issued; item < n_ring && alive; ++item) {
+        if (!item_exists(item)) continue;
+        const int j = item_tile(item);
         const int stage = item % C::kStages;
         const uint32_t round = static_cast<uint32_t>(item / C::kStages);
         if (round > 0) {
@@ -237,8 +304,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const uint32_t bar = smem_u32(&sync->kv_full[stage]);
         const uint32_t dst = kv_smem + stage * C::kTileBytes;
         mbar_arrive_expect_tx(bar, C::kTileBytes);
-        const CUtensorMap* map = (item & 1) ? &tm_v : &tm_k;
-        for (int bx = 0; bx < C::kBoxes; ++bx) tma_load_4d(dst + bx * kBoxBytes, map, bar, bx * 64, j * kBlockN, hk, b);
+        const CUtensorMap* map = item_is_v(item) ? &tm_v : &tm_k;
+        for (int bx = 0; bx < C::kBoxes; ++bx) tma_load_4d(dst + bx * kBoxBytes, map, bar, bx * 64, (key_tile0 + j) * kBlockN, hk, b);
         items_issued = item + 1;
       }
     }
@@ -260,7 +327,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       const uint64_t kv_desc_v = smem_desc_sw128(kv_smem, kBoxBytes, 1024);   // V tile as MN-major B operand
       auto issue_qk = [&](auto tile_const, uint32_t stage) {
         constexpr int t = decltype(tile_const)::value;
-        const uint64_t qd = t == 0 ? q_desc0 : q_desc1;
+        const uint64_t qd = t == 0 || dual ? q_desc0 : q_desc1;
         const uint64_t kd = kv_desc_k + static_cast<uint64_t>(stage * (C::kTileBytes >> 4));
         const uint32_t d_addr = tmem_base + static_cast<uint32_t>(t * 128);
         if (elect_one() && dbg_tmem(p.status, DBG_PREFILL * 100 + 1, d_addr, tmem_base, 128, 512)) {
@@ -308,6 +375,56 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         if (!alive && lane == 0) report(p.status, 2, -1, 0);
       }
       if (alive) alive = wait_full(0);
+      if (PACK && dual) {
+        // Tile t works on key tiles 2 j + t: K at ring item 4 j + t, V at 4 j + 2 + t, each with one reader.
+        auto scores = [&](auto tile_const, int j) {
+          constexpr int t = decltype(tile_const)::value;
+          const int item = 4 * j + t;
+          alive = wait_full(item);
+          if (!alive) return;
+          tc_fence_after_sync();
+          issue_qk(tile_const, stage_addr(item));
+          commit(smem_u32(&sync->s_full[t]));
+          commit(empty_bar(item));
+        };
+        auto serve = [&](auto tile_const, int j) {
+          constexpr int t = decltype(tile_const)::value;
+          const int nt = t == 0 ? tg0.n_tiles : tg1.n_tiles;
+          if (j >= nt) return;
+          if (C::kSplitP && j + 1 < nt) {   // as below: next scores first
+            alive = wait_clocked(smem_u32(&sync->s_free[t]), j & 1, abort_flag, wait_limit);
+            if (!alive) {
+              if (lane == 0) report(p.status, 9, j, t);
+              return;
+            }
+            scores(tile_const, j + 1);
+            if (!alive) return;
+          }
+          alive = wait_full(4 * j + 2 + t);
+          if (!alive) return;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            alive = wait_clocked(smem_u32(&sync->p_ready[t][half]), j & 1, abort_flag, wait_limit);
+            if (!alive) {
+              if (lane == 0) report(p.status, 3, j, t);
+              return;
+            }
+            tc_fence_after_sync();
+            issue_pv_half(tile_const, stage_addr(4 * j + 2 + t), half, j > 0);
+          }
+          commit(empty_bar(4 * j + 2 + t));
+          if (C::kSplitP) commit(smem_u32(&sync->pv_done[t]));
+          if (j + 1 >= nt) commit(smem_u32(&sync->o_done[t]));
+          else if (!C::kSplitP) scores(tile_const, j + 1);
+        };
+        if (alive && tg0.n_tiles > 0) scores(T0, 0);
+        if (alive && tg1.n_tiles > 0) scores(T1, 0);
+        for (int j = 0; j < n_iter && alive; ++j) {
+          serve(T0, j);
+          if (alive) serve(T1, j);
+        }
+        alive = false;   // done: the loop below is the plain order's
+      }
       if (alive) {
         tc_fence_after_sync();
         if (tg0.n_tiles > 0) {
@@ -401,7 +518,11 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         !dbg_tmem(p.status, DBG_PREFILL * 100 + 5, o_addr, tmem_base, D, 512) ||
         !dbg_tmem(p.status, DBG_PREFILL * 100 + 6, p_addr, tmem_base, 64, 512))
       *abort_flag = 1;
-    const int row_g = tg.row0 + r;
+    const int row_g = tg.row0 + (PACK ? r % pack.lb : r);
+    // (split form) a tile row that belongs to no query row holds whatever was in shared memory: its lane computes on
+    // that, in its own accumulator row, and stores nothing
+    const int head_g = PACK ? hq0 + r / pack.lb : head_of_tile[t];
+    const bool row_used = !PACK || (r < pack.lb * p.group && row_g < p.L);
     int lim = kv_limit;                      // keys [0, lim) are visible to this row
     if (p.causal) {
       const long long c = static_cast<long long>(row_g) + p.causal_shift + 1;
@@ -445,7 +566,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           break;
         }
         tc_fence_after_sync();
-        const int col0 = j * kBlockN;
+        const int col0 = (key_tile0 + (dual ? 2 * j + t : j)) * kBlockN;
         const bool need_mask = col0 + kBlockN > tg.min_lim;
 
         // S row -> registers in two halves; the second half is in flight while the
@@ -567,7 +688,41 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         }
         tc_fence_after_sync();
       }
-      if constexpr (ACC) {
+      if constexpr (PACK) {
+        if (alive) {
+          const int64_t slot = ((static_cast<int64_t>(b) * p.Hq + head_g) * p.L + row_g) * pack.n_split +
+                               (dual ? 2 * (key_tile0 / pack.split_tiles) + t : key_tile0 / pack.split_tiles);
+          const bool slot_ok = row_used && dbg_range(p.status, DBG_PREFILL * 100 + 9, slot, 1,
+                                                     static_cast<int64_t>(p.B) * p.Hq * p.L * pack.n_split);
+          if (slot_ok) *reinterpret_cast<float2*>(pack.part_ml + slot * 2) = make_float2(m_run * sl2, l_run);
+          // O: every lane holds a row; 32 columns at a time go through this warp's 4 KB of the (idle) Q slot, so
+          // that eight lanes store the 128 bytes of one row
+          const int64_t my_row = slot_ok && l_run > 0.f ? slot : -1;
+          uint8_t* buf = smem_raw + (q_smem[t] - raw_addr) + quad * 4096;
+          if (tg.n_tiles > 0) {
+#pragma unroll
+            for (int c = 0; c < D / 32; ++c) {
+              uint32_t v[32];
+              tmem_ld_32x32(o_addr + c * 32, v);
+              tmem_ld_wait();
+              __syncwarp();
+#pragma unroll
+              for (int u = 0; u < 8; ++u)
+                *reinterpret_cast<uint4*>(buf + lane * 128 + ((u ^ (lane & 7)) << 4)) =
+                    make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
+              __syncwarp();
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int row = i * 4 + (lane >> 3), u = lane & 7;
+                const int64_t dst = __shfl_sync(0xffffffffu, my_row, row);
+                if (dst >= 0)
+                  *reinterpret_cast<uint4*>(pack.part_o + dst * D + c * 32 + u * 4) =
+                      *reinterpret_cast<const uint4*>(buf + row * 128 + ((u ^ (row & 7)) << 4));
+              }
+            }
+          }
+        }
+      } else if constexpr (ACC) {
         // Accumulating form (a ring step): fold this block's result into the row's running fp32 pair
         // (acc, acc_lse) in place -- acc = acc * w_acc + O * w_o -- instead of writing out / lse.  Same
         // arithmetic as the persistent kernel's accumulating epilogue.  A tile without a visible key
@@ -707,7 +862,7 @@ int launch_variant(const Problem& p, cudaStream_t stream) {
   } else if (!make_map(&to, p.out, BF16, p.Dv, p.L, p.Hq, p.B, p.os)) {
     return B200_SDPA_ERR_CUDA;
   }
-  auto kern = prefill_kernel<D, BF16, BIAS, ACC, PAD>;
+  auto kern = prefill_kernel<D, BF16, BIAS, ACC, PAD, false>;
   // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute: set on every
   // launch (a cheap host-side call), so a process that drives several GPUs gets it on each of them
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) {
@@ -720,9 +875,9 @@ int launch_variant(const Problem& p, cudaStream_t stream) {
   const long long grid = static_cast<long long>(n_qblk) * (p.Hq / (pair_heads ? 2 : 1)) * p.B;
   if (grid <= 0 || grid > 0x7fffffffLL) return B200_SDPA_ERR_UNSUPPORTED;
   const int per_wave = kv_streams_per_wave(static_cast<long long>(p.S) * (p.E + p.Dv) * 2, static_cast<long long>(p.Hkv) * p.B);
-  kern<<<static_cast<unsigned>(grid), kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, to, p, n_qblk, pair_heads,
-                                                                         per_wave, wait_limit_cycles());
-  if (cudaGetLastError() != cudaSuccess) return B200_SDPA_ERR_CUDA;
+  if (!launch_pdl(kern, dim3(static_cast<unsigned>(grid)), kThreads, C::kSmemBytes, stream, tq, tk, tv, to, p, n_qblk, pair_heads,
+                  per_wave, wait_limit_cycles(), PackArgs{}))
+    return B200_SDPA_ERR_CUDA;
   count_launch(KID_PREFILL);
   return B200_SDPA_OK;
 }
@@ -758,6 +913,178 @@ void plan_per_cta(const Problem& p, long long grid, int rows, B200SdpaPlan* plan
   plan->workspace_bytes = 0;
 }
 
+// Merge of the split form's partials: one warp per query row, the row's columns spread over the lanes.
+template <typename T, int D>
+__global__ void __launch_bounds__(256) prefill_combine_kernel(const Problem p, const int n_split,
+                                                              const float* __restrict__ part_o,
+                                                              const float* __restrict__ part_ml) {
+  constexpr int C = D / 32;   // columns per lane
+  const int lane = threadIdx.x & 31;
+  const int64_t row_id = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  pdl_wait();
+  pdl_launch_dependents();
+  if (row_id >= static_cast<int64_t>(p.B) * p.Hq * p.L) return;
+  const int i = static_cast<int>(row_id % p.L);
+  const int h = static_cast<int>((row_id / p.L) % p.Hq);
+  const int b = static_cast<int>(row_id / p.L / p.Hq);
+  float2 ml = make_float2(-CUDART_INF_F, 0.f);
+  if (lane < n_split) ml = *reinterpret_cast<const float2*>(part_ml + (row_id * n_split + lane) * 2);
+  float mx = ml.x;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const float w = ml.y > 0.f ? ex2(ml.x - mx) : 0.f;
+  float lsum = w * ml.y;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+  float acc[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) acc[c] = 0.f;
+  const float* src = part_o + row_id * n_split * D + lane * C;
+#pragma unroll 4
+  for (int s = 0; s < n_split; ++s) {
+    const float ws = __shfl_sync(0xffffffffu, w, s);
+    if (ws > 0.f) {   // a split without a visible key for this row wrote nothing
+      float v[C];
+      if constexpr (C == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src + s * D);
+      else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(src + s * D);
+#pragma unroll
+      for (int c = 0; c < C; ++c) acc[c] = fmaf(v[c], ws, acc[c]);
+    }
+  }
+  const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
+  if (!dbg_bhrc(p.status, DBG_PREFILL * 100 + 10, b, p.B, h, p.Hq, i, p.L, lane * C, C, p.Dv)) return;
+  T* out = reinterpret_cast<T*>(p.out) + b * p.os[0] + static_cast<int64_t>(h) * p.os[1] + static_cast<int64_t>(i) * p.os[2] + lane * C;
+  T r[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) r[c] = from_f32<T>(acc[c] * inv);
+  if constexpr (C == 4) *reinterpret_cast<uint2*>(out) = *reinterpret_cast<const uint2*>(r);
+  else *reinterpret_cast<uint32_t*>(out) = *reinterpret_cast<const uint32_t*>(r);
+  if (p.lse != nullptr && lane == 0)
+    p.lse[b * p.ls[0] + h * p.ls[1] + i * p.ls[2]] = lsum > 0.f ? fmaf(mx, kLn2, lg2(lsum) * kLn2) : -CUDART_INF_F;
+}
+
+struct PackGeom {
+  int lb, n_pairs, dual, n_split, split_tiles;
+  long long grid;
+  uint64_t ws_bytes;
+};
+
+// Whether the split form serves a request, and how.  The plain form gives every 128 (or 256) rows of a head a CTA
+// that walks all its keys: with a handful of rows, or few heads and sequences, that leaves most SMs without work and
+// most of every tile without rows.  The rule compares estimates of both, in cycles of one SM:
+//   plain   the longest CTA, or all key tiles spread over the SMs, at kPairCycles each, + kCtaCycles per round of CTAs
+//   split   the same for the packed tiles, + the fp32 partials written and read once, + a second launch
+// neither below the time the keys and values need from HBM, and takes the split form where it saves a twentieth.
+// bf16, 32/8 heads: 8 x 8 rows against 4096 keys 72 -> 34 us (HBM floor 21), 1 x 16 rows against 8192 keys 123 -> 20,
+// 1 x 128 against 8192 keys 123 -> 29; 8/8 heads, 1024 rows and keys 23.7 -> 17.6.
+bool pack_geometry(const Problem& p, PackGeom* best) {
+  constexpr long long kSms = 148, kPairCycles = 3400, kPackedCycles = 3600, kCtaCycles = 9000, kLaunchCycles = 6000, kHbmBytesPerCycle = 3400;
+  constexpr int kMaxSplit = 32;
+  if (p.E != p.Dv || (p.E != 64 && p.E != 128) || p.bias != nullptr || p.acc_mode != 0 || p.group > kBlockM) return false;
+  const char* mode = getenv("B200_SDPA_PREFILL");
+  const bool forced = mode != nullptr && mode[0] == 's';   // "split"
+  if (mode != nullptr && !forced) return false;
+  const long long streams = static_cast<long long>(p.Hkv) * p.B;
+  const long long tiles = (p.S + kBlockN - 1) / kBlockN;
+  if (tiles < 2) return false;
+  auto key_tiles = [&](long long last_row) {   // tiles that rows up to last_row see
+    long long end = p.S;
+    if (p.causal) {
+      const long long e = (last_row < p.L ? last_row : p.L - 1) + p.causal_shift + 1;
+      end = e < end ? (e < 0 ? 0 : e) : end;
+    }
+    return (end + kBlockN - 1) / kBlockN;
+  };
+  const long long hbm = streams * key_tiles(p.L - 1) * kBlockN * (p.E + p.Dv) * 2 / kHbmBytesPerCycle;
+  auto estimate = [&](long long total, long long longest, long long ctas, long long per_tile) {
+    // equal CTAs run in whole rounds; unequal ones (a causal mask), longest first, spread out
+    const long long rounds = (ctas + kSms - 1) / kSms, spread = (total + kSms - 1) / kSms + longest / 2;
+    const bool equal = total * 4 > ctas * longest * 3;
+    const long long steps = equal ? rounds * longest : (ctas <= kSms || spread < longest ? longest : spread);
+    const long long work = steps * per_tile;
+    return kLaunchCycles + (work > hbm ? work : hbm) + kCtaCycles * rounds;
+  };
+  const int pair_heads = pair_heads_mode(p);
+  const int rows = pair_heads ? kBlockM : kRowsPerCta;
+  const long long blocks = (p.L + rows - 1) / rows, per_block = static_cast<long long>(p.Hq / (pair_heads ? 2 : 1)) * p.B;
+  if (!forced && blocks >= 64) return false;   // many rows: the plain form's tiles are full
+  long long total = 0, longest = 0;
+  for (long long i = 0; i < blocks; ++i) {
+    const long long n = key_tiles((i + 1) * rows - 1);
+    total += n * per_block;
+    longest = n > longest ? n : longest;
+  }
+  const long long plain = estimate(total, longest, blocks * per_block, kPairCycles);
+
+  PackGeom g;
+  g.lb = kBlockM / p.group < p.L ? kBlockM / p.group : p.L;
+  const int n_rt = (p.L + g.lb - 1) / g.lb;
+  g.n_pairs = (n_rt + 1) / 2;
+  g.dual = n_rt == 1 ? 1 : 0;
+  total = longest = 0;
+  for (long long i = 0; i < g.n_pairs; ++i) {
+    const long long n = key_tiles((i + 1) * 2 * g.lb - 1);
+    total += n * streams;
+    longest = n > longest ? n : longest;
+  }
+  const long long row_bytes = static_cast<long long>(p.B) * p.Hq * p.L * (p.Dv + 2) * 4;
+  long long best_cost = forced ? (1LL << 60) : plain * 19 / 20;
+  bool found = false;
+  const int per_cta = g.dual ? 2 : 1;   // partials a CTA leaves for a row
+  for (int n = 1; n * per_cta <= kMaxSplit && n <= tiles; ++n) {
+    g.split_tiles = static_cast<int>((tiles + n - 1) / n);
+    if ((tiles + g.split_tiles - 1) / g.split_tiles != n || (forced && n == 1 && !g.dual)) continue;
+    g.n_split = n * per_cta;
+    g.grid = g.n_pairs * streams * n;
+    g.ws_bytes = static_cast<uint64_t>(row_bytes) * g.n_split;
+    if (g.grid > 0x7fffffffLL) break;
+    const long long part = longest < g.split_tiles ? longest : g.split_tiles;
+    // two key tiles in the time of one where both tiles of the CTA are the same rows; partials written and read
+    // back at about 6 KB a cycle for the whole chip
+    const long long cost = estimate((total + per_cta - 1) / per_cta, (part + per_cta - 1) / per_cta, g.grid, g.dual ? kPairCycles : kPackedCycles) +
+                           kLaunchCycles + 2 * row_bytes * g.n_split / 6000;
+    if (cost < best_cost) {
+      best_cost = cost;
+      *best = g;
+      found = true;
+    }
+  }
+  return found;
+}
+
+template <int D, bool BF16>
+int launch_packed(const Problem& p, const PackGeom& g, float* workspace, cudaStream_t stream) {
+  using C = Cfg<D>;
+  CUtensorMap tq, tk, tv;
+  if (!make_map(&tq, p.q, BF16, D, p.L, p.Hq, p.B, p.qs, g.lb, p.group) || !make_map(&tk, p.k, BF16, D, p.S, p.Hkv, p.B, p.ks) ||
+      !make_map(&tv, p.v, BF16, D, p.S, p.Hkv, p.B, p.vs))
+    return B200_SDPA_ERR_CUDA;
+  auto kern = prefill_kernel<D, BF16, false, false, false, true>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) {
+    cudaGetLastError();
+    return B200_SDPA_ERR_CUDA;
+  }
+  const long long n_rows = static_cast<long long>(p.B) * p.Hq * p.L;
+  PackArgs a;
+  a.lb = g.lb;
+  a.dual = g.dual;
+  a.n_pairs = g.n_pairs;
+  a.n_split = g.n_split;
+  a.split_tiles = g.split_tiles;
+  a.part_o = workspace;
+  a.part_ml = workspace + n_rows * g.n_split * D;
+  if (!launch_pdl(kern, dim3(static_cast<unsigned>(g.grid)), kThreads, C::kSmemBytes, stream, tq, tk, tv, tq, p, 0, 0, 1,
+                  wait_limit_cycles(), a))
+    return B200_SDPA_ERR_CUDA;
+  count_launch(KID_PREFILL);
+  using T = std::conditional_t<BF16, __nv_bfloat16, __half>;
+  if (!launch_pdl(prefill_combine_kernel<T, D>, dim3(static_cast<unsigned>((n_rows + 7) / 8)), 256, 0, stream, p, g.n_split,
+                  a.part_o, a.part_ml))
+    return B200_SDPA_ERR_CUDA;
+  count_launch(KID_COMBINE);
+  return B200_SDPA_OK;
+}
+
 }  // namespace
 
 bool prefill_eligible(const Problem& p, int dtype, bool* alignment_only_failure) {
@@ -782,6 +1109,14 @@ bool prefill_padded_eligible(const Problem& p, int dtype) {
 int plan_prefill(const Problem& p, int dtype, B200SdpaPlan* plan) {
   if (p.E > 128) return plan_prefill_wide(p, dtype, plan);
   if (!prefill_eligible(p, dtype, nullptr)) return B200_SDPA_ERR_UNSUPPORTED;
+  PackGeom g;
+  if (pack_geometry(p, &g)) {
+    plan_per_cta(p, g.grid, g.lb * p.group, plan);
+    plan->kv_splits = g.n_split;
+    plan->launches = 2;
+    plan->workspace_bytes = g.ws_bytes;
+    return B200_SDPA_OK;
+  }
   if (prefill_persistent_wanted(p)) {
     plan_prefill_persistent(p, plan);
     return B200_SDPA_OK;
@@ -817,8 +1152,15 @@ int launch_prefill_padded(const Problem& p, int dtype, cudaStream_t stream) {
 int launch_prefill(const Problem& p, int dtype, void* workspace, uint64_t workspace_bytes, cudaStream_t stream) {
   if (p.E > 128) return launch_prefill_wide(p, dtype, stream);
   if (!prefill_eligible(p, dtype, nullptr)) return B200_SDPA_ERR_UNSUPPORTED;
-  if (prefill_persistent_wanted(p)) return launch_prefill_persistent(p, dtype, workspace, workspace_bytes, stream);
   const bool bf16 = dtype == B200_SDPA_BF16;
+  PackGeom g;
+  if (workspace != nullptr && reinterpret_cast<uintptr_t>(workspace) % 16 == 0 && pack_geometry(p, &g) &&
+      workspace_bytes >= g.ws_bytes) {
+    float* ws = reinterpret_cast<float*>(workspace);
+    if (p.E == 128) return bf16 ? launch_packed<128, true>(p, g, ws, stream) : launch_packed<128, false>(p, g, ws, stream);
+    return bf16 ? launch_packed<64, true>(p, g, ws, stream) : launch_packed<64, false>(p, g, ws, stream);
+  }
+  if (prefill_persistent_wanted(p)) return launch_prefill_persistent(p, dtype, workspace, workspace_bytes, stream);
   if (p.acc_mode != 0) {
     if (!prefill_accumulate_eligible(p)) return B200_SDPA_ERR_UNSUPPORTED;
     return bf16 ? launch_variant<128, true, false, true>(p, stream) : launch_variant<128, false, false, true>(p, stream);

@@ -161,9 +161,9 @@ inline EncodeTiledFn encode_fn() {
 }
 
 // (D, rows, heads, batch) view of a (B, H, S, D) tensor with unit inner stride; one copy moves `box_rows` rows of
-// 64 elements.
+// 64 elements (of `box_heads` heads).
 inline bool make_map(CUtensorMap* map, const void* base, bool bf16, int d, int rows, int heads, int batch,
-              const int64_t* stride /* elements, (B,H,S,D) order */, int box_rows = kTileRows) {
+              const int64_t* stride /* elements, (B,H,S,D) order */, int box_rows = kTileRows, int box_heads = 1) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return false;
   const cuuint64_t dims[4] = {static_cast<cuuint64_t>(d), static_cast<cuuint64_t>(rows),
@@ -173,7 +173,7 @@ inline bool make_map(CUtensorMap* map, const void* base, bool bf16, int d, int r
     return static_cast<cuuint64_t>((n == 1 ? static_cast<int64_t>(d) : s) * 2);
   };
   const cuuint64_t strides[3] = {fix(stride[2], rows), fix(stride[1], heads), fix(stride[0], batch)};
-  const cuuint32_t box[4] = {64, static_cast<cuuint32_t>(box_rows), 1, 1};
+  const cuuint32_t box[4] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(box_heads), 1};
   const cuuint32_t elem[4] = {1, 1, 1, 1};
   const CUresult rc = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
                          const_cast<void*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
