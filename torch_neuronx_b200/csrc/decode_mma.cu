@@ -106,25 +106,45 @@ template <bool BF16> __device__ __forceinline__ uint16_t f32_to_half(float x) {
   if (BF16) return __bfloat16_as_ushort(__float2bfloat16_rn(x));
   return __half_as_ushort(__float2half_rn(x));
 }
-// Rotary embedding of element `col` of a row: the partner element and the angle index.
-template <int D> __device__ __forceinline__ void rope_partner(int col, bool interleaved, int* partner, int* angle, float* sign) {
-  if (interleaved) {
-    *partner = col ^ 1;
-    *angle = col >> 1;
-    *sign = (col & 1) ? 1.f : -1.f;
-  } else {
-    *partner = col < D / 2 ? col + D / 2 : col - D / 2;
-    *angle = col < D / 2 ? col : col - D / 2;
-    *sign = col < D / 2 ? -1.f : 1.f;
-  }
-}
-
 // Row of the cos/sin tables for the token being decoded: its position is the sequence's old length;
 // a length beyond the tables uses their last row (never a read past the end).
 __device__ __forceinline__ int rope_row(const Problem& p, int b) {
   int len = p.kv_lens[b];
   len = len < 0 ? 0 : len;
   return len < p.rope_positions ? len : p.rope_positions - 1;
+}
+
+// Rotary embedding of the eight elements x of chunk `ch` of a row, at this step's position, in fp32 and rounded once:
+// x[c] cos + sign x[partner] sin.  Pairs are (2i, 2i + 1), inside the chunk, or (i, i + D / 2), in the chunk half a
+// row away, which `chunk8` fetches.
+template <int D, bool BF16, typename F>
+__device__ __forceinline__ void rotate8(const Problem& p, int b, int ch, uint16_t (&x)[8], F chunk8) {
+  constexpr int kHalf = D / 16;   // chunks in half a row
+  const int64_t at = static_cast<int64_t>(rope_row(p, b)) * p.rope_stride;
+  uint16_t rot[8];
+  if (p.rope_interleaved != 0) {
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      const int a = (ch * 8 + e) >> 1;
+      const float cs = p.rope_cos[at + a], sn = p.rope_sin[at + a];
+      const float x0 = half_to_f32<BF16>(x[e]), x1 = half_to_f32<BF16>(x[e + 1]);
+      rot[e] = f32_to_half<BF16>(fmaf(-x1, sn, x0 * cs));
+      rot[e + 1] = f32_to_half<BF16>(fmaf(x0, sn, x1 * cs));
+    }
+  } else {
+    const bool lo = ch < kHalf;
+    __align__(16) uint16_t y[8];
+    chunk8(lo ? ch + kHalf : ch - kHalf, y);
+    const float* cs = p.rope_cos + at + (lo ? ch : ch - kHalf) * 8;
+    const float* sn = p.rope_sin + at + (lo ? ch : ch - kHalf) * 8;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float part = half_to_f32<BF16>(y[e]);
+      rot[e] = f32_to_half<BF16>(fmaf(lo ? -part : part, sn[e], half_to_f32<BF16>(x[e]) * cs[e]));
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) x[e] = rot[e];
 }
 
 template <int D, bool BF16, bool PAGED, bool APPEND, bool ROPE>
@@ -142,6 +162,7 @@ __global__ void __launch_bounds__(kThreads, 3) decode_mma_kernel(const Problem p
   const int hk = blockIdx.x % p.Hkv;
   const int gsub = blockIdx.x / p.Hkv;
   const int b = blockIdx.y;
+  pdl_wait();
   const int n_keys = valid_keys(p, b);
   const int s0 = split * chunk;
   if (s0 >= n_keys && split != 0) return;  // split 0 still writes an (empty) partial
@@ -153,45 +174,6 @@ __global__ void __launch_bounds__(kThreads, 3) decode_mma_kernel(const Problem p
   const int h0 = hk * p.group + gsub * 16;          // first query head of this CTA
   const int n_heads = (p.group - gsub * 16) < 16 ? (p.group - gsub * 16) : 16;
   const bool row_lo = g < n_heads, row_hi = g + 8 < n_heads;
-
-  // ---- Q fragments (A operand), rows = query heads, zero for padding rows
-  uint32_t qf[KS][4];
-  {
-    const uint16_t* q16 = reinterpret_cast<const uint16_t*>(p.q);
-    const int64_t base = b * p.qs[0];
-#pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int row = g + (r & 1) * 8;
-        const int col = ks * 16 + tq * 2 + (r >> 1) * 8;
-        uint32_t v = 0;
-        if (row < n_heads) {
-          const int64_t o = base + (h0 + row) * p.qs[1] + col * p.qs[3];
-          if (ROPE) {
-            // out[c] = x[c] cos + sign x[partner] sin at this step's position, in fp32, rounded once
-            const int at = rope_row(p, b);
-            const float* cs = p.rope_cos + static_cast<int64_t>(at) * p.rope_stride;
-            const float* sn = p.rope_sin + static_cast<int64_t>(at) * p.rope_stride;
-            uint16_t outv[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              int partner, angle;
-              float sign;
-              rope_partner<D>(col + e, p.rope_interleaved != 0, &partner, &angle, &sign);
-              const float x = half_to_f32<BF16>(q16[o + e * p.qs[3]]);
-              const float y = half_to_f32<BF16>(q16[o + (partner - col) * p.qs[3]]);
-              outv[e] = f32_to_half<BF16>(fmaf(sign * y, sn[angle], x * cs[angle]));
-            }
-            v = static_cast<uint32_t>(outv[0]) | (static_cast<uint32_t>(outv[1]) << 16);
-          } else {
-            v = static_cast<uint32_t>(q16[o]) | (static_cast<uint32_t>(q16[o + p.qs[3]]) << 16);
-          }
-        }
-        qf[ks][r] = v;
-      }
-    }
-  }
 
   // ---- cache block loader: 64 keys of K and of V -> one ring stage
   // dense cache: (batch, head, row, element) strides; paged cache: (page, head, row-in-page, element)
@@ -221,21 +203,35 @@ __global__ void __launch_bounds__(kThreads, 3) decode_mma_kernel(const Problem p
     vnew = reinterpret_cast<const char*>(p.v_new) + (b * p.vns[0] + hk * p.vns[1]) * 2;
   }
   const uint32_t smem_base = smem_addr(smem);
+  // Pages of the rows this thread copies in one block.  They are looked up one block ahead, so that the table's
+  // latency passes under the block in flight instead of in front of its copies.
+  constexpr int kCopies = kBlockKeys * G::kChunksPerRow / kThreads;
+  int pages[PAGED ? kCopies : 1];
+  auto fetch_pages = [&](int blk) {
+    if constexpr (PAGED) {
+#pragma unroll
+      for (int i = 0; i < kCopies; ++i) {
+        const int row = s0 + blk * kBlockKeys + (tid + i * kThreads) / G::kChunksPerRow;
+        const int srow = row < s1 ? row : s0;
+        // (checked build: the block-table slot of this row exists; page numbers themselves are the caller's)
+        pages[i] = dbg_range(p.status, DBG_DECODE_MMA * 100 + 1, srow >> p.page_shift, 1, p.table_stride)
+                       ? table[srow >> p.page_shift]
+                       : 0;
+      }
+    }
+  };
   auto load_block = [&](int blk) {
     const uint32_t stage = smem_base + (blk % kStages) * G::kStageBytes;
     const int key0 = s0 + blk * kBlockKeys;
 #pragma unroll
-    for (int i = 0; i < kBlockKeys * G::kChunksPerRow / kThreads; ++i) {
+    for (int i = 0; i < kCopies; ++i) {
       const int c = tid + i * kThreads;
       const int row = c / G::kChunksPerRow, ch = c % G::kChunksPerRow;
       const bool ok = key0 + row < s1;
       const int srow = ok ? key0 + row : s0;
       int64_t k_off, v_off;
       if (PAGED) {
-        // (checked build: the block-table slot of this row exists; page numbers themselves are the caller's)
-        const int64_t page = dbg_range(p.status, DBG_DECODE_MMA * 100 + 1, srow >> p.page_shift, 1, p.table_stride)
-                                 ? table[srow >> p.page_shift]
-                                 : 0;
+        const int64_t page = pages[i];
         const int in_page = srow & page_mask;
         k_off = (page * p.ks[0]) * 2 + in_page * k_row;
         v_off = (page * p.vs[0]) * 2 + in_page * v_row;
@@ -250,24 +246,12 @@ __global__ void __launch_bounds__(kThreads, 3) decode_mma_kernel(const Problem p
         uint4 kq = *reinterpret_cast<const uint4*>(knew + ch * 16);
         const uint4 vq = *reinterpret_cast<const uint4*>(vnew + ch * 16);
         if (ROPE) {
-          // rotate the eight elements of this chunk (their partners sit in this chunk or in one other)
-          const int at = rope_row(p, b);
-          const float* cs = p.rope_cos + static_cast<int64_t>(at) * p.rope_stride;
-          const float* sn = p.rope_sin + static_cast<int64_t>(at) * p.rope_stride;
-          const uint16_t* row16 = reinterpret_cast<const uint16_t*>(knew);
-          uint16_t* kv16 = reinterpret_cast<uint16_t*>(&kq);
-          uint16_t rot[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            int partner, angle;
-            float sign;
-            rope_partner<D>(ch * 8 + e, p.rope_interleaved != 0, &partner, &angle, &sign);
-            const float x = half_to_f32<BF16>(kv16[e]);
-            const float y = half_to_f32<BF16>(row16[partner]);
-            rot[e] = f32_to_half<BF16>(fmaf(sign * y, sn[angle], x * cs[angle]));
-          }
-#pragma unroll
-          for (int e = 0; e < 8; ++e) kv16[e] = rot[e];
+          __align__(16) uint16_t x[8];
+          *reinterpret_cast<uint4*>(x) = kq;
+          rotate8<D, BF16>(p, b, ch, x, [&](int at, uint16_t (&y)[8]) {
+            *reinterpret_cast<uint4*>(y) = *reinterpret_cast<const uint4*>(knew + at * 16);
+          });
+          kq = *reinterpret_cast<const uint4*>(x);
           // the rotated chunk goes to shared memory by a plain store (visible after the block barrier
           // that follows the copy wait) instead of an asynchronous copy from k_new
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + row * G::kRowBytes + ch * 16), "r"(kq.x),
@@ -297,15 +281,51 @@ __global__ void __launch_bounds__(kThreads, 3) decode_mma_kernel(const Problem p
   float l_lo = 0.f, l_hi = 0.f;                       // this lane's share of the row sums
   const float sl2 = p.scale * kLog2e;
 
+  static_assert(kStages == 2, "the query rows are staged in the second stage before its first block arrives");
+  if (n_blocks > 0) {
+    fetch_pages(0);
+    load_block(0);
+  }
+  cp_async_commit();
+  if (n_blocks > 1) fetch_pages(1);
+
+  // ---- Q fragments (A operand; rows = query heads, padding rows zero): the rows go through the second stage with
+  // 16-byte loads while the first block travels, and are rotated there
+  uint32_t qf[KS][4];
+  {
+    const uint16_t* q16 = reinterpret_cast<const uint16_t*>(p.q) + b * p.qs[0];
+    uint8_t* stage = smem + G::kStageBytes;
+    const bool vec = p.qs[3] == 1 && reinterpret_cast<uintptr_t>(p.q) % 16 == 0 && p.qs[0] % 8 == 0 && p.qs[1] % 8 == 0;
+    for (int c = tid; c < 16 * G::kChunksPerRow; c += kThreads) {
+      const int row = c / G::kChunksPerRow, ch = c % G::kChunksPerRow;
+      const uint16_t* src = q16 + (h0 + row) * p.qs[1];
+      auto chunk8 = [&](int at, uint16_t (&x)[8]) {
+        if (vec) {
+          *reinterpret_cast<uint4*>(x) = *reinterpret_cast<const uint4*>(src + at * 8);
+        } else {
 #pragma unroll
-  for (int s = 0; s < kStages - 1; ++s) {
-    if (s < n_blocks) load_block(s);
-    cp_async_commit();
+          for (int e = 0; e < 8; ++e) x[e] = src[(at * 8 + e) * p.qs[3]];
+        }
+      };
+      __align__(16) uint16_t x[8] = {};
+      if (row < n_heads) {
+        chunk8(ch, x);
+        if (ROPE) rotate8<D, BF16>(p, b, ch, x, chunk8);
+      }
+      *reinterpret_cast<uint4*>(stage + row * G::kRowBytes + ch * 16) = *reinterpret_cast<const uint4*>(x);
+    }
+    __syncthreads();
+    // matrices = (heads 0-7, d lo), (heads 8-15, d lo), (heads 0-7, d hi), (heads 8-15, d hi)
+    const uint32_t a0 = smem_base + G::kStageBytes + ((lane & 7) + ((lane >> 3) & 1) * 8) * G::kRowBytes + (lane >> 4) * 16;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) ldsm_x4(a0 + ks * 32, qf[ks]);
+    __syncthreads();
   }
 
   for (int blk = 0; blk < n_blocks; ++blk) {
     if (blk + kStages - 1 < n_blocks) load_block(blk + kStages - 1);
     cp_async_commit();
+    if (blk + kStages < n_blocks) fetch_pages(blk + kStages);
     cp_async_wait<kStages - 1>();
     __syncthreads();
 
@@ -395,7 +415,7 @@ __global__ void __launch_bounds__(kThreads, 3) decode_mma_kernel(const Problem p
   cp_async_wait<0>();
   // the cache has been streamed: the combine kernel (a programmatic dependent launch) may be placed now;
   // it still waits for this grid to complete before it reads a partial
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_launch_dependents();
 
   // ---- quad-reduce the row sums, then merge the four warps through shared memory
   l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
@@ -454,8 +474,7 @@ int launch_one(const Problem& p, int chunk, int nsplit, float* po, float* pml, c
   }
   const int nsub = (p.group + 15) / 16;
   dim3 grid(p.Hkv * nsub, p.B, nsplit);
-  kern<<<grid, kThreads, G::kSmemBytes, stream>>>(p, chunk, nsplit, po, pml);
-  if (cudaGetLastError() != cudaSuccess) return B200_SDPA_ERR_CUDA;
+  if (!launch_pdl(kern, grid, kThreads, G::kSmemBytes, stream, p, chunk, nsplit, po, pml)) return B200_SDPA_ERR_CUDA;
   count_launch(KID_DECODE);
   return B200_SDPA_OK;
 }

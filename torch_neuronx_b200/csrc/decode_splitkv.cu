@@ -221,53 +221,107 @@ __global__ void __launch_bounds__(kThreads) decode_partial_kernel(const Problem 
   }
 }
 
+// Merge of the partials: one CTA of four warps per (batch, query head).  Every warp takes every fourth split (the
+// (max, sum) pairs of all splits are read once, 32 at a time), then the four states meet in shared memory.  Bound by
+// latency: two dependent rounds of loads, whatever the number of splits up to 128.
+constexpr int kCombineWarps = 4;
+
 template <typename T, int D>
-__global__ void __launch_bounds__(D) decode_combine_kernel(const Problem p, const int chunk, const int nsplit,
-                                                           const float* __restrict__ part_o,
-                                                           const float* __restrict__ part_ml) {
+__global__ void __launch_bounds__(kCombineWarps * 32) decode_combine_kernel(const Problem p, const int chunk, const int nsplit,
+                                                                            const float* __restrict__ part_o,
+                                                                            const float* __restrict__ part_ml) {
+  constexpr int C = D / 32;   // columns per lane
+  __shared__ float sm_o[kCombineWarps][D];
+  __shared__ float sm_l[kCombineWarps];
   const int h = blockIdx.x % p.Hq;
   const int b = blockIdx.x / p.Hq;
-  const int d = threadIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // launched as a programmatic dependent of the partial kernel: nothing may be read before it has completed
+  pdl_wait();
+  pdl_launch_dependents();
   const int n_keys = valid_keys(p, b);
-  // launched as a programmatic dependent of the partial kernel: nothing that kernel wrote may be read
-  // before it has completed
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (p.lens_out != nullptr && h == 0 && d == 0) p.lens_out[b] = n_keys;   // lengths after the append
+  if (p.lens_out != nullptr && h == 0 && threadIdx.x == 0) p.lens_out[b] = n_keys;   // lengths after the append
   int used = (n_keys + chunk - 1) / chunk;
   used = used < 1 ? 1 : (used > nsplit ? nsplit : used);
   const int64_t slot0 = (static_cast<int64_t>(b) * p.Hq + h) * nsplit;
   if (!dbg_range(p.status, DBG_DECODE_SIMT * 100 + 3, slot0, used, static_cast<int64_t>(p.B) * p.Hq * nsplit) ||
-      !dbg_bhrc(p.status, DBG_DECODE_SIMT * 100 + 4, b, p.B, h, p.Hq, 0, 1, d, 1, p.Dv))
+      !dbg_bhrc(p.status, DBG_DECODE_SIMT * 100 + 4, b, p.B, h, p.Hq, 0, 1, lane * C, C, p.Dv))
     return;
   float mx = -CUDART_INF_F;
-  for (int s = 0; s < used; ++s) mx = fmaxf(mx, part_ml[(slot0 + s) * 2]);
+  for (int s = lane; s < used; s += 32) mx = fmaxf(mx, part_ml[(slot0 + s) * 2]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   const float ms = (mx == -CUDART_INF_F) ? 0.f : mx;
-  float o = 0.f, lsum = 0.f;
-  for (int s = 0; s < used; ++s) {
-    const float w = exp2f(part_ml[(slot0 + s) * 2] - ms);
-    lsum = fmaf(part_ml[(slot0 + s) * 2 + 1], w, lsum);
-    o = fmaf(part_o[(slot0 + s) * D + d], w, o);
+  float acc[C], lsum = 0.f;
+#pragma unroll
+  for (int c = 0; c < C; ++c) acc[c] = 0.f;
+#pragma unroll 4
+  for (int s = warp; s < used; s += kCombineWarps) {
+    const float2 ml = *reinterpret_cast<const float2*>(part_ml + (slot0 + s) * 2);
+    const float* src = part_o + (slot0 + s) * D + lane * C;
+    float v[C];
+    if constexpr (C == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src);
+    else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(src);
+    const float w = exp2f(ml.x - ms);
+    lsum = fmaf(ml.y, w, lsum);
+#pragma unroll
+    for (int c = 0; c < C; ++c) acc[c] = fmaf(v[c], w, acc[c]);
   }
-  const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
-  T* out = reinterpret_cast<T*>(p.out);
-  out[b * p.os[0] + h * p.os[1] + d * p.os[3]] = from_f32<T>(o * inv);
-  if (p.lse != nullptr && d == 0)
-    p.lse[b * p.ls[0] + h * p.ls[1]] = (mx == -CUDART_INF_F) ? -CUDART_INF_F : fmaf(mx, kLn2, logf(lsum));
+#pragma unroll
+  for (int c = 0; c < C; ++c) sm_o[warp][lane * C + c] = acc[c];
+  if (lane == 0) sm_l[warp] = lsum;
+  __syncthreads();
+  float l = 0.f;
+#pragma unroll
+  for (int w = 0; w < kCombineWarps; ++w) l += sm_l[w];
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+  for (int d = threadIdx.x; d < D; d += kCombineWarps * 32) {
+    float o = 0.f;
+#pragma unroll
+    for (int w = 0; w < kCombineWarps; ++w) o += sm_o[w][d];
+    reinterpret_cast<T*>(p.out)[b * p.os[0] + h * p.os[1] + d * p.os[3]] = from_f32<T>(o * inv);
+  }
+  if (p.lse != nullptr && threadIdx.x == 0)
+    p.lse[b * p.ls[0] + h * p.ls[1]] = (mx == -CUDART_INF_F) ? -CUDART_INF_F : fmaf(mx, kLn2, logf(l));
 }
 
 int pick_group(int group) { return group >= 8 ? 8 : group > 2 ? 4 : group; }
 
+// Keys per CTA.  A model of the launch, fitted to measurements (bf16, head dimension 128, 1 to 128 sequences of 512 to
+// 32768 keys, within a tenth of the best chunk everywhere): up to kSlots CTAs run at a time; a CTA needs kFixed for its
+// start and end and, per block of 64 keys, kBlock alone (the latency of its two-stage ring) and kShared more when all
+// slots are taken (its share of the HBM rate).  Short chunks pay kFixed too often, long ones leave SMs without work.
+// More CTAs than slots cost, on average, a third of a round for the last, partly filled one -- less when their lengths
+// differ.  Lengths are not known here: with key lengths the cost for full caches and twice that for lengths spread
+// evenly up to S are added, else full caches are assumed.  A paged cache's block costs more alone (table and address
+// arithmetic).  16 sequences of 128..4000 keys, 4096 cached, 32/8 heads: 34.9 us at the 256 keys taken before, 32.3 at
+// the 1024 taken now (paged, with append: 41.1 -> 33.5 at 768); one sequence of 30000 keys 41.2 -> 31.8.
 int default_chunk(const Problem& p) {
-  // Enough CTAs to fill 148 SMs several times over even when half the splits of
-  // a ragged batch are empty, but never chunks so small that the per-CTA
-  // epilogue shows.
-  const int64_t units = static_cast<int64_t>(p.B) * p.Hkv;
-  int64_t want = (148LL * 16 + units - 1) / units;   // splits per (batch, kv head)
-  int64_t chunk = (p.S + want - 1) / want;
-  chunk = (chunk + 127) / 128 * 128;
-  if (chunk < 256) chunk = 256;
-  if (chunk > 2048) chunk = 2048;
-  return static_cast<int>(chunk);
+  constexpr double kSlots = 444, kFixed = 3.5;        // us
+  const double block = p.block_table != nullptr ? 1.12 : 0.71;
+  const int sub = (p.group + 15) / 16;
+  const double shared = 1.6 * (p.E + p.Dv) / 256.0;
+  const double units = static_cast<double>(p.B) * p.Hkv * sub;
+  auto launch_us = [&](double ctas, int chunk, bool ragged) {
+    const double blocks = chunk / 64.0, fill = ctas / kSlots;
+    if (fill <= 1.0) return kFixed + blocks * (block + shared * fill);
+    const double over = ragged && fill < 4.0 / 3.0 ? 3.0 * (fill - 1.0) : 1.0;
+    return (fill + 0.35 * over) * (kFixed + blocks * (block + shared));
+  };
+  int best = 256;
+  double best_us = 1e30;
+  for (int chunk = 64; chunk <= 2048; chunk += chunk < 512 ? 64 : 256) {
+    const int n = (p.S + chunk - 1) / chunk;
+    double t = launch_us(units * n, chunk, false);
+    if (p.kv_lens != nullptr) t += 2 * launch_us(units * (n + 1) / 2, chunk, true);
+    t *= 1.0 + 0.002 * n;   // equal: fewer partials
+    if (t < best_us) {
+      best_us = t;
+      best = chunk;
+    }
+    if (chunk >= p.S) break;
+  }
+  return best;
 }
 
 struct DecodeGeom {
@@ -288,25 +342,8 @@ DecodeGeom geometry(const Problem& p, int kv_chunk) {
 
 template <typename T, int D>
 int launch_combine(const Problem& p, const DecodeGeom& gm, float* po, float* pml, cudaStream_t stream) {
-  // Programmatic dependent launch: the combine grid may be placed while the partial kernel's last CTAs
-  // are finishing; its threads wait (griddepcontrol.wait) until that grid has completed and its stores
-  // are visible before they read a partial.
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.B * p.Hq);
-  cfg.blockDim = dim3(D);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const float* cpo = po;
-  const float* cpml = pml;
-  if (cudaLaunchKernelEx(&cfg, decode_combine_kernel<T, D>, p, gm.chunk, gm.nsplit, cpo, cpml) != cudaSuccess) {
-    cudaGetLastError();
+  if (!launch_pdl(decode_combine_kernel<T, D>, dim3(p.B * p.Hq), kCombineWarps * 32, 0, stream, p, gm.chunk, gm.nsplit, po, pml))
     return B200_SDPA_ERR_CUDA;
-  }
   count_launch(KID_COMBINE);
   return B200_SDPA_OK;
 }
