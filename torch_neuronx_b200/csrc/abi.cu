@@ -151,6 +151,14 @@ bool served_padded(const B200SdpaBwdParams* a, const BwdProblem& bp) {
   return a->force_path != B200_SDPA_PATH_GENERIC && bwd_padded_eligible(bp, a->dtype);
 }
 
+// ... and the tiled fp32 kernels what fits their layout.
+bool served_fp32(const B200SdpaParams* a, const Problem& p) {
+  return a->force_path != B200_SDPA_PATH_GENERIC && fp32_fwd_eligible(p, a->dtype);
+}
+bool served_fp32(const B200SdpaBwdParams* a, const BwdProblem& bp) {
+  return a->force_path != B200_SDPA_PATH_GENERIC && fp32_bwd_eligible(bp, a->dtype);
+}
+
 // Makes the requested device current for the duration of one entry point and puts the caller's
 // device back afterwards (a library call must not change which device the host thread is on).
 // Also the one place that checks the compute capability: every kernel here is sm_100a code.
@@ -346,6 +354,10 @@ int b200_sdpa_query_plan(const B200SdpaParams* params, B200SdpaPlan* plan) {
     plan->path = B200_SDPA_PATH_GENERIC;
     return rc;
   }
+  if (served_fp32(params, p)) {
+    plan_fp32_fwd(p, plan);
+    return B200_SDPA_OK;
+  }
   return plan_generic(p, params->dtype, plan);
 }
 
@@ -372,6 +384,7 @@ int b200_sdpa_fwd(const B200SdpaParams* params, void* stream) {
   }
   if (path == B200_SDPA_PATH_PREFILL) return launch_prefill(p, params->dtype, params->workspace, params->workspace_bytes, st);
   if (served_padded(params, p)) return launch_prefill_padded(p, params->dtype, st);
+  if (served_fp32(params, p)) return launch_fp32_fwd(p, st);
   return launch_generic(p, params->dtype, st);
 }
 
@@ -411,6 +424,10 @@ int b200_sdpa_bwd_query_plan(const B200SdpaBwdParams* a, B200SdpaPlan* plan) {
     plan->path = B200_SDPA_PATH_GENERIC;
     return rc;
   }
+  if (served_fp32(a, bp)) {
+    plan_fp32_bwd(bp, plan);
+    return B200_SDPA_OK;
+  }
   return plan_bwd_generic(bp, a->dtype, plan);
 }
 
@@ -429,6 +446,7 @@ int b200_sdpa_bwd(const B200SdpaBwdParams* a, void* stream) {
     // without scratch an automatic choice falls through to the kernels that need none
     if (rc != B200_SDPA_ERR_WORKSPACE || a->force_path == B200_SDPA_PATH_PREFILL) return rc;
   }
+  if (served_fp32(a, bp)) return launch_fp32_bwd(bp, st);
   return launch_bwd_generic(bp, a->dtype, st);
 }
 

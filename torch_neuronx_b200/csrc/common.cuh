@@ -87,6 +87,14 @@ enum KernelId {
 
 // Host launchers implemented in the per-kernel translation units.  Each returns
 // a b200_sdpa_status and never synchronises.
+// fp32, head dimension 64 or 128, aligned rows, no bias (fp32_sm100.cu); part of the generic path
+bool fp32_fwd_eligible(const Problem& p, int dtype);
+bool fp32_bwd_eligible(const BwdProblem& bp, int dtype);
+void plan_fp32_fwd(const Problem& p, B200SdpaPlan* plan);
+void plan_fp32_bwd(const BwdProblem& bp, B200SdpaPlan* plan);
+int launch_fp32_fwd(const Problem& p, cudaStream_t stream);
+int launch_fp32_bwd(const BwdProblem& bp, cudaStream_t stream);
+
 int launch_generic(const Problem& p, int dtype, cudaStream_t stream);
 int plan_generic(const Problem& p, int dtype, B200SdpaPlan* plan);
 

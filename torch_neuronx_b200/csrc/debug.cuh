@@ -29,7 +29,8 @@ enum DebugFile {
   DBG_PREFILL_PERSISTENT = 6,
   DBG_PREFILL_WIDE = 7,
   DBG_BWD_TC = 8,
-  DBG_BWD_WIDE = 9
+  DBG_BWD_WIDE = 9,
+  DBG_FP32 = 10
 };
 
 __device__ __forceinline__ bool dbg_fail(int* status, int site, long long index, long long limit) {
