@@ -122,7 +122,9 @@ struct PackArgs {
 
 // PAD: head dimensions E, Dv (multiples of 8) that do not fill the D = 128 tile.  The tensor maps carry the
 // real extents, so the copies fill the tile's remaining columns with zeros and the output store clips them;
-// the products run over ceil(E / 16) k-steps and ceil(Dv / 16) * 16 output columns only.
+// the products run over ceil(E / 16) k-steps and ceil(Dv / 16) * 16 output columns only.  These shapes had fp32
+// probabilities on the CUDA-core kernel, so P goes into the second product as hi + lo (remainder2), lo in the second
+// half of the columns of S.
 template <int D, bool BF16, bool BIAS, bool ACC, bool PAD, bool PACK>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -352,6 +354,8 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           for (int kk = 0; kk < 4; ++kk) {
             mma_ts(d_addr, a_addr + static_cast<uint32_t>(kk * 8), vd + static_cast<uint64_t>(kk * (2048 >> 4)), idesc_pv,
                    kk > 0 ? 1u : acc0);
+            if (PAD)
+              mma_ts(d_addr, a_addr + static_cast<uint32_t>(64 + kk * 8), vd + static_cast<uint64_t>(kk * (2048 >> 4)), idesc_pv, 1u);
           }
         }
       };
@@ -652,15 +656,17 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         uint64_t sum2[2] = {0ull, 0ull};           // two packed accumulators = four chains
 #pragma unroll
         for (int c = 0; c < kBlockN / 32; ++c) {
-          uint32_t pk[16];
+          uint32_t pk[16], lo[PAD ? 16 : 1];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
             const float p0 = ex2(fmaf(__uint_as_float(sv[c * 32 + i]), sl2, nms));
             const float p1 = ex2(fmaf(__uint_as_float(sv[c * 32 + i + 1]), sl2, nms));
             sum2[(i >> 1) & 1] = f2_add(sum2[(i >> 1) & 1], f2_pack(p0, p1));
             pk[i >> 1] = pack2<BF16>(p0, p1);
+            if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(p0, p1, pk[i >> 1]);
           }
           tmem_st_32x16(p_addr + c * 16, pk);
+          if constexpr (PAD) tmem_st_32x16(p_addr + 64 + c * 16, lo);
           if (c == 1) {
             // first 64 keys of P are in TMEM: let P V start on them while the rest is computed
             tmem_st_wait();
@@ -1097,7 +1103,7 @@ bool prefill_eligible(const Problem& p, int dtype, bool* alignment_only_failure)
 // Head dimensions between 64 and 128 (multiples of 8, so that rows stay on the 16-byte grid of a tensor copy):
 // 128-wide tiles with zero-filled columns.  Below 64 the exponentials bound a tile whatever its head dimension
 // and the requests are small; those keep the CUDA-core kernel.  Measured (fp16, 16 x 16 heads x 577 x 577, head
-// dimension 80): CUDA-core kernel 2463 us, these tiles 86 us.
+// dimension 80): CUDA-core kernel 2463 us, these tiles 79 us with a 16-bit P, 92 us with hi + lo.
 bool prefill_padded_eligible(const Problem& p, int dtype) {
   const int hi = p.E > p.Dv ? p.E : p.Dv;
   if (hi <= 64 || hi > 128 || p.E % 8 != 0 || p.Dv % 8 != 0) return false;

@@ -193,6 +193,23 @@ inline bool strides_ok(const void* base, const int64_t* s, int rows, int heads, 
   return true;
 }
 
+// What rounding (x0, x1) to the 16-bit pair `hi` left over, rounded to 16 bits itself.  Where a shape was served with
+// fp32 probabilities before, the second product takes both parts, hi + lo, as two operands: 2^-16 (bf16) or 2^-22
+// (fp16) of the value is lost, far below the rounding of the result.
+template <bool BF16>
+__device__ __forceinline__ uint32_t remainder2(float x0, float x1, uint32_t hi) {
+  float h0, h1;
+  if (BF16) {
+    h0 = __uint_as_float(hi << 16);
+    h1 = __uint_as_float(hi & 0xffff0000u);
+  } else {
+    const float2 h = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+    h0 = h.x;
+    h1 = h.y;
+  }
+  return pack2<BF16>(x0 - h0, x1 - h1);
+}
+
 // One thread's 8 N bias elements (16-bit) of a key tile: N 16-byte pieces, fetched as N / 2
 // 32-byte loads when the row allows it (`wide`: the row start and the key offset on a 32-byte
 // boundary) -- every thread reads its own row, so the number of load instructions is what the
