@@ -25,33 +25,33 @@ __device__ __forceinline__ uint64_t kmajor_step(int kk) {
 __device__ __forceinline__ uint64_t mnmajor_desc(uint32_t tile) { return smem_desc_sw128(tile, kBoxBytes, 1024); }
 __device__ __forceinline__ uint64_t mnmajor_step(int kk) { return static_cast<uint64_t>(kk * (2048 >> 4)); }
 
-// One thread's accumulator row (TMEM lane) -> 16-bit -> the 128-byte-swizzled staging
-// tile a TMA store expects.
-template <int D, bool BF16>
-__device__ __forceinline__ void stage_row(uint32_t acc_addr, bool have_acc, float mul, uint8_t* stage, int r,
-                                          int half) {
-  // the two threads of a lane share the row: D/64 chunks of 32 columns each
+// One arrival for a warp whose lanes have all done what the barrier stands for.
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+  __syncwarp();
+  if (lane == 0) mbar_arrive(smem_u32(bar));
+}
+
+// 32 columns (chunk c) of one thread's accumulator row (TMEM lane) -> 16-bit -> the 128-byte-swizzled staging tile a
+// TMA store expects.
+template <bool BF16>
+__device__ __forceinline__ void stage_chunk(uint32_t acc_addr, bool have_acc, float mul, uint8_t* stage, int r, int c) {
+  uint32_t v[32];
+  if (have_acc) {
+    tmem_ld_32x32(acc_addr + c * 32, v);
+    tmem_ld_wait();
+  } else {
 #pragma unroll
-  for (int cc = 0; cc < D / 64; ++cc) {
-    const int c = half * (D / 64) + cc;
-    uint32_t v[32];
-    if (have_acc) {
-      tmem_ld_32x32(acc_addr + c * 32, v);
-      tmem_ld_wait();
-    } else {
+    for (int i = 0; i < 32; ++i) v[i] = 0u;
+  }
+  uint32_t pk[16];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = 0u;
-    }
-    uint32_t pk[16];
+  for (int i = 0; i < 32; i += 2)
+    pk[i >> 1] = pack2<BF16>(__uint_as_float(v[i]) * mul, __uint_as_float(v[i + 1]) * mul);
+  uint8_t* box = stage + (c >> 1) * kBoxBytes + r * 128;
 #pragma unroll
-    for (int i = 0; i < 32; i += 2)
-      pk[i >> 1] = pack2<BF16>(__uint_as_float(v[i]) * mul, __uint_as_float(v[i + 1]) * mul);
-    uint8_t* box = stage + (c >> 1) * kBoxBytes + r * 128;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int unit = ((c & 1) * 4 + u) ^ (r & 7);
-      *reinterpret_cast<uint4*>(box + unit * 16) = make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
-    }
+  for (int u = 0; u < 4; ++u) {
+    const int unit = ((c & 1) * 4 + u) ^ (r & 7);
+    *reinterpret_cast<uint4*>(box + unit * 16) = make_uint4(pk[4 * u], pk[4 * u + 1], pk[4 * u + 2], pk[4 * u + 3]);
   }
 }
 

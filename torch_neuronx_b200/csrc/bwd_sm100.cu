@@ -19,18 +19,22 @@
 // in exchange dQ needs neither atomics nor an fp32 scratch tensor, and results are
 // deterministic.  Arithmetic: torch_neuronx/_sdpa_math.py:133-176 with P and dS rounded
 // to the input dtype before their second product (upstream rounds P the same way in the
-// forward, :94).  Roles per CTA (320 threads): warps 0-7 elementwise (two threads per TMEM
-// lane), warp 8 TMA producer, warp 9 MMA issuer.
+// forward, :94).  Roles per CTA (576 threads): warps 0-15 elementwise (four threads per TMEM
+// lane, 32 score columns each: four warps per scheduler hide one another's tensor-memory and
+// barrier latency), warp 16 TMA producer, warp 17 MMA issuer.
 //
-// The dK/dV kernel works in units of 64 score columns (half an operand tile) with the two
-// score-shaped accumulators double-buffered in tensor memory, so the elementwise role works
-// on unit u+1 while the tensor cores run the accumulating products of unit u and the score
-// products of unit u+2 (the MMA pipe executes in issue order, which makes "scores of u+2
-// after the accumulating products of u" safe on the shared buffer):
-//   TMEM columns  [0,64) [64,128)  S^T buffers 0/1   [128,192) [192,256)  dP^T buffers 0/1
-//                 [256, 256+2D)    dV and dK (fp32)
-// Its tensor memory is full with that; the dQ kernel has one accumulator less and works on
-// whole 128-column tiles instead (layout and pipeline described at the kernel).
+// The dK/dV kernel's tensor memory is full with one pair of score-shaped accumulators:
+//   TMEM columns  [0,128) S^T, P^T over it   [128,256) dP^T, dS^T over it   [256, 256+2D) dV and dK (fp32)
+// and still neither role waits for the other for long, because the two halves of a tile's
+// arithmetic alternate with two groups of products (in issue order, which is also the order
+// in which the MMA pipe touches the shared columns):
+//   elementwise  P^T(i) from S^T(i)        dS^T(i) from P^T(i), dP^T(i)
+//   MMA          dK(i-1), dP^T(i)          dV(i), S^T(i+1)
+// Whole 128-row query tiles: a score product with 64 columns costs the tensor pipe as much as one with 128 (its A
+// operand is fetched from shared memory either way).  Measured, 1 x 32/8 x 4096, no mask: 3350 cycles per tile against
+// 4024 for two 64-column units, of which the products take 2048 and the exponentials 1024 of the MUFU.
+// The dQ kernel has one accumulator less and releases its scores as soon as they are in registers
+// (layout and pipeline described at the kernel).
 // Every wait is bounded (see tc_common.cuh).
 #include "bwd_common.cuh"
 
@@ -41,12 +45,12 @@ namespace {
 using namespace ptx;
 using namespace tc;
 
-constexpr int kThreads = 320;
-constexpr int kEThreads = 256;            // elementwise role: two column halves x 128 lanes
-constexpr int kU = 64;                    // score columns per unit
-constexpr uint32_t kColS = 0, kColDP = 128, kColAcc = 256;   // TMEM layout (buffer b at + 64 b)
-constexpr int kProducerWarp = 8;
-constexpr int kMmaWarp = 9;
+constexpr int kEWarps = 16;               // elementwise role: four column quarters x four lane quadrants
+constexpr int kQ = kT / 4;                // score columns of one thread
+constexpr int kThreads = (kEWarps + 2) * 32;
+constexpr uint32_t kColS = 0, kColDP = 128, kColAcc = 256;   // TMEM layout of the dK/dV kernel
+constexpr int kProducerWarp = kEWarps;
+constexpr int kMmaWarp = kEWarps + 1;
 constexpr uint32_t kTmemCols = 512;
 constexpr int kMaxStages = 4;
 
@@ -63,8 +67,10 @@ struct BSync {
   uint64_t fixed_full;
   uint64_t ring_full[kMaxStages];
   uint64_t ring_empty[kMaxStages];
-  uint64_t sp_full[2];  // both score-shaped accumulators of a unit are complete (per buffer)
-  uint64_t e_ready[2];  // the elementwise role has written the unit's 16-bit operands
+  uint64_t s_full;      // S^T of a tile is complete
+  uint64_t dp_full;     // dP^T of a tile is complete
+  uint64_t p_ready;     // the elementwise role has written P^T (16-bit, over S^T)
+  uint64_t ds_ready;    // ... and dS^T (over dP^T)
   uint64_t acc_done;    // last accumulating MMA has retired
   uint64_t staged;
   uint64_t drain;
@@ -124,11 +130,11 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const BwdProblem bp, floa
   }
 }
 
-// acc[tmem d, 128 x 64] = A[smem tile, K-major] * B[rows 64 hh .. 64 hh + 63 of a smem tile, K-major]^T over D
+// acc[tmem d, 128 x 128] = A[smem tile, K-major] * B[smem tile, K-major]^T over D
 // (PAD: only the first `steps` of the D / 16 k-steps, the columns beyond hold zeros)
 template <int D, bool PAD>
-__device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint32_t a_tile, uint32_t b_tile, int hh, uint32_t idesc, int steps) {
-  const uint64_t ad = kmajor_desc(a_tile), bd = kmajor_desc(b_tile + static_cast<uint32_t>(hh) * (kU * 128));
+__device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint32_t a_tile, uint32_t b_tile, uint32_t idesc, int steps) {
+  const uint64_t ad = kmajor_desc(a_tile), bd = kmajor_desc(b_tile);
   if (elect_one()) {
 #pragma unroll
     for (int kk = 0; kk < D / 16; ++kk) {
@@ -137,27 +143,30 @@ __device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint32_t a_tile, uint3
     }
   }
 }
-// acc[tmem d] (+)= A[tmem] * B[rows 64 hh .. 64 hh + 63 of a smem tile, MN-major].  The 16-bit A
-// operand sits where the two column halves of the elementwise role left it: contraction
-// indices 0-31 packed into columns [0,16) of the unit's buffer, 32-63 into columns [32,48).
-__device__ __forceinline__ void issue_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_tile, int hh, uint32_t idesc,
-                                         bool accumulate) {
-  const uint64_t bd = mnmajor_desc(b_tile) + mnmajor_step(4 * hh);
+// acc[tmem d] (+)= A[tmem, 128 x 128] * B[smem tile, MN-major].  The 16-bit A operand sits where the four column
+// quarters of the elementwise role left it: contraction indices 32 q .. 32 q + 31 packed into columns
+// [32 q, 32 q + 16) of the score-shaped buffer they came from.  PAD: the quarter's other 16 columns hold the remainders
+// of that rounding (remainder2), a second set of products.
+template <bool PAD>
+__device__ __forceinline__ void issue_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_tile, uint32_t idesc, bool accumulate) {
+  const uint64_t bd = mnmajor_desc(b_tile);
   if (elect_one()) {
 #pragma unroll
-    for (int kk = 0; kk < kU / 16; ++kk)
-      mma_ts(d_tmem, a_tmem + static_cast<uint32_t>((kk >> 1) * 32 + (kk & 1) * 8), bd + mnmajor_step(kk), idesc,
-             (kk > 0 || accumulate) ? 1u : 0u);
+    for (int kk = 0; kk < kT / 16; ++kk) {
+      const uint32_t a = a_tmem + static_cast<uint32_t>((kk >> 1) * 32 + (kk & 1) * 8);
+      mma_ts(d_tmem, a, bd + mnmajor_step(kk), idesc, (kk > 0 || accumulate) ? 1u : 0u);
+      if (PAD) mma_ts(d_tmem, a + 16, bd + mnmajor_step(kk), idesc, 1u);
+    }
   }
 }
 
 __device__ __forceinline__ void init_common_barriers(BSync* sync) {
-  for (int i = 0; i < 2; ++i) {
-    mbar_init(smem_u32(&sync->sp_full[i]), 1);
-    mbar_init(smem_u32(&sync->e_ready[i]), kEThreads);
-  }
+  mbar_init(smem_u32(&sync->s_full), 1);
+  mbar_init(smem_u32(&sync->dp_full), 1);
+  mbar_init(smem_u32(&sync->p_ready), kEWarps);
+  mbar_init(smem_u32(&sync->ds_ready), kEWarps);
   mbar_init(smem_u32(&sync->acc_done), 1);
-  mbar_init(smem_u32(&sync->staged), kEThreads);
+  mbar_init(smem_u32(&sync->staged), kEWarps);
   mbar_init(smem_u32(&sync->drain), 1);
   sync->abort_flag = 0;
   mbar_fence_init();
@@ -289,13 +298,13 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   }
   if (tid == 0) {
     mbar_init(smem_u32(&sync->sp_full), 1);
-    mbar_init(smem_u32(&sync->f_free), kEThreads);
+    mbar_init(smem_u32(&sync->f_free), kEWarps);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&sync->e_ready[i]), kEThreads);
+      mbar_init(smem_u32(&sync->e_ready[i]), kEWarps);
       mbar_init(smem_u32(&sync->op_empty[i]), 1);
     }
     mbar_init(smem_u32(&sync->acc_done), 1);
-    mbar_init(smem_u32(&sync->staged), kEThreads);
+    mbar_init(smem_u32(&sync->staged), kEWarps);
     mbar_init(smem_u32(&sync->drain), 1);
     sync->abort_flag = 0;
     mbar_fence_init();
@@ -309,6 +318,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   tc_fence_after_sync();
   const uint32_t tmem_base = sync->tmem_base;
   constexpr uint32_t kColS = 0, kColDP = 128, kColOp = 256, kColDQ = 384;
+  constexpr int kBufs = PAD ? 1 : 2;   // dS operand buffers (PAD: the second one holds the remainders, see remainder2)
 
   if (warp == kProducerWarp) {
     if (lane == 0) {
@@ -380,7 +390,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     };
     if (alive) alive = issue_scores(0);
     for (int j = 0; j < n_tiles && alive; ++j) {
-      const int buf = j & 1, ks = j % C::kKSlots;
+      const int buf = j % kBufs, ks = j % C::kKSlots;
       // S_j and dP_j are in registers: the next tile's score products may overwrite them
       alive = wait_clocked(smem_u32(&sync->f_free), j & 1, abort_flag, wait_limit);
       if (!alive) {
@@ -392,7 +402,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         alive = issue_scores(j + 1);
         if (!alive) break;
       }
-      alive = wait_clocked(smem_u32(&sync->e_ready[buf]), (j >> 1) & 1, abort_flag, wait_limit);
+      alive = wait_clocked(smem_u32(&sync->e_ready[buf]), (j / kBufs) & 1, abort_flag, wait_limit);
       if (!alive) {
         if (lane == 0) report(p.status, 13, j, 0);
         break;
@@ -401,9 +411,11 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const uint64_t bd = mnmajor_desc(k_ring + ks * C::kTileBytes);
       if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < kT / 16; ++kk)   // dQ += dS_j K_j
-          mma_ts(tmem_base + kColDQ, tmem_base + kColOp + buf * 64 + static_cast<uint32_t>(kk * 8), bd + mnmajor_step(kk),
-                 idesc_acc, (kk > 0 || j > 0) ? 1u : 0u);
+        for (int kk = 0; kk < kT / 16; ++kk) {   // dQ += dS_j K_j
+          const uint32_t a = tmem_base + kColOp + buf * 64 + static_cast<uint32_t>(kk * 8);
+          mma_ts(tmem_base + kColDQ, a, bd + mnmajor_step(kk), idesc_acc, (kk > 0 || j > 0) ? 1u : 0u);
+          if (PAD) mma_ts(tmem_base + kColDQ, a + 64, bd + mnmajor_step(kk), idesc_acc, 1u);
+        }
         mma_commit(smem_u32(&sync->op_empty[buf]));
         mma_commit(smem_u32(&sync->k_empty[ks]));
         if (j + 1 == n_tiles) mma_commit(smem_u32(&sync->acc_done));
@@ -419,15 +431,15 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   } else {
     // -------------------------------------------------------- elementwise role
     const int r = tid & (kT - 1);              // query row inside the tile = TMEM lane
-    const int half = tid >> 7;                 // which 64 of the tile's 128 score columns
+    const int quarter = warp >> 2;             // which 32 of the tile's 128 score columns
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t s_addr = tmem_base + lane_off + kColS + half * 64;
-    const uint32_t dp_addr = tmem_base + lane_off + kColDP + half * 64;
-    const uint32_t op_addr = tmem_base + lane_off + kColOp + half * 32;
+    const uint32_t s_addr = tmem_base + lane_off + kColS + quarter * kQ;
+    const uint32_t dp_addr = tmem_base + lane_off + kColDP + quarter * kQ;
+    const uint32_t op_addr = tmem_base + lane_off + kColOp + quarter * (kQ / 2);
     const uint32_t dq_addr = tmem_base + lane_off + kColDQ;
     // checked build: the column ranges of this thread's tensor-memory traffic; a violation drains the CTA
-    if (!dbg_tmem(p.status, DBG_BWD_TC * 100 + 2, s_addr, tmem_base, 64, kTmemCols) || !dbg_tmem(p.status, DBG_BWD_TC * 100 + 3, dp_addr, tmem_base, 64, kTmemCols) ||
-        !dbg_tmem(p.status, DBG_BWD_TC * 100 + 4, op_addr, tmem_base, 32, kTmemCols) || !dbg_tmem(p.status, DBG_BWD_TC * 100 + 5, dq_addr, tmem_base, D, kTmemCols))
+    if (!dbg_tmem(p.status, DBG_BWD_TC * 100 + 2, s_addr, tmem_base, kQ, kTmemCols) || !dbg_tmem(p.status, DBG_BWD_TC * 100 + 3, dp_addr, tmem_base, kQ, kTmemCols) ||
+        !dbg_tmem(p.status, DBG_BWD_TC * 100 + 4, op_addr, tmem_base, 64 + kQ / 2, kTmemCols) || !dbg_tmem(p.status, DBG_BWD_TC * 100 + 5, dq_addr, tmem_base, D, kTmemCols))
       *abort_flag = 1;
     const int row_g = row0 + r;
     int lim = kv_limit;
@@ -451,9 +463,9 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     const bool bias_wide = BIAS && bias_rows_32b(p);
     for (int j = 0; j < n_tiles; ++j) {
-      const int buf = j & 1;
-      uint4 bv[BIAS ? 8 : 1];   // this thread's 64 bias elements of the tile, fetched under the wait
-      if constexpr (BIAS) load_bias_row(bv, bias_row, j * kT + half * 64, p.S, bias_wide);
+      const int buf = j % kBufs;
+      uint4 bv[BIAS ? kQ / 8 : 1];   // this thread's bias elements of the tile, fetched under the wait
+      if constexpr (BIAS) load_bias_row(bv, bias_row, j * kT + quarter * kQ, p.S, bias_wide);
       const uint32_t* bw = reinterpret_cast<const uint32_t*>(bv);
       bool ok = wait_clocked(smem_u32(&sync->sp_full), j & 1, abort_flag, wait_limit);
       ok = __all_sync(0xffffffffu, ok);
@@ -463,22 +475,19 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         break;
       }
       tc_fence_after_sync();
-      uint32_t sv[64], dv[64];
-      tmem_ld_32x32(s_addr, reinterpret_cast<uint32_t(&)[32]>(sv[0]));
-      tmem_ld_32x32(s_addr + 32, reinterpret_cast<uint32_t(&)[32]>(sv[32]));
-      tmem_ld_32x32(dp_addr, reinterpret_cast<uint32_t(&)[32]>(dv[0]));
-      tmem_ld_32x32(dp_addr + 32, reinterpret_cast<uint32_t(&)[32]>(dv[32]));
+      uint32_t sv[kQ], dv[kQ];
+      tmem_ld_32x32(s_addr, sv);
+      tmem_ld_32x32(dp_addr, dv);
       tmem_ld_wait();
       tc_fence_before_sync();
-      mbar_arrive(smem_u32(&sync->f_free));
-      const int col0 = j * kT + half * 64;
-      const bool need_mask = j * kT + kT > min_lim;
-      uint32_t pk[32];
-      // two columns per instruction (packed fp32 pairs) wherever the arithmetic allows: the loop is bound by
-      // what the eight warps can issue beside their 64 exponentials each
+      warp_arrive(&sync->f_free, lane);
+      const int col0 = j * kT + quarter * kQ;
+      const bool need_mask = col0 + kQ > min_lim;
+      uint32_t pk[kQ / 2], lo[PAD ? kQ / 2 : 1];
+      // two columns per instruction (packed fp32 pairs) wherever the arithmetic allows
       const uint64_t sl2_2 = f2_pack(sl2, sl2), neg_dl2 = f2_pack(-dl, -dl);
 #pragma unroll
-      for (int i = 0; i < 64; i += 2) {
+      for (int i = 0; i < kQ; i += 2) {
         float off0 = neg_l2, off1 = neg_l2;
         if constexpr (BIAS) {
           off0 = fmaf(bias_to_f32<BF16>(bw[i >> 1] & 0xffffu), kLog2e, neg_l2);
@@ -495,9 +504,10 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         float d0, d1;
         f2_unpack(f2_mul(f2_pack(p0, p1), f2_add(f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])), neg_dl2)), d0, d1);
         pk[i >> 1] = pack2<BF16>(d0, d1);
+        if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(d0, d1, pk[i >> 1]);
       }
-      if (j >= 2) {   // the product that read this operand buffer two tiles ago must have retired
-        ok = wait_clocked(smem_u32(&sync->op_empty[buf]), ((j >> 1) - 1) & 1, abort_flag, wait_limit);
+      if (j >= kBufs) {   // the product that read this operand buffer before must have retired
+        ok = wait_clocked(smem_u32(&sync->op_empty[buf]), (j / kBufs - 1) & 1, abort_flag, wait_limit);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) {
           if (lane == 0) report(p.status, 16, j, warp);
@@ -506,11 +516,11 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         tc_fence_after_sync();
       }
-      tmem_st_32x16(op_addr + buf * 64, reinterpret_cast<uint32_t(&)[16]>(pk[0]));
-      tmem_st_32x16(op_addr + buf * 64 + 16, reinterpret_cast<uint32_t(&)[16]>(pk[16]));
+      tmem_st_32x16(op_addr + buf * 64, pk);
+      if constexpr (PAD) tmem_st_32x16(op_addr + 64, lo);
       tmem_st_wait();
       tc_fence_before_sync();
-      mbar_arrive(smem_u32(&sync->e_ready[buf]));
+      warp_arrive(&sync->e_ready[buf], lane);
     }
     if (alive && n_tiles > 0) {
       bool ok = wait_clocked(smem_u32(&sync->acc_done), 0, abort_flag, wait_limit);
@@ -523,9 +533,9 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     if (alive) {
       uint8_t* stage = smem_raw + (q_tile - raw_addr);   // Q is no longer needed
-      stage_row<D, BF16>(dq_addr, n_tiles > 0, p.scale, stage, r, half);
+      for (int c = quarter; c < D / 32; c += 4) stage_chunk<BF16>(dq_addr, n_tiles > 0, p.scale, stage, r, c);
       fence_proxy_async_smem();
-      mbar_arrive(smem_u32(&sync->staged));
+      warp_arrive(&sync->staged, lane);
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {
         for (int bx = 0; bx < C::kBoxes; ++bx) {
           if (PAD && bx * 64 >= p.E) break;
@@ -628,7 +638,6 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   tc_fence_after_sync();
   const uint32_t tmem_base = sync->tmem_base;
   constexpr uint32_t kColDV = kColAcc, kColDK = kColAcc + D;
-  const int n_units = 2 * n_items;
 
   if (warp == kProducerWarp) {
     // the whole warp runs the loop: the lanes copy the query tile's row statistics into
@@ -682,7 +691,7 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
     __syncwarp();
   } else if (warp == kMmaWarp) {
-    constexpr uint32_t idesc_score = make_idesc(BF16, false, kT, kU);
+    constexpr uint32_t idesc_score = make_idesc(BF16, false, kT, kT);
     const uint32_t idesc_dk = make_idesc(BF16, true, kT, PAD ? (p.E + 15) / 16 * 16 : D);
     const uint32_t idesc_dv = make_idesc(BF16, true, kT, PAD ? (p.Dv + 15) / 16 * 16 : D);
     const int steps_e = PAD ? (p.E + 15) / 16 : D / 16, steps_v = PAD ? (p.Dv + 15) / 16 : D / 16;
@@ -691,56 +700,64 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       alive = wait_clocked(smem_u32(&sync->fixed_full), 0, abort_flag, wait_limit);
       if (!alive && lane == 0) report(p.status, 22, -1, 0);
     }
-    // S^T_u = K Q_u^T and dP^T_u = V dO_u^T into buffer u & 1 (waits for the query tile when the unit opens it)
-    auto issue_scores = [&](int u) -> bool {
-      const int it = u >> 1, hh = u & 1, buf = u & 1;
-      const int stage = it % C::kStages;
-      if (hh == 0) {
-        const uint32_t round = static_cast<uint32_t>(it / C::kStages);
-        if (!wait_clocked(smem_u32(&sync->ring_full[stage]), round & 1u, abort_flag, wait_limit)) {
-          if (lane == 0) report(p.status, 22, it, stage);
-          return false;
-        }
-        tc_fence_after_sync();
+    auto q_tile = [&](int it) { return ring + (it % C::kStages) * 2 * C::kTileBytes; };   // dO right behind it
+    // S^T_i = K Q_i^T (waits for the query tile); the MMA pipe executes in issue order, so it may be issued right
+    // behind the product that reads P^T_{i-1} from the same columns
+    auto issue_s = [&](int it) -> bool {
+      const uint32_t round = static_cast<uint32_t>(it / C::kStages);
+      if (!wait_clocked(smem_u32(&sync->ring_full[it % C::kStages]), round & 1u, abort_flag, wait_limit)) {
+        if (lane == 0) report(p.status, 22, it, it % C::kStages);
+        return false;
       }
-      const uint32_t q_tile = ring + stage * 2 * C::kTileBytes, do_tile = q_tile + C::kTileBytes;
-      issue_ss<D, PAD>(tmem_base + kColS + buf * kU, k_tile, q_tile, hh, idesc_score, steps_e);
-      issue_ss<D, PAD>(tmem_base + kColDP + buf * kU, v_tile, do_tile, hh, idesc_score, steps_v);
-      if (elect_one()) mma_commit(smem_u32(&sync->sp_full[buf]));
+      tc_fence_after_sync();
+      issue_ss<D, PAD>(tmem_base + kColS, k_tile, q_tile(it), idesc_score, steps_e);
+      if (elect_one()) mma_commit(smem_u32(&sync->s_full));
       return true;
     };
-    if (alive) alive = issue_scores(0);
-    if (alive) alive = issue_scores(1);
-    for (int u = 0; u < n_units && alive; ++u) {
-      const int it = u >> 1, hh = u & 1, buf = u & 1;
-      const int stage = it % C::kStages;
-      alive = wait_clocked(smem_u32(&sync->e_ready[buf]), (u >> 1) & 1, abort_flag, wait_limit);
+    auto issue_dp = [&](int it) {   // dP^T_i = V dO_i^T
+      issue_ss<D, PAD>(tmem_base + kColDP, v_tile, q_tile(it) + C::kTileBytes, idesc_score, steps_v);
+      if (elect_one()) mma_commit(smem_u32(&sync->dp_full));
+    };
+    if (alive) alive = issue_s(0);
+    if (alive) issue_dp(0);
+    for (int it = 0; it < n_items && alive; ++it) {
+      const bool more = it + 1 < n_items;
+      alive = wait_clocked(smem_u32(&sync->p_ready), it & 1, abort_flag, wait_limit);
       if (!alive) {
-        if (lane == 0) report(p.status, 23, u, 0);
+        if (lane == 0) report(p.status, 23, it, 0);
         break;
       }
       tc_fence_after_sync();
-      const uint32_t q_tile = ring + stage * 2 * C::kTileBytes, do_tile = q_tile + C::kTileBytes;
-      issue_ts(tmem_base + kColDV, tmem_base + kColS + buf * kU, do_tile, hh, idesc_dv, u > 0);   // dV += P^T_u dO_u
-      issue_ts(tmem_base + kColDK, tmem_base + kColDP + buf * kU, q_tile, hh, idesc_dk, u > 0);   // dK += dS^T_u Q_u
-      if (elect_one()) {
-        if (hh == 1) mma_commit(smem_u32(&sync->ring_empty[stage]));
-        if (u + 1 == n_units) mma_commit(smem_u32(&sync->acc_done));
+      issue_ts<PAD>(tmem_base + kColDV, tmem_base + kColS, q_tile(it) + C::kTileBytes, idesc_dv, it > 0);   // dV += P^T dO
+      if (more) {
+        alive = issue_s(it + 1);
+        if (!alive) break;
       }
-      if (u + 2 < n_units) alive = issue_scores(u + 2);
+      alive = wait_clocked(smem_u32(&sync->ds_ready), it & 1, abort_flag, wait_limit);
+      if (!alive) {
+        if (lane == 0) report(p.status, 23, it, 1);
+        break;
+      }
+      tc_fence_after_sync();
+      issue_ts<PAD>(tmem_base + kColDK, tmem_base + kColDP, q_tile(it), idesc_dk, it > 0);                  // dK += dS^T Q
+      if (elect_one()) {
+        mma_commit(smem_u32(&sync->ring_empty[it % C::kStages]));
+        if (!more) mma_commit(smem_u32(&sync->acc_done));
+      }
+      if (more) issue_dp(it + 1);
     }
     if (*abort_flag != 0) drain_after_abort(sync, wait_limit);
     __syncwarp();
   } else {
     // -------------------------------------------------------- elementwise role
     const int r = tid & (kT - 1);              // key inside the tile = TMEM lane
-    const int half = tid >> 7;                 // which 32 of the unit's 64 query columns
+    const int quarter = warp >> 2;             // which 32 of the tile's 128 query columns
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t s_addr = tmem_base + lane_off + kColS + half * 32;
-    const uint32_t dp_addr = tmem_base + lane_off + kColDP + half * 32;
-    // checked build: both buffers of the score-shaped units and the two accumulators
-    if (!dbg_tmem(p.status, DBG_BWD_TC * 100 + 7, s_addr, tmem_base, kU + 32, kTmemCols) ||
-        !dbg_tmem(p.status, DBG_BWD_TC * 100 + 8, dp_addr, tmem_base, kU + 32, kTmemCols) ||
+    const uint32_t s_addr = tmem_base + lane_off + kColS + quarter * kQ;
+    const uint32_t dp_addr = tmem_base + lane_off + kColDP + quarter * kQ;
+    // checked build: the score-shaped buffers and the two accumulators
+    if (!dbg_tmem(p.status, DBG_BWD_TC * 100 + 7, s_addr, tmem_base, kQ, kTmemCols) ||
+        !dbg_tmem(p.status, DBG_BWD_TC * 100 + 8, dp_addr, tmem_base, kQ, kTmemCols) ||
         !dbg_tmem(p.status, DBG_BWD_TC * 100 + 9, tmem_base + lane_off + kColDK, tmem_base, D, kTmemCols))
       *abort_flag = 1;
     const int key_g = j0 + r;
@@ -755,75 +772,104 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const float sl2 = p.scale * kLog2e;
     const uint64_t sl2_2 = f2_pack(sl2, sl2);
     bool alive = true;
-    for (int u = 0; u < n_units; ++u) {
-      const int it = u >> 1, hh = u & 1, buf = u & 1;
-      const int unit_row0 = (i_first + it % per_head) * kT + hh * kU;   // first query row of the unit
-      const int qrow0 = unit_row0 + half * 32;                          // ... and of this thread's columns
-      uint32_t bq[BIAS ? 32 : 1];   // bias of this key under the thread's 32 query rows, fetched under the wait
+    int head = hk * p.group, tile = 0;         // query head and row tile (from i_first) of an item
+    for (int it = 0; it < n_items; ++it) {
+      const int qrow0 = (i_first + tile) * kT + quarter * kQ;   // first query row of this thread's columns
+      uint32_t bq[BIAS ? kQ / 2 : 1];   // bias of this key under the thread's 32 query rows, fetched under the wait
       if constexpr (BIAS) {
         // neighbouring lanes are neighbouring keys: each of the 32 loads is one 64-byte piece per warp
-        const uint16_t* col = static_cast<const uint16_t*>(p.bias) + b * p.bs[0] +
-                              static_cast<long long>(hk * p.group + it / per_head) * p.bs[1] + key_g;
+        const uint16_t* col = static_cast<const uint16_t*>(p.bias) + b * p.bs[0] + static_cast<long long>(head) * p.bs[1] + key_g;
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          bq[i] = (key_g < p.S && qrow0 + i < p.L) ? __ldg(col + static_cast<long long>(qrow0 + i) * p.bs[2]) : 0u;
+        for (int i = 0; i < kQ; i += 2) {
+          uint32_t lo = 0u, hi = 0u;
+          if (key_g < p.S && qrow0 + i < p.L) lo = __ldg(col + static_cast<long long>(qrow0 + i) * p.bs[2]);
+          if (key_g < p.S && qrow0 + i + 1 < p.L) hi = __ldg(col + static_cast<long long>(qrow0 + i + 1) * p.bs[2]);
+          bq[i >> 1] = lo | (hi << 16);
+        }
       }
-      bool ok = wait_clocked(smem_u32(&sync->sp_full[buf]), (u >> 1) & 1, abort_flag, wait_limit);
+      if (++tile == per_head) {
+        tile = 0;
+        ++head;
+      }
+      bool ok = wait_clocked(smem_u32(&sync->s_full), it & 1, abort_flag, wait_limit);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) {
-        if (lane == 0) report(p.status, 24, u, warp);
+        if (lane == 0) report(p.status, 24, it, warp);
         alive = false;
         break;
       }
       tc_fence_after_sync();
-      const int stage = it % C::kStages;
-      const float4* st4 = reinterpret_cast<const float4*>(stats + stage * 2 * kT) + hh * 16 + half * 8;
-      // some key of this tile hides some row of this unit
+      const float4* st4 = reinterpret_cast<const float4*>(stats + (it % C::kStages) * 2 * kT) + quarter * (kQ / 4);
+      // some key of this tile hides some row of these columns
       const bool need_mask = tile_has_padding ||
-                             (p.causal && static_cast<long long>(unit_row0) < static_cast<long long>(j0) + kT - 1 - p.causal_shift);
-      uint32_t sv[32], dv[32];
-      tmem_ld_32x32(s_addr + buf * kU, sv);
-      tmem_ld_32x32(dp_addr + buf * kU, dv);
-      tmem_ld_wait();
-      uint32_t pkp[16], pkd[16];
+                             (p.causal && static_cast<long long>(qrow0) < static_cast<long long>(j0) + kT - 1 - p.causal_shift);
+      float pr[kQ];
+      {
+        uint32_t sv[kQ], pk[kQ / 2], lo[PAD ? kQ / 2 : 1];
+        tmem_ld_32x32(s_addr, sv);
+        tmem_ld_wait();
 #pragma unroll
-      for (int q4 = 0; q4 < 8; ++q4) {
-        const float4 l4 = st4[q4];
-        const float4 d4 = st4[32 + q4];
-        const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
-        const float ds_[4] = {d4.x, d4.y, d4.z, d4.w};
-        float pr[4], dsv[4];
+        for (int q4 = 0; q4 < kQ / 4; ++q4) {
+          const float4 l4 = st4[q4];
+          const float ls[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
-        for (int e = 0; e < 4; e += 2) {   // two query columns per instruction (packed fp32 pairs)
-          const int i = q4 * 4 + e;
-          float off0 = -ls[e], off1 = -ls[e + 1];
-          if constexpr (BIAS) {
-            off0 = fmaf(bias_to_f32<BF16>(bq[i]), kLog2e, off0);
-            off1 = fmaf(bias_to_f32<BF16>(bq[i + 1]), kLog2e, off1);
+          for (int e = 0; e < 4; e += 2) {   // two query columns per instruction (packed fp32 pairs)
+            const int i = q4 * 4 + e;
+            float off0 = -ls[e], off1 = -ls[e + 1];
+            if constexpr (BIAS) {
+              off0 = fmaf(bias_to_f32<BF16>(bq[i >> 1] & 0xffffu), kLog2e, off0);
+              off1 = fmaf(bias_to_f32<BF16>(bq[i >> 1] >> 16), kLog2e, off1);
+            }
+            float a0, a1;
+            f2_unpack(f2_fma(f2_pack(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2_2, f2_pack(off0, off1)), a0, a1);
+            float p0 = ex2(a0), p1 = ex2(a1);
+            if (need_mask) {
+              p0 = (qrow0 + i >= i_min) ? p0 : 0.f;
+              p1 = (qrow0 + i + 1 >= i_min) ? p1 : 0.f;
+            }
+            pr[i] = p0;
+            pr[i + 1] = p1;
+            pk[i >> 1] = pack2<BF16>(p0, p1);
+            if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(p0, p1, pk[i >> 1]);
           }
-          float a0, a1;
-          f2_unpack(f2_fma(f2_pack(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2_2, f2_pack(off0, off1)), a0, a1);
-          float p0 = ex2(a0), p1 = ex2(a1);
-          if (need_mask) {
-            p0 = (qrow0 + i >= i_min) ? p0 : 0.f;
-            p1 = (qrow0 + i + 1 >= i_min) ? p1 : 0.f;
-          }
-          pr[e] = p0;
-          pr[e + 1] = p1;
-          f2_unpack(f2_mul(f2_pack(p0, p1), f2_add(f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])),
-                                                    f2_pack(-ds_[e], -ds_[e + 1]))),
-                    dsv[e], dsv[e + 1]);
         }
-        pkp[q4 * 2] = pack2<BF16>(pr[0], pr[1]);
-        pkp[q4 * 2 + 1] = pack2<BF16>(pr[2], pr[3]);
-        pkd[q4 * 2] = pack2<BF16>(dsv[0], dsv[1]);
-        pkd[q4 * 2 + 1] = pack2<BF16>(dsv[2], dsv[3]);
+        tmem_st_32x16(s_addr, pk);
+        if constexpr (PAD) tmem_st_32x16(s_addr + 16, lo);
+        tmem_st_wait();
+        tc_fence_before_sync();
+        warp_arrive(&sync->p_ready, lane);
       }
-      tmem_st_32x16(s_addr + buf * kU, pkp);
-      tmem_st_32x16(dp_addr + buf * kU, pkd);
+      ok = wait_clocked(smem_u32(&sync->dp_full), it & 1, abort_flag, wait_limit);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        if (lane == 0) report(p.status, 26, it, warp);
+        alive = false;
+        break;
+      }
+      tc_fence_after_sync();
+      uint32_t dv[kQ], pk[kQ / 2], lo[PAD ? kQ / 2 : 1];
+      tmem_ld_32x32(dp_addr, dv);
+      tmem_ld_wait();
+#pragma unroll
+      for (int q4 = 0; q4 < kQ / 4; ++q4) {
+        const float4 d4 = st4[kT / 4 + q4];
+        const float nd[4] = {-d4.x, -d4.y, -d4.z, -d4.w};
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+          const int i = q4 * 4 + e;
+          float d0, d1;
+          f2_unpack(f2_mul(f2_pack(pr[i], pr[i + 1]), f2_add(f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])),
+                                                              f2_pack(nd[e], nd[e + 1]))),
+                    d0, d1);
+          pk[i >> 1] = pack2<BF16>(d0, d1);
+          if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(d0, d1, pk[i >> 1]);
+        }
+      }
+      tmem_st_32x16(dp_addr, pk);
+      if constexpr (PAD) tmem_st_32x16(dp_addr + 16, lo);
       tmem_st_wait();
       tc_fence_before_sync();
-      mbar_arrive(smem_u32(&sync->e_ready[buf]));
+      warp_arrive(&sync->ds_ready, lane);
     }
     if (alive && n_items > 0) {
       bool ok = wait_clocked(smem_u32(&sync->acc_done), 0, abort_flag, wait_limit);
@@ -838,10 +884,12 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       // ring slot 0 is idle by now: its two tiles stage dK and dV
       uint8_t* stage_k = smem_raw + (ring - raw_addr);
       uint8_t* stage_v = stage_k + C::kTileBytes;
-      stage_row<D, BF16>(tmem_base + lane_off + kColDK, n_items > 0, p.scale, stage_k, r, half);
-      stage_row<D, BF16>(tmem_base + lane_off + kColDV, n_items > 0, 1.f, stage_v, r, half);
+      for (int c = quarter; c < D / 16; c += 4) {
+        if (c < D / 32) stage_chunk<BF16>(tmem_base + lane_off + kColDK, n_items > 0, p.scale, stage_k, r, c);
+        else stage_chunk<BF16>(tmem_base + lane_off + kColDV, n_items > 0, 1.f, stage_v, r, c - D / 32);
+      }
       fence_proxy_async_smem();
-      mbar_arrive(smem_u32(&sync->staged));
+      warp_arrive(&sync->staged, lane);
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {
         for (int bx = 0; bx < C::kBoxes; ++bx) {
           if (!PAD || bx * 64 < p.E) tma_store_4d(&tm_dk, ring + bx * kBoxBytes, bx * 64, j0, hk, b);

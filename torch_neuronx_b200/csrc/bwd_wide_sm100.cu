@@ -14,12 +14,15 @@
 // launch (neighbouring CTAs, which read the same query tiles), the dQ walk is a programmatic dependent of it.
 // Bound: the tensor pipe.  NT = 128 at 192/128; at 256 the fixed operands alone take 128 KB and NT is 64.
 // Before, these shapes ran on the CUDA-core kernels.  1 x 24 x 2048, 192/128, causal, forward and backward: 19.8 ms
-// then, 0.246 ms with these kernels (0.05 of it the forward).
+// then, 0.273 ms with these kernels (0.05 of it the forward).
 //
-// Roles per CTA (320 threads): warps 0-7 elementwise (two threads per TMEM lane), warp 8 TMA producer, warp 9 MMA
+// Roles per CTA (576 threads): warps 0-15 elementwise (four threads per TMEM lane), warp 16 TMA producer, warp 17 MMA
 // issuer.  The elementwise warps copy a tile's scores into registers and release the accumulators at once, so the
 // score products of the next tile run under their arithmetic; the 16-bit operand they leave in tensor memory has
-// columns of its own.  Roundings, masks, bounded waits: as in bwd_sm100.cu.
+// columns of its own.  These shapes had fp32 probabilities on the CUDA-core kernels, so P and dS go into their second
+// product as hi + lo, two 16-bit operands (remainder2).  The dQ and dK walks at E = 192 have no columns for lo: it
+// takes the place of dP (kHold), whose next product then follows the one that reads lo.
+// Masks, bounded waits: as in bwd_sm100.cu.
 #include "bwd_common.cuh"
 
 namespace b200 {
@@ -29,10 +32,10 @@ namespace {
 using namespace ptx;
 using namespace tc;
 
-constexpr int kThreads = 320;
-constexpr int kEThreads = 256;
-constexpr int kProducerWarp = 8;
-constexpr int kMmaWarp = 9;
+constexpr int kEWarps = 16;
+constexpr int kThreads = (kEWarps + 2) * 32;
+constexpr int kProducerWarp = kEWarps;
+constexpr int kMmaWarp = kEWarps + 1;
 constexpr uint32_t kTmemCols = 512;
 
 enum Walk { kDQ = 0, kDK = 1, kDV = 2 };
@@ -50,12 +53,14 @@ template <int WALK, int E, int DV> struct WCfg {
   static constexpr int kStatBytes = 2 * 2 * kNT * 4;               // (lse2, delta) of a streamed query tile, two slots
   static constexpr int kSmemBytes = kTiles + kStatBytes + 256 /*barriers*/;
   static constexpr int kAccW = WALK == kDV ? DV : E;
-  // tensor memory: S, dP, one or two operand buffers, accumulator
+  // tensor memory: S, dP, one or two operand buffers (hi, then lo), accumulator
   static constexpr uint32_t kColS = 0, kColDP = kNT;
   static constexpr uint32_t kColOp = WALK == kDV ? kNT : 2 * kNT;
-  static constexpr int kOpBufs = (2 * kNT + kNT + kAccW <= 512) ? 2 : 1;
   static constexpr uint32_t kColAcc = 512 - kAccW;
-  static_assert(kColOp + kOpBufs * (kNT / 2) <= kColAcc, "tensor memory");
+  static constexpr bool kHold = kColOp + kNT > kColAcc;            // room for hi, not for lo
+  static constexpr int kOpCols = kHold ? kNT / 2 : kNT;            // columns of an operand buffer
+  static constexpr int kOpBufs = kColOp + 2 * kOpCols <= kColAcc ? 2 : 1;
+  static_assert(kColOp + kOpBufs * kOpCols <= kColAcc, "tensor memory");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 };
 
@@ -74,6 +79,12 @@ struct WSync {
   int abort_flag;
 };
 static_assert(sizeof(WSync) <= 256, "barrier block must fit its reserve");
+
+// 32 or 16 consecutive columns of this thread's tensor-memory lane to or from registers.
+__device__ __forceinline__ void tmem_ld_row(uint32_t addr, uint32_t (&v)[32]) { tmem_ld_32x32(addr, v); }
+__device__ __forceinline__ void tmem_ld_row(uint32_t addr, uint32_t (&v)[16]) { tmem_ld_32x16(addr, v); }
+__device__ __forceinline__ void tmem_st_row(uint32_t addr, const uint32_t (&v)[16]) { tmem_st_32x16(addr, v); }
+__device__ __forceinline__ void tmem_st_row(uint32_t addr, const uint32_t (&v)[8]) { tmem_st_32x8(addr, v); }
 
 // Where a CTA works, decoded by the kernels below.
 struct WWork {
@@ -125,13 +136,13 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
   }
   if (tid == 0) {
     mbar_init(smem_u32(&sync->sp_full), 1);
-    mbar_init(smem_u32(&sync->f_free), kEThreads);
+    mbar_init(smem_u32(&sync->f_free), kEWarps);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&sync->e_ready[i]), kEThreads);
+      mbar_init(smem_u32(&sync->e_ready[i]), kEWarps);
       mbar_init(smem_u32(&sync->op_empty[i]), 1);
     }
     mbar_init(smem_u32(&sync->acc_done), 1);
-    mbar_init(smem_u32(&sync->staged), kEThreads);
+    mbar_init(smem_u32(&sync->staged), kEWarps);
     mbar_init(smem_u32(&sync->drain), 1);
     sync->abort_flag = 0;
     mbar_fence_init();
@@ -218,21 +229,37 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
     }
     // k-step kk (16 elements of the head dimension) of a K-major streamed tile
     auto stream_step = [](int kk) { return static_cast<uint64_t>(((kk >> 2) * C::kStreamBox + (kk & 3) * 32) >> 4); };
-    auto issue_scores = [&](int j) -> bool {
-      const int ls = j % C::kLongSlots, ss = j % C::kShortSlots;
-      if (!wait_clocked(smem_u32(&sync->long_full[ls]), (j / C::kLongSlots) & 1u, abort_flag, wait_limit) ||
-          !wait_clocked(smem_u32(&sync->short_full[ss]), (j / C::kShortSlots) & 1u, abort_flag, wait_limit)) {
-        if (lane == 0) report(p.status, 32, j, ls);
-        return false;
-      }
+    auto wait_long = [&](int j) -> bool {
+      const int ls = j % C::kLongSlots;
+      const bool ok = wait_clocked(smem_u32(&sync->long_full[ls]), (j / C::kLongSlots) & 1u, abort_flag, wait_limit);
+      if (!ok && lane == 0) report(p.status, 32, j, ls);
+      return ok;
+    };
+    auto wait_short = [&](int j) -> bool {
+      const int ss = j % C::kShortSlots;
+      const bool ok = wait_clocked(smem_u32(&sync->short_full[ss]), (j / C::kShortSlots) & 1u, abort_flag, wait_limit);
+      if (!ok && lane == 0) report(p.status, 32, j, 8 + ss);
+      return ok;
+    };
+    auto issue_s = [&](int j) -> bool {
+      if (!(WALK == kDV ? wait_short(j) : wait_long(j))) return false;
       tc_fence_after_sync();
-      const uint32_t e_tile = WALK == kDV ? short_ring + ss * C::kShortBytes : long_ring + ls * C::kLongBytes;
+      const uint32_t e_tile = WALK == kDV ? short_ring + (j % C::kShortSlots) * C::kShortBytes
+                                          : long_ring + (j % C::kLongSlots) * C::kLongBytes;
       const uint64_t fd = kmajor_desc(fe_tile), gd = kmajor_desc(e_tile);
-      const uint64_t fvd = kmajor_desc(fv_tile), gvd = kmajor_desc(short_ring + ss * C::kShortBytes);
       if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < E / 16; ++kk)
           mma_ss(tmem_base + C::kColS, fd + kmajor_step(kk), gd + stream_step(kk), idesc_score, kk > 0 ? 1u : 0u);
+      }
+      return true;
+    };
+    auto issue_dp = [&](int j) -> bool {   // ... after which the tile's scores are complete
+      if (!(WALK == kDV ? wait_long(j) : wait_short(j))) return false;
+      tc_fence_after_sync();
+      const int ss = j % C::kShortSlots;
+      const uint64_t fvd = kmajor_desc(fv_tile), gvd = kmajor_desc(short_ring + ss * C::kShortBytes);
+      if (elect_one()) {
         if (WALK != kDV) {
 #pragma unroll
           for (int kk = 0; kk < DV / 16; ++kk)
@@ -243,17 +270,18 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
       }
       return true;
     };
-    if (alive) alive = issue_scores(0);
+    if (alive) alive = issue_s(0) && issue_dp(0);
     for (int j = 0; j < w.n_tiles && alive; ++j) {
       const int buf = j % C::kOpBufs, ls = j % C::kLongSlots;
+      const bool more = j + 1 < w.n_tiles;
       alive = wait_clocked(smem_u32(&sync->f_free), j & 1, abort_flag, wait_limit);
       if (!alive) {
         if (lane == 0) report(p.status, 33, j, 1);
         break;
       }
       tc_fence_after_sync();
-      if (j + 1 < w.n_tiles) {
-        alive = issue_scores(j + 1);
+      if (more) {
+        alive = issue_s(j + 1) && (C::kHold || issue_dp(j + 1));
         if (!alive) break;
       }
       alive = wait_clocked(smem_u32(&sync->e_ready[buf]), (j / C::kOpBufs) & 1, abort_flag, wait_limit);
@@ -263,14 +291,26 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
       }
       tc_fence_after_sync();
       const uint64_t bd = smem_desc_sw128(long_ring + ls * C::kLongBytes, C::kStreamBox, 1024);   // MN-major B operand
+      const uint32_t op = tmem_base + C::kColOp + buf * C::kOpCols;
+      if (elect_one()) {
+#pragma unroll
+        for (int kk = 0; kk < NT / 16; ++kk) {   // the remainders
+          const uint32_t a = C::kHold ? tmem_base + C::kColDP + static_cast<uint32_t>((kk >> 1) * 32 + (kk & 1) * 8)
+                                      : op + NT / 2 + static_cast<uint32_t>(kk * 8);
+          mma_ts(tmem_base + C::kColAcc, a, bd + mnmajor_step(kk), idesc_acc, (kk > 0 || j > 0) ? 1u : 0u);
+        }
+      }
+      if (C::kHold && more) {   // in issue order behind the products that read lo from its columns
+        alive = issue_dp(j + 1);
+        if (!alive) break;
+      }
       if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < NT / 16; ++kk)
-          mma_ts(tmem_base + C::kColAcc, tmem_base + C::kColOp + buf * (NT / 2) + static_cast<uint32_t>(kk * 8),
-                 bd + mnmajor_step(kk), idesc_acc, (kk > 0 || j > 0) ? 1u : 0u);
+          mma_ts(tmem_base + C::kColAcc, op + static_cast<uint32_t>(kk * 8), bd + mnmajor_step(kk), idesc_acc, 1u);
         mma_commit(smem_u32(&sync->op_empty[buf]));
         mma_commit(smem_u32(&sync->long_empty[ls]));
-        if (j + 1 == w.n_tiles) mma_commit(smem_u32(&sync->acc_done));
+        if (!more) mma_commit(smem_u32(&sync->acc_done));
       }
     }
     if (*abort_flag != 0) {
@@ -280,17 +320,17 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
     __syncwarp();
   } else {
     // -------------------------------------------------------- elementwise role
-    constexpr int HC = NT / 2;                 // score columns of one thread
+    constexpr int HC = NT / 4;                 // score columns of one thread
     const int r = tid & (kT - 1);              // fixed row = TMEM lane
-    const int half = tid >> 7;
+    const int quarter = warp >> 2;
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t s_addr = tmem_base + lane_off + C::kColS + half * HC;
-    const uint32_t dp_addr = tmem_base + lane_off + C::kColDP + half * HC;
-    const uint32_t op_addr = tmem_base + lane_off + C::kColOp + half * (HC / 2);
+    const uint32_t s_addr = tmem_base + lane_off + C::kColS + quarter * HC;
+    const uint32_t dp_addr = tmem_base + lane_off + C::kColDP + quarter * HC;
+    const uint32_t op_addr = tmem_base + lane_off + C::kColOp + quarter * (HC / 2);
     const uint32_t acc_addr = tmem_base + lane_off + C::kColAcc;
     if (!dbg_tmem(p.status, DBG_BWD_WIDE * 100 + 2, s_addr, tmem_base, HC, kTmemCols) ||
         !dbg_tmem(p.status, DBG_BWD_WIDE * 100 + 3, dp_addr, tmem_base, HC, kTmemCols) ||
-        !dbg_tmem(p.status, DBG_BWD_WIDE * 100 + 4, op_addr, tmem_base, (C::kOpBufs - 1) * (NT / 2) + HC / 2, kTmemCols) ||
+        !dbg_tmem(p.status, DBG_BWD_WIDE * 100 + 4, op_addr, tmem_base, (C::kOpBufs - 1) * C::kOpCols + (C::kHold ? 0 : NT / 2) + HC / 2, kTmemCols) ||
         !dbg_tmem(p.status, DBG_BWD_WIDE * 100 + 5, acc_addr, tmem_base, C::kAccW, kTmemCols))
       *abort_flag = 1;
     const int row_g = w.row0 + r;
@@ -329,23 +369,19 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
       }
       tc_fence_after_sync();
       uint32_t sv[HC], dv[WALK == kDV ? 1 : HC];
-#pragma unroll
-      for (int c = 0; c < HC / 32; ++c) tmem_ld_32x32(s_addr + c * 32, reinterpret_cast<uint32_t(&)[32]>(sv[c * 32]));
-      if constexpr (WALK != kDV) {
-#pragma unroll
-        for (int c = 0; c < HC / 32; ++c) tmem_ld_32x32(dp_addr + c * 32, reinterpret_cast<uint32_t(&)[32]>(dv[c * 32]));
-      }
+      tmem_ld_row(s_addr, sv);
+      if constexpr (WALK != kDV) tmem_ld_row(dp_addr, dv);
       tmem_ld_wait();
       tc_fence_before_sync();
-      mbar_arrive(smem_u32(&sync->f_free));
+      warp_arrive(&sync->f_free, lane);
       const int tile0 = tile_row(j);           // first streamed row
-      const int col0 = tile0 + half * HC;      // ... of this thread's columns
+      const int col0 = tile0 + quarter * HC;      // ... of this thread's columns
       const bool need_mask = WALK == kDQ ? tile0 + NT > w.min_lim
                                          : (w.row0 + kT > w.n_keys ||
                                             (p.causal && static_cast<long long>(tile0) <
                                                              static_cast<long long>(w.row0) + kT - 1 - p.causal_shift));
-      const float4* st4 = reinterpret_cast<const float4*>(stats + (j % C::kLongSlots) * 2 * NT + half * HC);
-      uint32_t pk[HC / 2];
+      const float4* st4 = reinterpret_cast<const float4*>(stats + (j % C::kLongSlots) * 2 * NT + quarter * HC);
+      uint32_t pk[HC / 2], lo[HC / 2];
 #pragma unroll
       for (int q4 = 0; q4 < HC / 4; ++q4) {
         float nl[4] = {neg_l2, neg_l2, neg_l2, neg_l2}, nd[4] = {-dl, -dl, -dl, -dl};
@@ -372,6 +408,7 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
                       p0, p1);
           }
           pk[i >> 1] = pack2<BF16>(p0, p1);
+          lo[i >> 1] = remainder2<BF16>(p0, p1, pk[i >> 1]);
         }
       }
       if (j >= C::kOpBufs) {   // the product that read this operand buffer before must have retired
@@ -384,12 +421,11 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
         }
         tc_fence_after_sync();
       }
-#pragma unroll
-      for (int c = 0; c < HC / 32; ++c)
-        tmem_st_32x16(op_addr + buf * (NT / 2) + c * 16, reinterpret_cast<uint32_t(&)[16]>(pk[c * 16]));
+      tmem_st_row(op_addr + buf * C::kOpCols, pk);
+      tmem_st_row(C::kHold ? dp_addr : op_addr + buf * C::kOpCols + NT / 2, lo);
       tmem_st_wait();
       tc_fence_before_sync();
-      mbar_arrive(smem_u32(&sync->e_ready[buf]));
+      warp_arrive(&sync->e_ready[buf], lane);
     }
     if (alive && w.n_tiles > 0) {
       bool ok = wait_clocked(smem_u32(&sync->acc_done), 0, abort_flag, wait_limit);
@@ -402,9 +438,10 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
     }
     if (alive) {
       // the fixed operands are no longer needed: their area stages the gradient
-      stage_row<C::kAccW, BF16>(acc_addr, w.n_tiles > 0, WALK == kDV ? 1.f : p.scale, smem_raw, r, half);
+      for (int c = quarter; c < C::kAccW / 32; c += 4)
+        stage_chunk<BF16>(acc_addr, w.n_tiles > 0, WALK == kDV ? 1.f : p.scale, smem_raw, r, c);
       fence_proxy_async_smem();
-      mbar_arrive(smem_u32(&sync->staged));
+      warp_arrive(&sync->staged, lane);
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {
         const int head = WALK == kDQ ? w.h : w.hk;
         for (int bx = 0; bx < C::kAccW / 64; ++bx) tma_store_4d(tm_out, tiles + bx * kBoxBytes, bx * 64, w.row0, head, w.b);
