@@ -102,9 +102,12 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const BwdProblem bp, floa
   const int b = static_cast<int>(bh / p.Hq);
   float d = 0.f, l2 = CUDART_INF_F;
   const bool live = in_range && i < p.L;
+  // between the forward and the dK/dV kernel, both of whose launches this one overlaps
+  pdl_wait();
+  pdl_launch_dependents();
   if (live) {
-    const T* __restrict__ go = reinterpret_cast<const T*>(bp.dout) + b * bp.dos[0] + h * bp.dos[1] + i * bp.dos[2];
-    const T* __restrict__ o = reinterpret_cast<const T*>(p.out) + b * p.os[0] + h * p.os[1] + i * p.os[2];
+    const T* go = reinterpret_cast<const T*>(bp.dout) + b * bp.dos[0] + h * bp.dos[1] + i * bp.dos[2];
+    const T* o = reinterpret_cast<const T*>(p.out) + b * p.os[0] + h * p.os[1] + i * p.os[2];
     if (VEC) {
       for (int e = sub * 8; e < p.Dv; e += 64) {
         const uint4 a = *reinterpret_cast<const uint4*>(go + e);
@@ -567,7 +570,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                   const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
-                  const Problem p, const float* __restrict__ lse2, const float* __restrict__ delta, const int l_pad,
+                  const Problem p, const float* lse2, const float* delta, const int l_pad,
                   const int n_kblk, const int streams_per_wave, const long long wait_limit) {
   using C = BCfg<D>;
   extern __shared__ uint8_t smem_raw[];
@@ -579,10 +582,6 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
-
-  // the dQ kernel (a programmatic dependent launch that does not read anything this kernel writes) may be
-  // placed on SMs as soon as every CTA of this grid is resident
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   // Earliest key blocks (seen by the most query tiles under a causal mask) first, within waves of
   // `streams_per_wave` (batch, kv head) groups whose query-side operands fit in L2 together.
@@ -633,6 +632,12 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     tmem_alloc(smem_u32(&sync->tmem_base), kTmemCols);
     tmem_relinquish();
   }
+  // A programmatic dependent of the prep kernel.  Everything above, the copies of K and V too, may run before that
+  // grid is done: it writes the row statistics only, and its own wait was over before this grid could start.  The
+  // dQ kernel reads the statistics without a wait of its own and nothing that this kernel writes, so it may start
+  // once every CTA of this grid is past the wait.
+  pdl_wait();
+  pdl_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -925,14 +930,9 @@ int launch_bwd_prep(const BwdProblem& bp, bool bf16, float* lse2, float* delta, 
   const long long blocks = (warps * 32 + 255) / 256;
   if (blocks > 0x7fffffffLL) return B200_SDPA_ERR_UNSUPPORTED;
   const unsigned grid = static_cast<unsigned>(blocks);
-  if (bf16) {
-    if (vec) bwd_prep_kernel<__nv_bfloat16, true><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
-    else bwd_prep_kernel<__nv_bfloat16, false><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
-  } else {
-    if (vec) bwd_prep_kernel<__half, true><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
-    else bwd_prep_kernel<__half, false><<<grid, 256, 0, stream>>>(bp, lse2, delta, l_pad);
-  }
-  if (cudaGetLastError() != cudaSuccess) return B200_SDPA_ERR_CUDA;
+  auto kern = bf16 ? (vec ? bwd_prep_kernel<__nv_bfloat16, true> : bwd_prep_kernel<__nv_bfloat16, false>)
+                   : (vec ? bwd_prep_kernel<__half, true> : bwd_prep_kernel<__half, false>);
+  if (!launch_pdl(kern, dim3(grid), 256, 0, stream, bp, lse2, delta, l_pad)) return B200_SDPA_ERR_CUDA;
   count_launch(KID_BWD_PREP);
   return B200_SDPA_OK;
 }
@@ -974,26 +974,15 @@ int launch_tc(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t stre
   // resident; the dQ kernel is a programmatic dependent launch, so its CTAs take the SMs the first kernel's
   // tail leaves idle.  It waits for the first kernel's completion only before it exits (stream order for
   // whatever follows).
-  kkv<<<static_cast<unsigned>(grid_kv), kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, tdo, tdk, tdv, p, lse2, delta,
-                                                                          l_pad, n_kblk, wave_kv, limit);
-  if (cudaGetLastError() != cudaSuccess) return B200_SDPA_ERR_CUDA;
-  count_launch(KID_BWD_DKV);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid_q));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = ACfg<D>::kSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   const float* c_lse2 = lse2;
   const float* c_delta = delta;
-  if (cudaLaunchKernelEx(&cfg, kq, tq, tk, tv, tdo, tdq, p, c_lse2, c_delta, l_pad, n_qblk, wave_q, limit) != cudaSuccess) {
-    cudaGetLastError();
+  if (!launch_pdl(kkv, dim3(static_cast<unsigned>(grid_kv)), kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, tdk, tdv, p, c_lse2,
+                  c_delta, l_pad, n_kblk, wave_kv, limit))
     return B200_SDPA_ERR_CUDA;
-  }
+  count_launch(KID_BWD_DKV);
+  if (!launch_pdl(kq, dim3(static_cast<unsigned>(grid_q)), kThreads, ACfg<D>::kSmemBytes, stream, tq, tk, tv, tdo, tdq, p, c_lse2,
+                  c_delta, l_pad, n_qblk, wave_q, limit))
+    return B200_SDPA_ERR_CUDA;
   count_launch(KID_BWD_DQ);
   return B200_SDPA_OK;
 }

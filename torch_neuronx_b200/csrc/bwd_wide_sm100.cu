@@ -100,8 +100,7 @@ struct WWork {
 template <int WALK, int E, int DV, bool BF16>
 __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap* tm_fv, const CUtensorMap* tm_long,
                                      const CUtensorMap* tm_short, const CUtensorMap* tm_out, const Problem& p,
-                                     const float* __restrict__ lse2, const float* __restrict__ delta, const int l_pad,
-                                     const long long wait_limit, const WWork w, uint8_t* smem_raw) {
+                                     const float* lse2, const float* delta, const int l_pad, const long long wait_limit, const WWork w, uint8_t* smem_raw) {
   using C = WCfg<WALK, E, DV>;
   constexpr int NT = C::kNT;
   const uint32_t tiles = smem_u32(smem_raw);
@@ -150,6 +149,10 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
   if (warp == kMmaWarp) {
     tmem_alloc(smem_u32(&sync->tmem_base), kTmemCols);
     tmem_relinquish();
+  }
+  if (WALK != kDQ) {   // as in bwd_sm100.cu: the row statistics are not read before the prep kernel is done
+    pdl_wait();
+    pdl_launch_dependents();
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -517,11 +520,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 bwd_wide_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                     const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                     const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
-                    const Problem p, const float* __restrict__ lse2, const float* __restrict__ delta, const int l_pad,
+                    const Problem p, const float* lse2, const float* delta, const int l_pad,
                     const int n_kblk, const int streams_per_wave, const long long wait_limit) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (!smem_aligned(smem_raw, p)) return;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   constexpr int NT = WCfg<kDK, E, DV>::kNT;
   // Earliest key blocks (seen by the most query tiles under a causal mask) first, within waves of groups whose
   // query-side operands fit in L2 together; neighbouring CTAs do dK and dV of the same keys.
@@ -591,26 +593,15 @@ int launch_wide(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t st
   const long long n_streams = static_cast<long long>(p.Hkv) * p.B;
   const int wave_q = kv_streams_per_wave(static_cast<long long>(p.S) * (E + DV) * 2, n_streams);
   const int wave_kv = kv_streams_per_wave(static_cast<long long>(p.L) * p.group * ((E + DV) * 2 + 8), n_streams);
-  kkv<<<static_cast<unsigned>(grid_kv), kThreads, kSmemKV, stream>>>(k_f, v_f, q_s, do_s, dk, dv, p, lse2, delta, l_pad, n_kblk,
-                                                                    wave_kv, limit);
-  if (cudaGetLastError() != cudaSuccess) return B200_SDPA_ERR_CUDA;
-  count_launch(KID_BWD_DKV);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(grid_q));
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmemQ;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   const float* c_lse2 = lse2;
   const float* c_delta = delta;
-  if (cudaLaunchKernelEx(&cfg, kq, q_f, do_f, k_s, v_s, dq, p, c_lse2, c_delta, l_pad, n_qblk, wave_q, limit) != cudaSuccess) {
-    cudaGetLastError();
+  if (!launch_pdl(kkv, dim3(static_cast<unsigned>(grid_kv)), kThreads, kSmemKV, stream, k_f, v_f, q_s, do_s, dk, dv, p, c_lse2, c_delta,
+                  l_pad, n_kblk, wave_kv, limit))
     return B200_SDPA_ERR_CUDA;
-  }
+  count_launch(KID_BWD_DKV);
+  if (!launch_pdl(kq, dim3(static_cast<unsigned>(grid_q)), kThreads, kSmemQ, stream, q_f, do_f, k_s, v_s, dq, p, c_lse2, c_delta, l_pad,
+                  n_qblk, wave_q, limit))
+    return B200_SDPA_ERR_CUDA;
   count_launch(KID_BWD_DQ);
   return B200_SDPA_OK;
 }
