@@ -383,7 +383,7 @@ int b200_sdpa_fwd(const B200SdpaParams* params, void* stream) {
     path = prefill_eligible(p, params->dtype, &unused) ? B200_SDPA_PATH_PREFILL : B200_SDPA_PATH_GENERIC;
   }
   if (path == B200_SDPA_PATH_PREFILL) return launch_prefill(p, params->dtype, params->workspace, params->workspace_bytes, st);
-  if (served_padded(params, p)) return launch_prefill_padded(p, params->dtype, st);
+  if (served_padded(params, p)) return launch_prefill_padded(p, params->dtype, params->workspace, params->workspace_bytes, st);
   if (served_fp32(params, p)) return launch_fp32_fwd(p, st);
   return launch_generic(p, params->dtype, st);
 }

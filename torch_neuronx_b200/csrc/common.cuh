@@ -114,7 +114,7 @@ bool prefill_eligible(const Problem& p, int dtype, bool* alignment_only_failure)
 // head dimensions between 64 and 128 on zero-filled 128-wide tiles
 bool prefill_padded_eligible(const Problem& p, int dtype);
 int plan_prefill_padded(const Problem& p, B200SdpaPlan* plan);
-int launch_prefill_padded(const Problem& p, int dtype, cudaStream_t stream);
+int launch_prefill_padded(const Problem& p, int dtype, void* workspace, uint64_t workspace_bytes, cudaStream_t stream);
 // persistent form of the prefill kernel (prefill_persistent_sm100.cu): head dimension 128, large problems
 bool prefill_persistent_wanted(const Problem& p);
 bool prefill_accumulate_eligible(const Problem& p);   // accumulating form: layout rules of (acc, acc_lse)

@@ -205,7 +205,10 @@ __device__ __forceinline__ ItemRec decode_item(const Problem& p, int idx, int n_
 
 // ACC: the accumulating form (a ring step folded into a running fp32 result).  A template parameter, not a
 // run-time branch: the softmax loop has no register to spare for state it does not use.
-template <int D, bool BF16, bool BIAS, bool ACC>
+// PAD: head dimensions E, Dv (multiples of 8) that do not fill the D = 128 tile, as in prefill_sm100.cu: the copies
+// fill the tile with zeros, the products stop at ceil(E / 16) k-steps and ceil(Dv / 16) * 16 output columns, the
+// epilogue stores Dv columns, and P is kept as hi + lo (remainder2), lo in the second half of the columns of S.
+template <int D, bool BF16, bool BIAS, bool ACC, bool PAD>
 __global__ void __launch_bounds__(kThreads, 1)
 prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const Problem p, const int n_qblk, const int pair_heads,
@@ -262,6 +265,10 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     tmem_alloc(smem_u32(&sync->tmem_base), kTmemCols);
     tmem_relinquish();
   }
+  // A programmatic dependent of what precedes it in the stream: everything above ran under that kernel's tail, and
+  // nothing of global memory is touched before the wait returns.
+  pdl_wait();
+  pdl_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -294,8 +301,10 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         // tensor cores, which covers the round trip of the atomic).  Drawing earlier would tie the next
         // item to a CTA that may still be busy for a long time while others run dry.
         auto fetch = [&](int k) -> int {
-          const unsigned int i = next_item != nullptr ? atomicAdd(next_item, 1u)
-                                                      : blockIdx.x + static_cast<unsigned int>(k) * gridDim.x;
+          // without a counter: rounds over the list, every other one backwards, so that a CTA with a long item
+          // of one round gets a short one of the next
+          const unsigned int c = (k & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+          const unsigned int i = next_item != nullptr ? atomicAdd(next_item, 1u) : c + static_cast<unsigned int>(k) * gridDim.x;
           return i < static_cast<unsigned int>(n_items) ? static_cast<int>(i) : -1;
         };
         for (int k = 0; alive; ++k) {
@@ -362,7 +371,8 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       // descriptors stay in the uniform datapath; one elected lane issues.  The tile
       // index is a compile-time constant everywhere for the same reason.
       constexpr uint32_t idesc_qk = make_idesc(BF16, false, kBlockM, kBlockN);
-      constexpr uint32_t idesc_pv = make_idesc(BF16, true, kBlockM, D);
+      const uint32_t idesc_pv = make_idesc(BF16, true, kBlockM, PAD ? (p.Dv + 15) / 16 * 16 : D);
+      const int qk_steps = PAD ? (p.E + 15) / 16 : D / 16;
       // descriptors: fixed fields once, then only the 16-byte-unit start address moves
       const uint64_t q_desc0 = smem_desc_sw128(q_smem[0], 16, 1024), q_desc1 = smem_desc_sw128(q_smem[1], 16, 1024);
       const uint64_t kv_desc_k = smem_desc_sw128(kv_smem, 16, 1024);          // K tile as K-major B operand
@@ -375,6 +385,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         if (elect_one() && dbg_tmem(p.status, DBG_PREFILL_PERSISTENT * 100 + 1, d_addr, tmem_base, 128, kTmemCols)) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
+            if (PAD && kk >= qk_steps) break;
             const uint64_t off = static_cast<uint64_t>(((kk >> 2) * kBoxBytes + (kk & 3) * 32) >> 4);
             mma_ss(d_addr, qd + off, kd + off, idesc_qk, kk > 0 ? 1u : 0u);
           }
@@ -393,6 +404,8 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           for (int kk = 0; kk < 4; ++kk) {
             mma_ts(d_addr, a_addr + static_cast<uint32_t>(kk * 8), vd + static_cast<uint64_t>(kk * (2048 >> 4)), idesc_pv,
                    kk > 0 ? 1u : acc0);
+            if (PAD)
+              mma_ts(d_addr, a_addr + static_cast<uint32_t>(64 + kk * 8), vd + static_cast<uint64_t>(kk * (2048 >> 4)), idesc_pv, 1u);
           }
         }
       };
@@ -582,7 +595,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         const uint32_t o_addr = tmem_base + lane_off + 256u + static_cast<uint32_t>(t) * D;
         // checked build: the columns drained below, and the row this thread is about to store
         if (!dbg_tmem(p.status, DBG_PREFILL_PERSISTENT * 100 + 4, o_addr, tmem_base, D, kTmemCols)) *abort_flag = 1;
-        const bool store_ok = dbg_bhrc(p.status, DBG_PREFILL_PERSISTENT * 100 + 5, it.b, p.B, head, p.Hq, row_ok ? row_g : 0, p.L, 0, D, p.Dv);
+        const bool store_ok = dbg_bhrc(p.status, DBG_PREFILL_PERSISTENT * 100 + 5, it.b, p.B, head, p.Hq, row_ok ? row_g : 0, p.L, 0, PAD ? p.Dv : D, p.Dv);
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
           uint32_t v[32];
@@ -614,6 +627,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           } else if (!ACC && row_ok && store_ok) {
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
+              if (PAD && c * 32 + u * 8 >= p.Dv) break;
               uint4 w;
               w.x = pack2<BF16>(__uint_as_float(v[8 * u]) * inv, __uint_as_float(v[8 * u + 1]) * inv);
               w.y = pack2<BF16>(__uint_as_float(v[8 * u + 2]) * inv, __uint_as_float(v[8 * u + 3]) * inv);
@@ -792,7 +806,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         uint64_t sum2[2] = {0ull, 0ull};           // two packed accumulators = four chains
 #pragma unroll
         for (int c = 0; c < kBlockN / 32; ++c) {
-          uint32_t pk[16];
+          uint32_t pk[16], lo[PAD ? 16 : 1];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
             float a0, a1;   // both exponents with one packed fma
@@ -801,8 +815,10 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             const float p1 = ex2(a1);
             sum2[(i >> 1) & 1] = f2_add(sum2[(i >> 1) & 1], f2_pack(p0, p1));
             pk[i >> 1] = pack2<BF16>(p0, p1);
+            if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(p0, p1, pk[i >> 1]);
           }
           tmem_st_32x16(p_addr + c * 16, pk);
+          if constexpr (PAD) tmem_st_32x16(p_addr + 64 + c * 16, lo);
           if (c == 1) {
             // first 64 keys of P are in TMEM: let P V start on them while the rest is computed
             tmem_st_wait();
@@ -924,14 +940,20 @@ PrefillGeom prefill_geometry(const Problem& p) {
   return g;
 }
 
-template <int D, bool BF16, bool BIAS, bool ACC>
+// With few items to a CTA the order hardly matters and the counter does: the memset that clears it is an operation of its
+// own in the stream and keeps the launch from being a programmatic dependent of the kernel before.  Measured (fixed
+// order / counter, us, head dimension 128 unless said): 2 x 32/8 x 1024 causal, 256 items, 36.8 / 39.0; 8 x 16 x 577, 384 items,
+// 50.0 / 51.2; but 16 x 16 x 577 at head dimension 80, 768 items, 84.9 / 80.0 and 4 x 32/8 x 4096, 2048 items, 609 / 496.
+bool items_in_fixed_order(const PrefillGeom& g) { return g.n_items < 3LL * kAssumedSms; }
+
+template <int D, bool BF16, bool BIAS, bool ACC, bool PAD = false>
 int launch_variant(const Problem& p, void* workspace, uint64_t workspace_bytes, cudaStream_t stream) {
   using C = Cfg<D>;
   CUtensorMap tq, tk, tv;
-  if (!make_map(&tq, p.q, BF16, D, p.L, p.Hq, p.B, p.qs) || !make_map(&tk, p.k, BF16, D, p.S, p.Hkv, p.B, p.ks) ||
-      !make_map(&tv, p.v, BF16, D, p.S, p.Hkv, p.B, p.vs))
+  if (!make_map(&tq, p.q, BF16, p.E, p.L, p.Hq, p.B, p.qs) || !make_map(&tk, p.k, BF16, p.E, p.S, p.Hkv, p.B, p.ks) ||
+      !make_map(&tv, p.v, BF16, p.Dv, p.S, p.Hkv, p.B, p.vs))
     return B200_SDPA_ERR_CUDA;
-  auto kern = prefill_persistent_kernel<D, BF16, BIAS, ACC>;
+  auto kern = prefill_persistent_kernel<D, BF16, BIAS, ACC, PAD>;
   // the opt-in to more than 48 KB of dynamic shared memory is a per-device attribute: set on every
   // launch (a cheap host-side call), so a process that drives several GPUs gets it on each of them
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) {
@@ -943,34 +965,25 @@ int launch_variant(const Problem& p, void* workspace, uint64_t workspace_bytes, 
   const int sms = sm_count();
   const int grid = g.n_items < sms ? static_cast<int>(g.n_items) : sms;
   // With scratch for one counter the items are handed out one at a time (longest first, whoever is free
-  // takes the next); without it every CTA takes items c, c + grid, c + 2 grid, ... of the same list.
+  // takes the next); without it, or where items_in_fixed_order() holds, every CTA has its own places in the list.
   unsigned int* counter = nullptr;
-  if (workspace != nullptr && workspace_bytes >= sizeof(unsigned int) && reinterpret_cast<uintptr_t>(workspace) % 4 == 0) {
+  if (!items_in_fixed_order(g) && workspace != nullptr && workspace_bytes >= sizeof(unsigned int) && reinterpret_cast<uintptr_t>(workspace) % 4 == 0) {
     counter = reinterpret_cast<unsigned int*>(workspace);
     if (cudaMemsetAsync(counter, 0, sizeof(unsigned int), stream) != cudaSuccess) {
       cudaGetLastError();
       return B200_SDPA_ERR_CUDA;
     }
   }
-  const int per_wave = kv_streams_per_wave(static_cast<long long>(p.S) * 2 * D * 2, static_cast<long long>(p.Hkv) * p.B);
-  kern<<<grid, kThreads, C::kSmemBytes, stream>>>(tq, tk, tv, p, g.n_qblk, g.pair_heads, per_wave,
-                                                  static_cast<int>(g.n_items), counter, wait_limit_cycles());
-  if (cudaGetLastError() != cudaSuccess) return B200_SDPA_ERR_CUDA;
+  const int per_wave = kv_streams_per_wave(static_cast<long long>(p.S) * (p.E + p.Dv) * 2, static_cast<long long>(p.Hkv) * p.B);
+  if (!launch_pdl(kern, dim3(static_cast<unsigned>(grid)), kThreads, C::kSmemBytes, stream, tq, tk, tv, p, g.n_qblk,
+                  g.pair_heads, per_wave, static_cast<int>(g.n_items), counter, wait_limit_cycles()))
+    return B200_SDPA_ERR_CUDA;
   count_launch(KID_PREFILL);
   return B200_SDPA_OK;
 }
 
 }  // namespace
 
-// How the two prefill kernels share the work.  What the persistent kernel saves is the cost of going from
-// one work item to the next (no CTA launch, set-up or tear-down; the next item's Q and first key tile
-// already in flight; the epilogue on its own warps); what it pays is a heavier steady state (sixteen warps
-// share the register file, and under a power cap it clocks a little lower).  Measured on one B200: with up
-// to 32 key tiles per item it is 3-5 % faster in bursts (8-14 % with a bias) and about 2 % slower when the
-// GPU sits at its power cap for seconds; with 256 key tiles per item (32768 keys, and the blocks of a ring
-// over 131072) the per-CTA kernel is 5 % faster either way.  So: head dimension 128, at least three items
-// per SM, and at most 64 key tiles per item.  B200_SDPA_PREFILL = "persistent" or "per_cta" overrides the
-// choice where both kernels can serve the request (for tests and measurements).
 // (acc, acc_lse) of the accumulating form: fp32 rows read and written as 16-byte pieces
 bool prefill_accumulate_eligible(const Problem& p) {
   if (p.E != 128 || p.Dv != 128 || p.acc == nullptr || p.acc_lse == nullptr || p.bias != nullptr) return false;
@@ -981,8 +994,22 @@ bool prefill_accumulate_eligible(const Problem& p) {
   return true;
 }
 
+// How the two prefill kernels share the work.  What the persistent kernel saves is the cost of going from
+// one work item to the next (no CTA launch, set-up or tear-down; the next item's Q and first key tile
+// already in flight; the epilogue on its own warps); what it pays is a heavier steady state (sixteen warps
+// share the register file, and under a power cap it clocks a little lower).  Measured on one B200: with up
+// to 32 key tiles per item it is 3-5 % faster in bursts (8-14 % with a bias) and about 2 % slower when the
+// GPU sits at its power cap for seconds; with 256 key tiles per item (32768 keys, and the blocks of a ring
+// over 131072) the per-CTA kernel is 5 % faster either way.  So: at least three items per SM and at most 64 key
+// tiles per item, or more than one item per SM and at most 16 key tiles (2 x 32/8 x 1024 causal, 256 items: 37.8 us
+// per CTA, 36.8 here; 8 x 32 x 256, 256 items: 33.7 / 29.6; at 64 key tiles 146.4 / 148.6).  Padded head dimensions
+// follow the same rule (fp16 16 x 16 x 577, head dimension 80: 92.2 / 80.0).  At head dimension 64 the exponentials
+// bound the loop and this form measured up to 15 % slower.  B200_SDPA_PREFILL = "persistent" or "per_cta" overrides the
+// choice where both kernels can serve the request (for tests and measurements).
 bool prefill_persistent_wanted(const Problem& p) {
-  if (p.E != 128 || p.Dv != 128) return false;
+  const int hi = p.E > p.Dv ? p.E : p.Dv;
+  if (hi <= 64 || hi > 128) return false;
+  if (p.acc_mode != 0 && !prefill_accumulate_eligible(p)) return false;
   const char* e = getenv("B200_SDPA_PREFILL");
   if (e != nullptr && e[0] == 'p' && e[1] == 'e' && e[2] == 'r' && e[3] == 's') return true;    // "persistent"
   if (e != nullptr && e[0] == 'p' && e[1] == 'e' && e[2] == 'r' && e[3] == '_') return false;   // "per_cta"
@@ -990,7 +1017,9 @@ bool prefill_persistent_wanted(const Problem& p) {
   // one item per CTA was the faster one at every block size measured (eight ranks' blocks: 272.7 ms against
   // 291.5 ms for this kernel).
   if (p.acc_mode != 0) return false;
-  return prefill_geometry(p).n_items >= 3LL * kAssumedSms && (p.S + kBlockN - 1) / kBlockN <= 64;
+  const long long items = prefill_geometry(p).n_items;
+  const int key_tiles = (p.S + kBlockN - 1) / kBlockN;
+  return (items >= 3LL * kAssumedSms && key_tiles <= 64) || (items > kAssumedSms && key_tiles <= 16);
 }
 
 void plan_prefill_persistent(const Problem& p, B200SdpaPlan* plan) {
@@ -1017,11 +1046,15 @@ int launch_prefill_persistent(const Problem& p, int dtype, void* workspace, uint
     return bf16 ? launch_variant<128, true, false, true>(p, workspace, workspace_bytes, stream)
                 : launch_variant<128, false, false, true>(p, workspace, workspace_bytes, stream);
   }
-  if (p.bias != nullptr)
-    return bf16 ? launch_variant<128, true, true, false>(p, workspace, workspace_bytes, stream)
-                : launch_variant<128, false, true, false>(p, workspace, workspace_bytes, stream);
-  return bf16 ? launch_variant<128, true, false, false>(p, workspace, workspace_bytes, stream)
-              : launch_variant<128, false, false, false>(p, workspace, workspace_bytes, stream);
+  auto run = [&](auto bf16_c, auto bias_c) {
+    constexpr bool kBf16 = decltype(bf16_c)::value, kBias = decltype(bias_c)::value;
+    if (p.E == 128 && p.Dv == 128) return launch_variant<128, kBf16, kBias, false>(p, workspace, workspace_bytes, stream);
+    return launch_variant<128, kBf16, kBias, false, true>(p, workspace, workspace_bytes, stream);
+  };
+  const std::true_type yes{};
+  const std::false_type no{};
+  if (p.bias != nullptr) return bf16 ? run(yes, yes) : run(no, yes);
+  return bf16 ? run(yes, no) : run(no, no);
 }
 
 }  // namespace b200

@@ -1137,6 +1137,10 @@ int plan_prefill(const Problem& p, int dtype, B200SdpaPlan* plan) {
 }
 
 int plan_prefill_padded(const Problem& p, B200SdpaPlan* plan) {
+  if (prefill_persistent_wanted(p)) {
+    plan_prefill_persistent(p, plan);
+    return B200_SDPA_OK;
+  }
   const int pair_heads = pair_heads_mode(p);
   const int rows = pair_heads ? kBlockM : kRowsPerCta;
   const long long grid = static_cast<long long>((p.L + rows - 1) / rows) * (p.Hq / (pair_heads ? 2 : 1)) * p.B;
@@ -1146,7 +1150,8 @@ int plan_prefill_padded(const Problem& p, B200SdpaPlan* plan) {
 }
 
 // The caller has checked prefill_padded_eligible().
-int launch_prefill_padded(const Problem& p, int dtype, cudaStream_t stream) {
+int launch_prefill_padded(const Problem& p, int dtype, void* workspace, uint64_t workspace_bytes, cudaStream_t stream) {
+  if (prefill_persistent_wanted(p)) return launch_prefill_persistent(p, dtype, workspace, workspace_bytes, stream);
   const bool bf16 = dtype == B200_SDPA_BF16;
   if (p.bias != nullptr)
     return bf16 ? launch_variant<128, true, true, false, true>(p, stream)
