@@ -172,14 +172,14 @@ class DeviceScope {
       return;
     }
     int want = device < 0 ? cur : device;
-    if (want != cur) {
-      if (cudaSetDevice(want) != cudaSuccess) {
-        cudaGetLastError();
-        rc_ = B200_SDPA_ERR_CUDA;
-        return;
-      }
-      restore_ = cur;
+    // also when it is the current one: a thread whose first CUDA call this is (autograd's, with all its memory from the
+    // allocator's cache) has no context yet, and the tensor-map encoder needs one
+    if (cudaSetDevice(want) != cudaSuccess) {
+      cudaGetLastError();
+      rc_ = B200_SDPA_ERR_CUDA;
+      return;
     }
+    if (want != cur) restore_ = cur;
     rc_ = is_sm100(want) ? B200_SDPA_OK : B200_SDPA_ERR_DEVICE;
   }
   ~DeviceScope() {
