@@ -52,6 +52,7 @@ int validate(const B200SdpaParams* a, Problem* p) {
   p->kv_lens = a->kv_lens;
   p->bias = a->bias;
   p->bias_dtype = a->bias_dtype;
+  p->bias_padded = 0;
   p->status = a->status;
   p->block_table = a->block_table;
   p->table_stride = a->block_table_stride;
@@ -146,6 +147,13 @@ int choose(const B200SdpaParams* a, const Problem& p, int* path) {
 // CUDA-core kernel (force_path).  Plans keep the name of the path; their geometry fields describe the kernel.
 bool served_padded(const B200SdpaParams* a, const Problem& p) {
   return a->force_path != B200_SDPA_PATH_GENERIC && prefill_padded_eligible(p, a->dtype);
+}
+// ... a bias that they cannot read where it is among it: they work on a copy in the first `bytes` of the scratch.  Not
+// for a handful of rows, which the CUDA-core kernel finishes in the time of the extra launches.  (With the copy the
+// padded tiles serve head dimensions 64 and 128 too: their hi + lo probabilities keep that kernel's accuracy.)
+bool served_packed(const B200SdpaParams* a, const Problem& p, void* base, Problem* packed, uint64_t* bytes) {
+  return a->force_path == B200_SDPA_PATH_AUTO && p.L >= 16 && bias_pack_geometry(p, a->dtype, base, packed, bytes) &&
+         prefill_padded_eligible(*packed, a->dtype);
 }
 bool served_padded(const B200SdpaBwdParams* a, const BwdProblem& bp) {
   return a->force_path != B200_SDPA_PATH_GENERIC && bwd_padded_eligible(bp, a->dtype);
@@ -261,6 +269,7 @@ int validate_bwd(const B200SdpaBwdParams* a, BwdProblem& bp) {
   p.kv_lens = a->kv_lens;
   p.bias = a->bias;
   p.bias_dtype = a->bias_dtype;
+  p.bias_padded = 0;
   p.status = a->status;
   p.block_table = nullptr;
   p.table_stride = 0;
@@ -354,6 +363,15 @@ int b200_sdpa_query_plan(const B200SdpaParams* params, B200SdpaPlan* plan) {
     plan->path = B200_SDPA_PATH_GENERIC;
     return rc;
   }
+  Problem packed;
+  uint64_t copy = 0;
+  if (served_packed(params, p, reinterpret_cast<void*>(256), &packed, &copy)) {   // (planning: any aligned address)
+    rc = plan_prefill_padded(packed, plan);
+    plan->path = B200_SDPA_PATH_GENERIC;
+    plan->launches += 1;
+    plan->workspace_bytes += copy;
+    return rc;
+  }
   if (served_fp32(params, p)) {
     plan_fp32_fwd(p, plan);
     return B200_SDPA_OK;
@@ -384,6 +402,13 @@ int b200_sdpa_fwd(const B200SdpaParams* params, void* stream) {
   }
   if (path == B200_SDPA_PATH_PREFILL) return launch_prefill(p, params->dtype, params->workspace, params->workspace_bytes, st);
   if (served_padded(params, p)) return launch_prefill_padded(p, params->dtype, params->workspace, params->workspace_bytes, st);
+  Problem packed;
+  uint64_t copy = 0;
+  if (params->workspace != nullptr && served_packed(params, p, params->workspace, &packed, &copy) && params->workspace_bytes >= copy) {
+    rc = launch_bias_pack(p, packed, params->dtype, st);
+    if (rc != B200_SDPA_OK) return rc;
+    return launch_prefill_padded(packed, params->dtype, static_cast<char*>(params->workspace) + copy, params->workspace_bytes - copy, st);
+  }
   if (served_fp32(params, p)) return launch_fp32_fwd(p, st);
   return launch_generic(p, params->dtype, st);
 }

@@ -30,6 +30,7 @@ struct Problem {
   const void* bias;
   int bias_dtype;
   int64_t bs[4];
+  int bias_padded;       // the bias is the copy of bias_pack.cu: its rows may be read up to a multiple of 16 elements
   int* status;
   // Paged key/value cache (decode only): when block_table is set, k and v point at page
   // pools, ks/vs hold (page, head, row-in-page, element) strides and key s of batch b lives
@@ -114,6 +115,8 @@ bool prefill_eligible(const Problem& p, int dtype, bool* alignment_only_failure)
 // head dimensions between 64 and 128 on zero-filled 128-wide tiles
 bool prefill_padded_eligible(const Problem& p, int dtype);
 int plan_prefill_padded(const Problem& p, B200SdpaPlan* plan);
+bool bias_pack_geometry(const Problem& p, int dtype, void* base, Problem* packed, uint64_t* bytes);
+int launch_bias_pack(const Problem& p, const Problem& packed, int dtype, cudaStream_t stream);
 int launch_prefill_padded(const Problem& p, int dtype, void* workspace, uint64_t workspace_bytes, cudaStream_t stream);
 // persistent form of the prefill kernel (prefill_persistent_sm100.cu): head dimension 128, large problems
 bool prefill_persistent_wanted(const Problem& p);

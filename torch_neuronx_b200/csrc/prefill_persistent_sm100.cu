@@ -43,6 +43,7 @@
 #include "debug.cuh"
 
 #include <cstdlib>
+#include <cstring>
 #include <type_traits>
 
 namespace b200 {
@@ -104,6 +105,15 @@ struct ItemRec {
   int lim0, lim1;          // visible-key count of each tile's first row (may be <= 0)
   int in_range;            // bit t: tile t starts inside L
   int kv_limit;
+  uint64_t tiles;          // (bias) the key tiles to visit, one bit each; 0: all of [0, max(nt0, nt1))
+};
+
+// Key tiles that an additive bias leaves visible: one bit per 128 x 128 tile that holds an element other than -inf,
+// one 64-bit word per 128 bias rows.  nullptr: not known, every tile is visited.
+struct TileLists {
+  const uint64_t* words;   // [bias batches][bias heads][row tiles]
+  int64_t batch_stride, head_stride;   // in words; 0 where the bias is broadcast
+  int row_stride;                      // 0 where one bias row serves all query rows, else 1
 };
 
 struct Sync {
@@ -169,9 +179,11 @@ __device__ __forceinline__ TileGeom tile_geometry(const Problem& p, int row0, in
 //   pair_heads == 1: the same 128 rows of two query heads that share a kv head
 //     (even group size) -- both tiles then see exactly the same keys, so under a
 //     causal mask neither waits for the other's extra diagonal tile.
-__device__ __forceinline__ ItemRec decode_item(const Problem& p, int idx, int n_qblk, int pair_heads, int streams_per_wave) {
+__device__ __forceinline__ ItemRec decode_item(const Problem& p, int idx, int n_qblk, int pair_heads, int streams_per_wave,
+                                               const TileLists& lists) {
   ItemRec it;
   it.idx = idx;
+  it.tiles = 0;
   const int heads_per_cta = pair_heads ? 2 : 1;
   const int ctas_per_stream = p.group / heads_per_cta;            // per query block
   const int n_streams = p.Hkv * p.B;
@@ -200,7 +212,30 @@ __device__ __forceinline__ ItemRec decode_item(const Problem& p, int idx, int n_
   it.lim0 = g0.min_lim;
   it.lim1 = g1.min_lim;
   it.in_range = (g0.in_range ? 1 : 0) | (g1.in_range ? 2 : 0);
+  if (lists.words != nullptr) {
+    // Both query tiles walk the union of their lists, each up to its own end: what one of them does not see of a
+    // tile of the other is masked element by element as before.
+    auto word = [&](int head, int row0) {
+      return lists.words[it.b * lists.batch_stride + head * lists.head_stride + row0 / kBlockM * lists.row_stride];
+    };
+    auto below = [](int n) { return n >= 64 ? ~0ull : (1ull << n) - 1; };
+    uint64_t seen = 0;
+    if (it.nt0 > 0) seen |= word(it.head0, it.row0_0) & below(it.nt0);
+    if (it.nt1 > 0) seen |= word(it.head1, it.row0_1) & below(it.nt1);
+    it.nt0 = __popcll(seen & below(it.nt0));
+    it.nt1 = __popcll(seen & below(it.nt1));
+    it.tiles = seen;
+  }
   return it;
+}
+
+// The key tile after `j`: the lowest bit of `rest`, which it loses, or j + 1 where there is no list.
+template <bool BIAS>
+__device__ __forceinline__ int next_tile(int j, uint64_t& rest) {
+  if (!BIAS || rest == 0) return j + 1;
+  const int t = __ffsll(static_cast<long long>(rest)) - 1;
+  rest &= rest - 1;
+  return t;
 }
 
 // ACC: the accumulating form (a ring step folded into a running fp32 result).  A template parameter, not a
@@ -213,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                const __grid_constant__ CUtensorMap tm_v, const Problem p, const int n_qblk, const int pair_heads,
                const int streams_per_wave, const int n_items, unsigned int* __restrict__ next_item,
-               const long long wait_limit) {
+               const long long wait_limit, const TileLists lists) {
   using C = Cfg<D>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t tiles = smem_u32(smem_raw);                     // tile area: 1024-byte aligned (swizzled TMA boxes)
@@ -319,7 +354,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           }
           ItemRec it;
           it.idx = -1;
-          if (idx >= 0) it = decode_item(p, idx, n_qblk, pair_heads, streams_per_wave);
+          if (idx >= 0) it = decode_item(p, idx, n_qblk, pair_heads, streams_per_wave, BIAS ? lists : TileLists{});
           sync->item[slot] = it;
           mbar_arrive(smem_u32(&sync->item_full[slot]));
           if (idx < 0) break;
@@ -343,8 +378,10 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                           t == 0 ? it.head0 : it.head1, it.b);
             ++q_loads[t];
           }
+          uint64_t rest = it.tiles;   // key tiles not yet requested
+          int j = -1;
           for (int item = 0; item < 2 * n_iter && alive; ++item) {
-            const int j = item >> 1;
+            if ((item & 1) == 0) j = next_tile<BIAS>(j, rest);
             const int stage = ring_pos % C::kStages;
             const uint32_t round = static_cast<uint32_t>(ring_pos / C::kStages);
             if (round > 0) {
@@ -705,11 +742,14 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                                                     static_cast<long long>(row_g) * p.bs[2]);
       }
 
+      uint64_t rest = it.tiles;
+      int key_tile = -1;
       for (int j = 0; j < n_tiles; ++j) {
+        key_tile = next_tile<BIAS>(key_tile, rest);
         uint4 bv[BIAS ? kBlockN / 8 : 1];
         if constexpr (BIAS) {
           // the bias of this key tile travels while the scores are awaited
-          load_bias_row(bv, bias_row, j * kBlockN, p.S, bias_wide);
+          load_bias_row(bv, bias_row, key_tile * kBlockN, p.S, bias_wide);
         }
         bool ok = wait_clocked(smem_u32(&sync->s_full[t]), n_s & 1, abort_flag, wait_limit);
         ok = __all_sync(0xffffffffu, ok);
@@ -719,7 +759,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           break;
         }
         tc_fence_after_sync();
-        const int col0 = j * kBlockN;
+        const int col0 = key_tile * kBlockN;
         const bool need_mask = col0 + kBlockN > min_lim;
 
         // S row -> registers in two halves; the second half is in flight while the
@@ -946,6 +986,81 @@ PrefillGeom prefill_geometry(const Problem& p) {
 // 50.0 / 51.2; but 16 x 16 x 577 at head dimension 80, 768 items, 84.9 / 80.0 and 4 x 32/8 x 4096, 2048 items, 609 / 496.
 bool items_in_fixed_order(const PrefillGeom& g) { return g.n_items < 3LL * kAssumedSms; }
 
+// One CTA per 128 bias rows: which of its key tiles (at most 64) hold an element other than -inf.  The warps share the
+// tiles, or split the rows of each; a visible tile usually ends at its first two rows, a hidden one is read whole,
+// which is what the attention kernel then need not do.  Also clears that kernel's item counter.
+constexpr int kListThreads = 1024;
+
+__global__ void __launch_bounds__(kListThreads) bias_tiles_kernel(const Problem p, uint64_t* words, const int row_stride,
+                                                                  unsigned int* counter, const int n_heads, const int n_row_tiles,
+                                                                  const uint32_t hidden) {
+  __shared__ unsigned int seen[64];
+  const int rt = blockIdx.x % n_row_tiles;
+  const int h = blockIdx.x / n_row_tiles % n_heads;
+  const int b = blockIdx.x / n_row_tiles / n_heads;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < 64) seen[threadIdx.x] = 0;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *counter = 0;
+  __syncthreads();
+  const int n_tiles = (p.S + kBlockN - 1) / kBlockN;
+  const int row0 = rt * kBlockM;
+  const int n_rows = row_stride == 0 ? 1 : (p.L - row0 < kBlockM ? p.L - row0 : kBlockM);
+  int parts = kListThreads / 32 / n_tiles;
+  parts = parts < 1 ? 1 : (parts > 8 ? 8 : parts);
+  const int part_rows = 16 * ((8 + parts - 1) / parts);
+  const uint16_t* base = static_cast<const uint16_t*>(p.bias) + b * p.bs[0] + h * p.bs[1] + static_cast<int64_t>(row0) * p.bs[2];
+  for (int unit = warp; unit < n_tiles * parts; unit += kListThreads / 32) {
+    const int tile = unit / parts;
+    const int r0 = unit % parts * part_rows, r1 = r0 + part_rows < n_rows ? r0 + part_rows : n_rows;
+    const int col = tile * kBlockN + (lane & 15) * 8;   // rows start on 16 bytes and are readable up to a multiple of 8
+    bool any = false;
+    for (int r = r0, step = 2; r < r1 && !any; r += step, step = 16) {
+      uint4 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int row = r + 2 * i + (lane >> 4);
+        v[i] = make_uint4(hidden, hidden, hidden, hidden);
+        if (2 * i < step && row < r1 && col < p.S) v[i] = *reinterpret_cast<const uint4*>(base + row * p.bs[2] + col);
+      }
+      bool mine = false;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mine |= v[i].x != hidden || v[i].y != hidden || v[i].z != hidden || v[i].w != hidden;
+      any = __any_sync(0xffffffffu, mine);
+    }
+    if (any && lane == 0) atomicOr(&seen[tile], 1u);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const unsigned int lo = __ballot_sync(0xffffffffu, seen[lane] != 0), hi = __ballot_sync(0xffffffffu, seen[32 + lane] != 0);
+    if (lane == 0) words[blockIdx.x] = lo | (static_cast<uint64_t>(hi) << 32);
+  }
+}
+
+// Where the bias is looked over first: up to the 64 key tiles that a word holds, and where a CTA has at least eight
+// tile steps (2 us each) in front of it, against the launch's 5-8 (1 x 8 x 512, four steps: 23.4 us without, 31.7 with;
+// 4 x 12 x 1024, head dimension 64, a causal bias, 16 steps: 69.6 / 50.2; 2 x 32/8 x 2048 with a window of 512, 64 steps: 259 / 120).
+// Counter and words share the scratch.
+struct ListGeom {
+  int n_batches, n_heads, n_row_tiles;
+  uint64_t bytes;          // 0: no lists
+};
+ListGeom list_geometry(const Problem& p) {
+  ListGeom g{1, 1, 1, 0};
+  const int n_tiles = (p.S + kBlockN - 1) / kBlockN;
+  if (p.bias == nullptr || n_tiles > 64) return g;
+  const char* mode = getenv("B200_SDPA_PREFILL");
+  const bool forced = mode != nullptr && strncmp(mode, "pers", 4) == 0;
+  if (!forced && (prefill_geometry(p).n_items + kAssumedSms - 1) / kAssumedSms * n_tiles < 8) return g;
+  if (p.bs[0] != 0) g.n_batches = p.B;
+  if (p.bs[1] != 0) g.n_heads = p.Hq;
+  if (p.bs[2] != 0) g.n_row_tiles = (p.L + kBlockM - 1) / kBlockM;
+  const int64_t n = static_cast<int64_t>(g.n_batches) * g.n_heads * g.n_row_tiles;
+  if (n <= 0x7fffffffLL) g.bytes = 16 + 8 * static_cast<uint64_t>(n);
+  return g;
+}
+
 template <int D, bool BF16, bool BIAS, bool ACC, bool PAD = false>
 int launch_variant(const Problem& p, void* workspace, uint64_t workspace_bytes, cudaStream_t stream) {
   using C = Cfg<D>;
@@ -967,7 +1082,20 @@ int launch_variant(const Problem& p, void* workspace, uint64_t workspace_bytes, 
   // With scratch for one counter the items are handed out one at a time (longest first, whoever is free
   // takes the next); without it, or where items_in_fixed_order() holds, every CTA has its own places in the list.
   unsigned int* counter = nullptr;
-  if (!items_in_fixed_order(g) && workspace != nullptr && workspace_bytes >= sizeof(unsigned int) && reinterpret_cast<uintptr_t>(workspace) % 4 == 0) {
+  TileLists lists{};
+  const ListGeom lg = list_geometry(p);
+  if (BIAS && lg.bytes != 0 && workspace != nullptr && workspace_bytes >= lg.bytes && reinterpret_cast<uintptr_t>(workspace) % 8 == 0) {
+    counter = reinterpret_cast<unsigned int*>(workspace);
+    uint64_t* words = reinterpret_cast<uint64_t*>(workspace) + 2;
+    lists.words = words;
+    lists.row_stride = lg.n_row_tiles > 1 ? 1 : 0;
+    lists.head_stride = lg.n_heads > 1 ? lg.n_row_tiles : 0;
+    lists.batch_stride = lg.n_batches > 1 ? static_cast<int64_t>(lg.n_row_tiles) * lg.n_heads : 0;
+    const unsigned blocks = static_cast<unsigned>(static_cast<int64_t>(lg.n_batches) * lg.n_heads * lg.n_row_tiles);
+    if (!launch_pdl(bias_tiles_kernel, dim3(blocks), kListThreads, 0, stream, p, words, p.bs[2] != 0 ? 1 : 0, counter, lg.n_heads,
+                    lg.n_row_tiles, BF16 ? 0xff80ff80u : 0xfc00fc00u))
+      return B200_SDPA_ERR_CUDA;
+  } else if (!items_in_fixed_order(g) && workspace != nullptr && workspace_bytes >= sizeof(unsigned int) && reinterpret_cast<uintptr_t>(workspace) % 4 == 0) {
     counter = reinterpret_cast<unsigned int*>(workspace);
     if (cudaMemsetAsync(counter, 0, sizeof(unsigned int), stream) != cudaSuccess) {
       cudaGetLastError();
@@ -976,7 +1104,7 @@ int launch_variant(const Problem& p, void* workspace, uint64_t workspace_bytes, 
   }
   const int per_wave = kv_streams_per_wave(static_cast<long long>(p.S) * (p.E + p.Dv) * 2, static_cast<long long>(p.Hkv) * p.B);
   if (!launch_pdl(kern, dim3(static_cast<unsigned>(grid)), kThreads, C::kSmemBytes, stream, tq, tk, tv, p, g.n_qblk,
-                  g.pair_heads, per_wave, static_cast<int>(g.n_items), counter, wait_limit_cycles()))
+                  g.pair_heads, per_wave, static_cast<int>(g.n_items), counter, wait_limit_cycles(), lists))
     return B200_SDPA_ERR_CUDA;
   count_launch(KID_PREFILL);
   return B200_SDPA_OK;
@@ -1001,14 +1129,16 @@ bool prefill_accumulate_eligible(const Problem& p) {
 // to 32 key tiles per item it is 3-5 % faster in bursts (8-14 % with a bias) and about 2 % slower when the
 // GPU sits at its power cap for seconds; with 256 key tiles per item (32768 keys, and the blocks of a ring
 // over 131072) the per-CTA kernel is 5 % faster either way.  So: at least three items per SM and at most 64 key
-// tiles per item, or more than one item per SM and at most 16 key tiles (2 x 32/8 x 1024 causal, 256 items: 37.8 us
+// tiles per item, or more than one item per SM and at most 8 key tiles (2 x 32/8 x 1024 causal, 256 items: 37.8 us
 // per CTA, 36.8 here; 8 x 32 x 256, 256 items: 33.7 / 29.6; at 64 key tiles 146.4 / 148.6).  Padded head dimensions
 // follow the same rule (fp16 16 x 16 x 577, head dimension 80: 92.2 / 80.0).  At head dimension 64 the exponentials
-// bound the loop and this form measured up to 15 % slower.  B200_SDPA_PREFILL = "persistent" or "per_cta" overrides the
+// bound the loop and this form measured up to 15 % slower; it serves those shapes only with a bias whose hidden key
+// tiles it can leave out.  B200_SDPA_PREFILL = "persistent" or "per_cta" overrides the
 // choice where both kernels can serve the request (for tests and measurements).
 bool prefill_persistent_wanted(const Problem& p) {
   const int hi = p.E > p.Dv ? p.E : p.Dv;
-  if (hi <= 64 || hi > 128) return false;
+  if (hi < 64 || hi > 128) return false;
+  if (p.E == 64 && p.Dv == 64 && list_geometry(p).bytes == 0) return false;
   if (p.acc_mode != 0 && !prefill_accumulate_eligible(p)) return false;
   const char* e = getenv("B200_SDPA_PREFILL");
   if (e != nullptr && e[0] == 'p' && e[1] == 'e' && e[2] == 'r' && e[3] == 's') return true;    // "persistent"
@@ -1017,9 +1147,10 @@ bool prefill_persistent_wanted(const Problem& p) {
   // one item per CTA was the faster one at every block size measured (eight ranks' blocks: 272.7 ms against
   // 291.5 ms for this kernel).
   if (p.acc_mode != 0) return false;
+  if (list_geometry(p).bytes != 0) return true;   // leaving out hidden key tiles is worth more than the choice of kernel
   const long long items = prefill_geometry(p).n_items;
   const int key_tiles = (p.S + kBlockN - 1) / kBlockN;
-  return (items >= 3LL * kAssumedSms && key_tiles <= 64) || (items > kAssumedSms && key_tiles <= 16);
+  return (items >= 3LL * kAssumedSms && key_tiles <= 64) || (items > kAssumedSms && key_tiles <= 8);
 }
 
 void plan_prefill_persistent(const Problem& p, B200SdpaPlan* plan) {
@@ -1030,11 +1161,13 @@ void plan_prefill_persistent(const Problem& p, B200SdpaPlan* plan) {
   plan->grid_x = static_cast<int32_t>(g.n_items < kAssumedSms ? g.n_items : kAssumedSms);
   plan->grid_y = plan->grid_z = 1;
   plan->threads = kThreads;
-  plan->smem_bytes = Cfg<128>::kSmemBytes;
+  plan->smem_bytes = p.E == 64 && p.Dv == 64 ? Cfg<64>::kSmemBytes : Cfg<128>::kSmemBytes;
   plan->kv_splits = 1;
-  plan->launches = 1;
-  // optional: with 16 bytes of scratch the CTAs draw their work items from a shared counter
-  plan->workspace_bytes = 16;
+  // optional: with 16 bytes of scratch the CTAs draw their work items from a shared counter, with more they skip the
+  // key tiles that a bias hides
+  const uint64_t lists = list_geometry(p).bytes;
+  plan->launches = lists != 0 ? 2 : 1;
+  plan->workspace_bytes = lists != 0 ? lists : 16;
 }
 
 // The caller has checked prefill_eligible() and prefill_persistent_wanted().
@@ -1048,7 +1181,10 @@ int launch_prefill_persistent(const Problem& p, int dtype, void* workspace, uint
   }
   auto run = [&](auto bf16_c, auto bias_c) {
     constexpr bool kBf16 = decltype(bf16_c)::value, kBias = decltype(bias_c)::value;
-    if (p.E == 128 && p.Dv == 128) return launch_variant<128, kBf16, kBias, false>(p, workspace, workspace_bytes, stream);
+    if constexpr (kBias) {
+      if (p.E == 64 && p.Dv == 64 && !p.bias_padded) return launch_variant<64, kBf16, true, false>(p, workspace, workspace_bytes, stream);
+    }
+    if (p.E == 128 && p.Dv == 128 && !p.bias_padded) return launch_variant<128, kBf16, kBias, false>(p, workspace, workspace_bytes, stream);
     return launch_variant<128, kBf16, kBias, false, true>(p, workspace, workspace_bytes, stream);
   };
   const std::true_type yes{};

@@ -1106,8 +1106,9 @@ bool prefill_eligible(const Problem& p, int dtype, bool* alignment_only_failure)
 // dimension 80): CUDA-core kernel 2463 us, these tiles 79 us with a 16-bit P, 92 us with hi + lo.
 bool prefill_padded_eligible(const Problem& p, int dtype) {
   const int hi = p.E > p.Dv ? p.E : p.Dv;
-  if (hi <= 64 || hi > 128 || p.E % 8 != 0 || p.Dv % 8 != 0) return false;
-  if (p.E == p.Dv && p.E == 128) return false;
+  if (hi < 64 || hi > 128 || p.E % 8 != 0 || p.Dv % 8 != 0) return false;
+  if (p.E == p.Dv && (p.E == 128 || p.E == 64) && !p.bias_padded) return false;
+  if (hi == 64 && !p.bias_padded) return false;
   if (p.block_table != nullptr || p.k_new != nullptr || p.acc_mode != 0) return false;
   return operands_eligible(p, dtype, nullptr);
 }

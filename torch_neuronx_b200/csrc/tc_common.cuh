@@ -213,7 +213,7 @@ __device__ __forceinline__ uint32_t remainder2(float x0, float x1, uint32_t hi) 
 // One thread's 8 N bias elements (16-bit) of a key tile: N 16-byte pieces, fetched as N / 2
 // 32-byte loads when the row allows it (`wide`: the row start and the key offset on a 32-byte
 // boundary) -- every thread reads its own row, so the number of load instructions is what the
-// load/store unit feels.  Pieces at or beyond `n_cols` (a multiple of 8) read as zero.  The loads bypass L1
+// load/store unit feels.  Pieces at or beyond `n_cols` read as zero (a piece that straddles it is read whole).  The loads bypass L1
 // (every byte is read once): the softmax loop's spilled registers live there and must not be evicted.
 template <int N>
 __device__ __forceinline__ void load_bias_row(uint4 (&bv)[N], const uint4* row, const int col0, const int n_cols,
@@ -278,7 +278,7 @@ __device__ __forceinline__ void add_bias8(uint32_t* sv, const uint4 bias, const 
 // unit stride along the keys, a key count that is a multiple of 8, every row start on a 16-byte
 // boundary (broadcast dimensions have stride 0).
 inline bool bias_readable(const Problem& p, int dtype, bool* alignment_only_failure) {
-  if (p.bias_dtype != dtype || p.bs[3] != 1 || p.S % 8 != 0) return false;
+  if (p.bias_dtype != dtype || p.bs[3] != 1 || (p.S % 8 != 0 && !p.bias_padded)) return false;
   if (reinterpret_cast<uintptr_t>(p.bias) % 16 != 0 || p.bs[0] % 8 != 0 || p.bs[1] % 8 != 0 || p.bs[2] % 8 != 0) {
     if (alignment_only_failure) *alignment_only_failure = true;
     return false;
