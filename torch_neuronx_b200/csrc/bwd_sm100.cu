@@ -19,8 +19,9 @@
 // in exchange dQ needs neither atomics nor an fp32 scratch tensor, and results are
 // deterministic.  Arithmetic: torch_neuronx/_sdpa_math.py:133-176 with P and dS rounded
 // to the input dtype before their second product (upstream rounds P the same way in the
-// forward, :94).  Roles per CTA (320 threads): warps 0-7 elementwise (two threads per TMEM
-// lane, 64 score columns each), warp 8 TMA producer, warp 9 MMA issuer.
+// forward, :94).  Roles per CTA (576 threads): warps 0-15 elementwise (four threads per TMEM
+// lane, 32 score columns each: four warps per scheduler hide one another's tensor-memory and
+// barrier latency), warp 16 TMA producer, warp 17 MMA issuer.
 //
 // The dK/dV kernel's tensor memory is full with one pair of score-shaped accumulators:
 //   TMEM columns  [0,128) S^T, P^T over it   [128,256) dP^T, dS^T over it   [256, 256+2D) dV and dK (fp32)
@@ -29,7 +30,6 @@
 // in which the MMA pipe touches the shared columns):
 //   elementwise  P^T(i) from S^T(i)        dS^T(i) from P^T(i), dP^T(i)
 //   MMA          dK(i-1), dP^T(i)          dV(i), S^T(i+1)
-// At D = 64 there is room for a second S^T, and no wait of the elementwise role for the products between.
 // Whole 128-row query tiles: a score product with 64 columns costs the tensor pipe as much as one with 128 (its A
 // operand is fetched from shared memory either way).  Measured, 1 x 32/8 x 4096, no mask: 3350 cycles per tile against
 // 4024 for two 64-column units, of which the products take 2048 and the exponentials 1024 of the MUFU.
@@ -45,10 +45,8 @@ namespace {
 using namespace ptx;
 using namespace tc;
 
-constexpr int kEWarps = 8;                // elementwise role: two column halves x four lane quadrants
-constexpr int kParts = kEWarps / 4;
-constexpr int kQ = kT / kParts;           // score columns of one thread, in chunks of 32
-constexpr int kChunks = kQ / 32;
+constexpr int kEWarps = 16;               // elementwise role: four column quarters x four lane quadrants
+constexpr int kQ = kT / 4;                // score columns of one thread
 constexpr int kThreads = (kEWarps + 2) * 32;
 constexpr uint32_t kColS = 0, kColDP = 128, kColAcc = 256;   // TMEM layout of the dK/dV kernel
 constexpr int kProducerWarp = kEWarps;
@@ -69,7 +67,7 @@ struct BSync {
   uint64_t fixed_full;
   uint64_t ring_full[kMaxStages];
   uint64_t ring_empty[kMaxStages];
-  uint64_t s_full[2];   // S^T of a tile is complete (per buffer)
+  uint64_t s_full;      // S^T of a tile is complete
   uint64_t dp_full;     // dP^T of a tile is complete
   uint64_t p_ready;     // the elementwise role has written P^T (16-bit, over S^T)
   uint64_t ds_ready;    // ... and dS^T (over dP^T)
@@ -135,17 +133,6 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const BwdProblem bp, floa
   }
 }
 
-// This thread's score columns to registers; 16-bit operands back, chunk c at + STEP c.
-__device__ __forceinline__ void ld_chunks(uint32_t addr, uint32_t (&v)[kQ]) {
-#pragma unroll
-  for (int c = 0; c < kChunks; ++c) tmem_ld_32x32(addr + c * 32, reinterpret_cast<uint32_t(&)[32]>(v[c * 32]));
-}
-template <int STEP>
-__device__ __forceinline__ void st_chunks(uint32_t addr, const uint32_t (&v)[kQ / 2]) {
-#pragma unroll
-  for (int c = 0; c < kChunks; ++c) tmem_st_32x16(addr + c * STEP, reinterpret_cast<const uint32_t(&)[16]>(v[c * 16]));
-}
-
 // acc[tmem d, 128 x 128] = A[smem tile, K-major] * B[smem tile, K-major]^T over D
 // (PAD: only the first `steps` of the D / 16 k-steps, the columns beyond hold zeros)
 template <int D, bool PAD>
@@ -159,10 +146,10 @@ __device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint32_t a_tile, uint3
     }
   }
 }
-// acc[tmem d] (+)= A[tmem, 128 x 128] * B[smem tile, MN-major].  The 16-bit A operand sits where the elementwise
-// role left it: contraction indices 32 c .. 32 c + 31 packed into columns [32 c, 32 c + 16) of the score-shaped
-// buffer they came from.  PAD: the other 16 columns hold the remainders of that rounding (remainder2), a second set of
-// products.
+// acc[tmem d] (+)= A[tmem, 128 x 128] * B[smem tile, MN-major].  The 16-bit A operand sits where the four column
+// quarters of the elementwise role left it: contraction indices 32 q .. 32 q + 31 packed into columns
+// [32 q, 32 q + 16) of the score-shaped buffer they came from.  PAD: the quarter's other 16 columns hold the remainders
+// of that rounding (remainder2), a second set of products.
 template <bool PAD>
 __device__ __forceinline__ void issue_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_tile, uint32_t idesc, bool accumulate) {
   const uint64_t bd = mnmajor_desc(b_tile);
@@ -177,8 +164,7 @@ __device__ __forceinline__ void issue_ts(uint32_t d_tmem, uint32_t a_tmem, uint3
 }
 
 __device__ __forceinline__ void init_common_barriers(BSync* sync) {
-  mbar_init(smem_u32(&sync->s_full[0]), 1);
-  mbar_init(smem_u32(&sync->s_full[1]), 1);
+  mbar_init(smem_u32(&sync->s_full), 1);
   mbar_init(smem_u32(&sync->dp_full), 1);
   mbar_init(smem_u32(&sync->p_ready), kEWarps);
   mbar_init(smem_u32(&sync->ds_ready), kEWarps);
@@ -448,11 +434,11 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   } else {
     // -------------------------------------------------------- elementwise role
     const int r = tid & (kT - 1);              // query row inside the tile = TMEM lane
-    const int part = warp >> 2;                // which 64 of the tile's 128 score columns
+    const int quarter = warp >> 2;             // which 32 of the tile's 128 score columns
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t s_addr = tmem_base + lane_off + kColS + part * kQ;
-    const uint32_t dp_addr = tmem_base + lane_off + kColDP + part * kQ;
-    const uint32_t op_addr = tmem_base + lane_off + kColOp + part * (kQ / 2);
+    const uint32_t s_addr = tmem_base + lane_off + kColS + quarter * kQ;
+    const uint32_t dp_addr = tmem_base + lane_off + kColDP + quarter * kQ;
+    const uint32_t op_addr = tmem_base + lane_off + kColOp + quarter * (kQ / 2);
     const uint32_t dq_addr = tmem_base + lane_off + kColDQ;
     // checked build: the column ranges of this thread's tensor-memory traffic; a violation drains the CTA
     if (!dbg_tmem(p.status, DBG_BWD_TC * 100 + 2, s_addr, tmem_base, kQ, kTmemCols) || !dbg_tmem(p.status, DBG_BWD_TC * 100 + 3, dp_addr, tmem_base, kQ, kTmemCols) ||
@@ -482,7 +468,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     for (int j = 0; j < n_tiles; ++j) {
       const int buf = j % kBufs;
       uint4 bv[BIAS ? kQ / 8 : 1];   // this thread's bias elements of the tile, fetched under the wait
-      if constexpr (BIAS) load_bias_row(bv, bias_row, j * kT + part * kQ, p.S, bias_wide);
+      if constexpr (BIAS) load_bias_row(bv, bias_row, j * kT + quarter * kQ, p.S, bias_wide);
       const uint32_t* bw = reinterpret_cast<const uint32_t*>(bv);
       bool ok = wait_clocked(smem_u32(&sync->sp_full), j & 1, abort_flag, wait_limit);
       ok = __all_sync(0xffffffffu, ok);
@@ -493,12 +479,12 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       tc_fence_after_sync();
       uint32_t sv[kQ], dv[kQ];
-      ld_chunks(s_addr, sv);
-      ld_chunks(dp_addr, dv);
+      tmem_ld_32x32(s_addr, sv);
+      tmem_ld_32x32(dp_addr, dv);
       tmem_ld_wait();
       tc_fence_before_sync();
       warp_arrive(&sync->f_free, lane);
-      const int col0 = j * kT + part * kQ;
+      const int col0 = j * kT + quarter * kQ;
       const bool need_mask = col0 + kQ > min_lim;
       uint32_t pk[kQ / 2], lo[PAD ? kQ / 2 : 1];
       // two columns per instruction (packed fp32 pairs) wherever the arithmetic allows
@@ -533,8 +519,8 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         tc_fence_after_sync();
       }
-      st_chunks<16>(op_addr + buf * 64, pk);
-      if constexpr (PAD) st_chunks<16>(op_addr + 64, lo);
+      tmem_st_32x16(op_addr + buf * 64, pk);
+      if constexpr (PAD) tmem_st_32x16(op_addr + 64, lo);
       tmem_st_wait();
       tc_fence_before_sync();
       warp_arrive(&sync->e_ready[buf], lane);
@@ -550,7 +536,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     if (alive) {
       uint8_t* stage = smem_raw + (q_tile - raw_addr);   // Q is no longer needed
-      for (int c = part; c < D / 32; c += kParts) stage_chunk<BF16>(dq_addr, n_tiles > 0, p.scale, stage, r, c);
+      for (int c = quarter; c < D / 32; c += 4) stage_chunk<BF16>(dq_addr, n_tiles > 0, p.scale, stage, r, c);
       fence_proxy_async_smem();
       warp_arrive(&sync->staged, lane);
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {
@@ -657,9 +643,6 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   tc_fence_after_sync();
   const uint32_t tmem_base = sync->tmem_base;
   constexpr uint32_t kColDV = kColAcc, kColDK = kColAcc + D;
-  // D = 64 leaves [384, 512) for a second S^T: the next tile's is issued before this tile's P^T is awaited
-  constexpr int kSBufs = D == 64 ? 2 : 1;
-  auto s_col = [](int it) -> uint32_t { return kSBufs == 2 && (it & 1) ? 384u : kColS; };
 
   if (warp == kProducerWarp) {
     // the whole warp runs the loop: the lanes copy the query tile's row statistics into
@@ -732,8 +715,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         return false;
       }
       tc_fence_after_sync();
-      issue_ss<D, PAD>(tmem_base + s_col(it), k_tile, q_tile(it), idesc_score, steps_e);
-      if (elect_one()) mma_commit(smem_u32(&sync->s_full[it % kSBufs]));
+      issue_ss<D, PAD>(tmem_base + kColS, k_tile, q_tile(it), idesc_score, steps_e);
+      if (elect_one()) mma_commit(smem_u32(&sync->s_full));
       return true;
     };
     auto issue_dp = [&](int it) {   // dP^T_i = V dO_i^T
@@ -744,18 +727,14 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     if (alive) issue_dp(0);
     for (int it = 0; it < n_items && alive; ++it) {
       const bool more = it + 1 < n_items;
-      if (kSBufs == 2 && more) {
-        alive = issue_s(it + 1);
-        if (!alive) break;
-      }
       alive = wait_clocked(smem_u32(&sync->p_ready), it & 1, abort_flag, wait_limit);
       if (!alive) {
         if (lane == 0) report(p.status, 23, it, 0);
         break;
       }
       tc_fence_after_sync();
-      issue_ts<PAD>(tmem_base + kColDV, tmem_base + s_col(it), q_tile(it) + C::kTileBytes, idesc_dv, it > 0);   // dV += P^T dO
-      if (kSBufs == 1 && more) {
+      issue_ts<PAD>(tmem_base + kColDV, tmem_base + kColS, q_tile(it) + C::kTileBytes, idesc_dv, it > 0);   // dV += P^T dO
+      if (more) {
         alive = issue_s(it + 1);
         if (!alive) break;
       }
@@ -777,12 +756,12 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   } else {
     // -------------------------------------------------------- elementwise role
     const int r = tid & (kT - 1);              // key inside the tile = TMEM lane
-    const int part = warp >> 2;                // which 64 of the tile's 128 query columns
+    const int quarter = warp >> 2;             // which 32 of the tile's 128 query columns
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t s_base = tmem_base + lane_off + part * kQ;
-    const uint32_t dp_addr = tmem_base + lane_off + kColDP + part * kQ;
+    const uint32_t s_addr = tmem_base + lane_off + kColS + quarter * kQ;
+    const uint32_t dp_addr = tmem_base + lane_off + kColDP + quarter * kQ;
     // checked build: the score-shaped buffers and the two accumulators
-    if (!dbg_tmem(p.status, DBG_BWD_TC * 100 + 7, s_base + s_col(kSBufs - 1), tmem_base, kQ, kTmemCols) ||
+    if (!dbg_tmem(p.status, DBG_BWD_TC * 100 + 7, s_addr, tmem_base, kQ, kTmemCols) ||
         !dbg_tmem(p.status, DBG_BWD_TC * 100 + 8, dp_addr, tmem_base, kQ, kTmemCols) ||
         !dbg_tmem(p.status, DBG_BWD_TC * 100 + 9, tmem_base + lane_off + kColDK, tmem_base, D, kTmemCols))
       *abort_flag = 1;
@@ -800,10 +779,10 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     bool alive = true;
     int head = hk * p.group, tile = 0;         // query head and row tile (from i_first) of an item
     for (int it = 0; it < n_items; ++it) {
-      const int qrow0 = (i_first + tile) * kT + part * kQ;   // first query row of this thread's columns
-      uint32_t bq[BIAS ? kQ / 2 : 1];   // bias of this key under the thread's query rows, fetched under the wait
+      const int qrow0 = (i_first + tile) * kT + quarter * kQ;   // first query row of this thread's columns
+      uint32_t bq[BIAS ? kQ / 2 : 1];   // bias of this key under the thread's 32 query rows, fetched under the wait
       if constexpr (BIAS) {
-        // neighbouring lanes are neighbouring keys: each load is one 64-byte piece per warp
+        // neighbouring lanes are neighbouring keys: each of the 32 loads is one 64-byte piece per warp
         const uint16_t* col = static_cast<const uint16_t*>(p.bias) + b * p.bs[0] + static_cast<long long>(head) * p.bs[1] + key_g;
 #pragma unroll
         for (int i = 0; i < kQ; i += 2) {
@@ -817,8 +796,7 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         tile = 0;
         ++head;
       }
-      const uint32_t s_addr = s_base + s_col(it);
-      bool ok = wait_clocked(smem_u32(&sync->s_full[it % kSBufs]), (it / kSBufs) & 1, abort_flag, wait_limit);
+      bool ok = wait_clocked(smem_u32(&sync->s_full), it & 1, abort_flag, wait_limit);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) {
         if (lane == 0) report(p.status, 24, it, warp);
@@ -826,14 +804,14 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         break;
       }
       tc_fence_after_sync();
-      const float4* st4 = reinterpret_cast<const float4*>(stats + (it % C::kStages) * 2 * kT) + part * (kQ / 4);
+      const float4* st4 = reinterpret_cast<const float4*>(stats + (it % C::kStages) * 2 * kT) + quarter * (kQ / 4);
       // some key of this tile hides some row of these columns
       const bool need_mask = tile_has_padding ||
                              (p.causal && static_cast<long long>(qrow0) < static_cast<long long>(j0) + kT - 1 - p.causal_shift);
       float pr[kQ];
       {
         uint32_t sv[kQ], pk[kQ / 2], lo[PAD ? kQ / 2 : 1];
-        ld_chunks(s_addr, sv);
+        tmem_ld_32x32(s_addr, sv);
         tmem_ld_wait();
 #pragma unroll
         for (int q4 = 0; q4 < kQ / 4; ++q4) {
@@ -860,8 +838,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(p0, p1, pk[i >> 1]);
           }
         }
-        st_chunks<32>(s_addr, pk);
-        if constexpr (PAD) st_chunks<32>(s_addr + 16, lo);
+        tmem_st_32x16(s_addr, pk);
+        if constexpr (PAD) tmem_st_32x16(s_addr + 16, lo);
         tmem_st_wait();
         tc_fence_before_sync();
         warp_arrive(&sync->p_ready, lane);
@@ -875,7 +853,7 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
       tc_fence_after_sync();
       uint32_t dv[kQ], pk[kQ / 2], lo[PAD ? kQ / 2 : 1];
-      ld_chunks(dp_addr, dv);
+      tmem_ld_32x32(dp_addr, dv);
       tmem_ld_wait();
 #pragma unroll
       for (int q4 = 0; q4 < kQ / 4; ++q4) {
@@ -892,8 +870,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(d0, d1, pk[i >> 1]);
         }
       }
-      st_chunks<32>(dp_addr, pk);
-      if constexpr (PAD) st_chunks<32>(dp_addr + 16, lo);
+      tmem_st_32x16(dp_addr, pk);
+      if constexpr (PAD) tmem_st_32x16(dp_addr + 16, lo);
       tmem_st_wait();
       tc_fence_before_sync();
       warp_arrive(&sync->ds_ready, lane);
@@ -911,7 +889,7 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       // ring slot 0 is idle by now: its two tiles stage dK and dV
       uint8_t* stage_k = smem_raw + (ring - raw_addr);
       uint8_t* stage_v = stage_k + C::kTileBytes;
-      for (int c = part; c < D / 16; c += kParts) {
+      for (int c = quarter; c < D / 16; c += 4) {
         if (c < D / 32) stage_chunk<BF16>(tmem_base + lane_off + kColDK, n_items > 0, p.scale, stage_k, r, c);
         else stage_chunk<BF16>(tmem_base + lane_off + kColDV, n_items > 0, 1.f, stage_v, r, c - D / 32);
       }
@@ -1065,7 +1043,7 @@ int plan_bwd_tc(const BwdProblem& bp, int dtype, B200SdpaPlan* plan) {
   plan->grid_x = static_cast<int32_t>(static_cast<long long>((p.L + kT - 1) / kT) * p.Hq * p.B);
   plan->grid_y = static_cast<int32_t>(static_cast<long long>((p.S + kT - 1) / kT) * p.Hkv * p.B);
   plan->grid_z = 1;
-  plan->threads = bwd_wide_dims(p) ? 576 : kThreads;
+  plan->threads = kThreads;
   plan->smem_bytes = p.E == 64 && p.Dv == 64 ? BCfg<64>::kSmemBytes : BCfg<128>::kSmemBytes;
   plan->kv_splits = 1;
   plan->launches = 3;
