@@ -19,9 +19,8 @@
 // in exchange dQ needs neither atomics nor an fp32 scratch tensor, and results are
 // deterministic.  Arithmetic: torch_neuronx/_sdpa_math.py:133-176 with P and dS rounded
 // to the input dtype before their second product (upstream rounds P the same way in the
-// forward, :94).  Roles per CTA (576 threads): warps 0-15 elementwise (four threads per TMEM
-// lane, 32 score columns each: four warps per scheduler hide one another's tensor-memory and
-// barrier latency), warp 16 TMA producer, warp 17 MMA issuer.
+// forward, :94).  Roles per CTA (320 threads): warps 0-7 elementwise (two threads per TMEM
+// lane, 64 score columns each), warp 8 TMA producer, warp 9 MMA issuer.
 //
 // The dK/dV kernel's tensor memory is full with one pair of score-shaped accumulators:
 //   TMEM columns  [0,128) S^T, P^T over it   [128,256) dP^T, dS^T over it   [256, 256+2D) dV and dK (fp32)
@@ -45,8 +44,10 @@ namespace {
 using namespace ptx;
 using namespace tc;
 
-constexpr int kEWarps = 16;               // elementwise role: four column quarters x four lane quadrants
-constexpr int kQ = kT / 4;                // score columns of one thread
+constexpr int kEWarps = 8;                // elementwise role: two column halves x four lane quadrants
+constexpr int kParts = kEWarps / 4;
+constexpr int kQ = kT / kParts;           // score columns of one thread, in chunks of 32
+constexpr int kChunks = kQ / 32;
 constexpr int kThreads = (kEWarps + 2) * 32;
 constexpr uint32_t kColS = 0, kColDP = 128, kColAcc = 256;   // TMEM layout of the dK/dV kernel
 constexpr int kProducerWarp = kEWarps;
@@ -133,6 +134,17 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const BwdProblem bp, floa
   }
 }
 
+// This thread's score columns to registers; 16-bit operands back, chunk c at + STEP c.
+__device__ __forceinline__ void ld_chunks(uint32_t addr, uint32_t (&v)[kQ]) {
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) tmem_ld_32x32(addr + c * 32, reinterpret_cast<uint32_t(&)[32]>(v[c * 32]));
+}
+template <int STEP>
+__device__ __forceinline__ void st_chunks(uint32_t addr, const uint32_t (&v)[kQ / 2]) {
+#pragma unroll
+  for (int c = 0; c < kChunks; ++c) tmem_st_32x16(addr + c * STEP, reinterpret_cast<const uint32_t(&)[16]>(v[c * 16]));
+}
+
 // acc[tmem d, 128 x 128] = A[smem tile, K-major] * B[smem tile, K-major]^T over D
 // (PAD: only the first `steps` of the D / 16 k-steps, the columns beyond hold zeros)
 template <int D, bool PAD>
@@ -146,10 +158,10 @@ __device__ __forceinline__ void issue_ss(uint32_t d_tmem, uint32_t a_tile, uint3
     }
   }
 }
-// acc[tmem d] (+)= A[tmem, 128 x 128] * B[smem tile, MN-major].  The 16-bit A operand sits where the four column
-// quarters of the elementwise role left it: contraction indices 32 q .. 32 q + 31 packed into columns
-// [32 q, 32 q + 16) of the score-shaped buffer they came from.  PAD: the quarter's other 16 columns hold the remainders
-// of that rounding (remainder2), a second set of products.
+// acc[tmem d] (+)= A[tmem, 128 x 128] * B[smem tile, MN-major].  The 16-bit A operand sits where the elementwise
+// role left it: contraction indices 32 c .. 32 c + 31 packed into columns [32 c, 32 c + 16) of the score-shaped
+// buffer they came from.  PAD: the other 16 columns hold the remainders of that rounding (remainder2), a second set of
+// products.
 template <bool PAD>
 __device__ __forceinline__ void issue_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_tile, uint32_t idesc, bool accumulate) {
   const uint64_t bd = mnmajor_desc(b_tile);
@@ -434,11 +446,11 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   } else {
     // -------------------------------------------------------- elementwise role
     const int r = tid & (kT - 1);              // query row inside the tile = TMEM lane
-    const int quarter = warp >> 2;             // which 32 of the tile's 128 score columns
+    const int part = warp >> 2;                // which 64 of the tile's 128 score columns
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t s_addr = tmem_base + lane_off + kColS + quarter * kQ;
-    const uint32_t dp_addr = tmem_base + lane_off + kColDP + quarter * kQ;
-    const uint32_t op_addr = tmem_base + lane_off + kColOp + quarter * (kQ / 2);
+    const uint32_t s_addr = tmem_base + lane_off + kColS + part * kQ;
+    const uint32_t dp_addr = tmem_base + lane_off + kColDP + part * kQ;
+    const uint32_t op_addr = tmem_base + lane_off + kColOp + part * (kQ / 2);
     const uint32_t dq_addr = tmem_base + lane_off + kColDQ;
     // checked build: the column ranges of this thread's tensor-memory traffic; a violation drains the CTA
     if (!dbg_tmem(p.status, DBG_BWD_TC * 100 + 2, s_addr, tmem_base, kQ, kTmemCols) || !dbg_tmem(p.status, DBG_BWD_TC * 100 + 3, dp_addr, tmem_base, kQ, kTmemCols) ||
@@ -468,7 +480,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     for (int j = 0; j < n_tiles; ++j) {
       const int buf = j % kBufs;
       uint4 bv[BIAS ? kQ / 8 : 1];   // this thread's bias elements of the tile, fetched under the wait
-      if constexpr (BIAS) load_bias_row(bv, bias_row, j * kT + quarter * kQ, p.S, bias_wide);
+      if constexpr (BIAS) load_bias_row(bv, bias_row, j * kT + part * kQ, p.S, bias_wide);
       const uint32_t* bw = reinterpret_cast<const uint32_t*>(bv);
       bool ok = wait_clocked(smem_u32(&sync->sp_full), j & 1, abort_flag, wait_limit);
       ok = __all_sync(0xffffffffu, ok);
@@ -479,12 +491,12 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       tc_fence_after_sync();
       uint32_t sv[kQ], dv[kQ];
-      tmem_ld_32x32(s_addr, sv);
-      tmem_ld_32x32(dp_addr, dv);
+      ld_chunks(s_addr, sv);
+      ld_chunks(dp_addr, dv);
       tmem_ld_wait();
       tc_fence_before_sync();
       warp_arrive(&sync->f_free, lane);
-      const int col0 = j * kT + quarter * kQ;
+      const int col0 = j * kT + part * kQ;
       const bool need_mask = col0 + kQ > min_lim;
       uint32_t pk[kQ / 2], lo[PAD ? kQ / 2 : 1];
       // two columns per instruction (packed fp32 pairs) wherever the arithmetic allows
@@ -519,8 +531,8 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         tc_fence_after_sync();
       }
-      tmem_st_32x16(op_addr + buf * 64, pk);
-      if constexpr (PAD) tmem_st_32x16(op_addr + 64, lo);
+      st_chunks<16>(op_addr + buf * 64, pk);
+      if constexpr (PAD) st_chunks<16>(op_addr + 64, lo);
       tmem_st_wait();
       tc_fence_before_sync();
       warp_arrive(&sync->e_ready[buf], lane);
@@ -536,7 +548,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     if (alive) {
       uint8_t* stage = smem_raw + (q_tile - raw_addr);   // Q is no longer needed
-      for (int c = quarter; c < D / 32; c += 4) stage_chunk<BF16>(dq_addr, n_tiles > 0, p.scale, stage, r, c);
+      for (int c = part; c < D / 32; c += kParts) stage_chunk<BF16>(dq_addr, n_tiles > 0, p.scale, stage, r, c);
       fence_proxy_async_smem();
       warp_arrive(&sync->staged, lane);
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {
@@ -756,10 +768,10 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   } else {
     // -------------------------------------------------------- elementwise role
     const int r = tid & (kT - 1);              // key inside the tile = TMEM lane
-    const int quarter = warp >> 2;             // which 32 of the tile's 128 query columns
+    const int part = warp >> 2;                // which 64 of the tile's 128 query columns
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t s_addr = tmem_base + lane_off + kColS + quarter * kQ;
-    const uint32_t dp_addr = tmem_base + lane_off + kColDP + quarter * kQ;
+    const uint32_t s_addr = tmem_base + lane_off + kColS + part * kQ;
+    const uint32_t dp_addr = tmem_base + lane_off + kColDP + part * kQ;
     // checked build: the score-shaped buffers and the two accumulators
     if (!dbg_tmem(p.status, DBG_BWD_TC * 100 + 7, s_addr, tmem_base, kQ, kTmemCols) ||
         !dbg_tmem(p.status, DBG_BWD_TC * 100 + 8, dp_addr, tmem_base, kQ, kTmemCols) ||
@@ -779,10 +791,10 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     bool alive = true;
     int head = hk * p.group, tile = 0;         // query head and row tile (from i_first) of an item
     for (int it = 0; it < n_items; ++it) {
-      const int qrow0 = (i_first + tile) * kT + quarter * kQ;   // first query row of this thread's columns
-      uint32_t bq[BIAS ? kQ / 2 : 1];   // bias of this key under the thread's 32 query rows, fetched under the wait
+      const int qrow0 = (i_first + tile) * kT + part * kQ;   // first query row of this thread's columns
+      uint32_t bq[BIAS ? kQ / 2 : 1];   // bias of this key under the thread's query rows, fetched under the wait
       if constexpr (BIAS) {
-        // neighbouring lanes are neighbouring keys: each of the 32 loads is one 64-byte piece per warp
+        // neighbouring lanes are neighbouring keys: each load is one 64-byte piece per warp
         const uint16_t* col = static_cast<const uint16_t*>(p.bias) + b * p.bs[0] + static_cast<long long>(head) * p.bs[1] + key_g;
 #pragma unroll
         for (int i = 0; i < kQ; i += 2) {
@@ -804,14 +816,14 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         break;
       }
       tc_fence_after_sync();
-      const float4* st4 = reinterpret_cast<const float4*>(stats + (it % C::kStages) * 2 * kT) + quarter * (kQ / 4);
+      const float4* st4 = reinterpret_cast<const float4*>(stats + (it % C::kStages) * 2 * kT) + part * (kQ / 4);
       // some key of this tile hides some row of these columns
       const bool need_mask = tile_has_padding ||
                              (p.causal && static_cast<long long>(qrow0) < static_cast<long long>(j0) + kT - 1 - p.causal_shift);
       float pr[kQ];
       {
         uint32_t sv[kQ], pk[kQ / 2], lo[PAD ? kQ / 2 : 1];
-        tmem_ld_32x32(s_addr, sv);
+        ld_chunks(s_addr, sv);
         tmem_ld_wait();
 #pragma unroll
         for (int q4 = 0; q4 < kQ / 4; ++q4) {
@@ -838,8 +850,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(p0, p1, pk[i >> 1]);
           }
         }
-        tmem_st_32x16(s_addr, pk);
-        if constexpr (PAD) tmem_st_32x16(s_addr + 16, lo);
+        st_chunks<32>(s_addr, pk);
+        if constexpr (PAD) st_chunks<32>(s_addr + 16, lo);
         tmem_st_wait();
         tc_fence_before_sync();
         warp_arrive(&sync->p_ready, lane);
@@ -853,7 +865,7 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
       tc_fence_after_sync();
       uint32_t dv[kQ], pk[kQ / 2], lo[PAD ? kQ / 2 : 1];
-      tmem_ld_32x32(dp_addr, dv);
+      ld_chunks(dp_addr, dv);
       tmem_ld_wait();
 #pragma unroll
       for (int q4 = 0; q4 < kQ / 4; ++q4) {
@@ -870,8 +882,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(d0, d1, pk[i >> 1]);
         }
       }
-      tmem_st_32x16(dp_addr, pk);
-      if constexpr (PAD) tmem_st_32x16(dp_addr + 16, lo);
+      st_chunks<32>(dp_addr, pk);
+      if constexpr (PAD) st_chunks<32>(dp_addr + 16, lo);
       tmem_st_wait();
       tc_fence_before_sync();
       warp_arrive(&sync->ds_ready, lane);
@@ -889,7 +901,7 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       // ring slot 0 is idle by now: its two tiles stage dK and dV
       uint8_t* stage_k = smem_raw + (ring - raw_addr);
       uint8_t* stage_v = stage_k + C::kTileBytes;
-      for (int c = quarter; c < D / 16; c += 4) {
+      for (int c = part; c < D / 16; c += kParts) {
         if (c < D / 32) stage_chunk<BF16>(tmem_base + lane_off + kColDK, n_items > 0, p.scale, stage_k, r, c);
         else stage_chunk<BF16>(tmem_base + lane_off + kColDV, n_items > 0, 1.f, stage_v, r, c - D / 32);
       }
@@ -1043,7 +1055,7 @@ int plan_bwd_tc(const BwdProblem& bp, int dtype, B200SdpaPlan* plan) {
   plan->grid_x = static_cast<int32_t>(static_cast<long long>((p.L + kT - 1) / kT) * p.Hq * p.B);
   plan->grid_y = static_cast<int32_t>(static_cast<long long>((p.S + kT - 1) / kT) * p.Hkv * p.B);
   plan->grid_z = 1;
-  plan->threads = kThreads;
+  plan->threads = bwd_wide_dims(p) ? 576 : kThreads;
   plan->smem_bytes = p.E == 64 && p.Dv == 64 ? BCfg<64>::kSmemBytes : BCfg<128>::kSmemBytes;
   plan->kv_splits = 1;
   plan->launches = 3;
