@@ -703,7 +703,7 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           if (slot_ok) *reinterpret_cast<float2*>(pack.part_ml + slot * 2) = make_float2(m_run * sl2, l_run);
           // O: every lane holds a row; 32 columns at a time go through this warp's 4 KB of the (idle) Q slot, so
           // that eight lanes store the 128 bytes of one row
-          const int64_t my_row = slot_ok && l_run > 0.f ? slot : -1;
+          const int64_t my_row = slot_ok && l_run != 0.f ? slot : -1;   // (a NaN sum is not an empty one)
           uint8_t* buf = smem_raw + (q_smem[t] - raw_addr) + quad * 4096;
           if (tg.n_tiles > 0) {
 #pragma unroll
@@ -938,8 +938,11 @@ __global__ void __launch_bounds__(256) prefill_combine_kernel(const Problem p, c
   float mx = ml.x;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const float w = ml.y > 0.f ? ex2(ml.x - mx) : 0.f;
-  float lsum = w * ml.y;
+  // A split without a visible key for this row has a sum of 0 and wrote nothing else.  Everything but 0 counts: NaN in
+  // a score must come out as NaN, as it does where one CTA walks all keys.
+  const unsigned seen = __ballot_sync(0xffffffffu, ml.y != 0.f);
+  const float w = ml.y != 0.f ? ex2(ml.x - mx) : 0.f;
+  float lsum = ml.y != 0.f ? w * ml.y : 0.f;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
   float acc[C];
@@ -949,7 +952,7 @@ __global__ void __launch_bounds__(256) prefill_combine_kernel(const Problem p, c
 #pragma unroll 4
   for (int s = 0; s < n_split; ++s) {
     const float ws = __shfl_sync(0xffffffffu, w, s);
-    if (ws > 0.f) {   // a split without a visible key for this row wrote nothing
+    if ((seen >> s) & 1u) {
       float v[C];
       if constexpr (C == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src + s * D);
       else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(src + s * D);
@@ -957,7 +960,7 @@ __global__ void __launch_bounds__(256) prefill_combine_kernel(const Problem p, c
       for (int c = 0; c < C; ++c) acc[c] = fmaf(v[c], ws, acc[c]);
     }
   }
-  const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
+  const float inv = lsum != 0.f ? 1.f / lsum : 0.f;
   if (!dbg_bhrc(p.status, DBG_PREFILL * 100 + 10, b, p.B, h, p.Hq, i, p.L, lane * C, C, p.Dv)) return;
   T* out = reinterpret_cast<T*>(p.out) + b * p.os[0] + static_cast<int64_t>(h) * p.os[1] + static_cast<int64_t>(i) * p.os[2] + lane * C;
   T r[C];
