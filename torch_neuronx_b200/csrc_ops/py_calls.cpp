@@ -5,8 +5,8 @@
 // (sdpa_forward) to 52 us (scaled_dot_product_attention with kv_lens) to enqueue one, so the GPU waited.  Here the
 // whole call -- checks, output and scratch allocation, parameter block, launch -- is native.
 //
-// Every function returns None when the call is not one of the plain ones it serves (subclasses, active modes,
-// gradients, other dtypes, anything malformed); the Python layer then takes its own path, which serves the rest and
+// Every function returns None when the call is not one of the plain ones it serves (subclasses, active modes and
+// transforms, tracing, forward-mode tangents, gradients, other dtypes, anything malformed); the Python layer then takes its own path, which serves the rest and
 // raises the errors.  So nothing here raises for a bad argument.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -14,6 +14,7 @@
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/core/grad_mode.h>
 #include <ATen/ops/_scaled_dot_product_fused_attention_overrideable.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -44,17 +45,23 @@ void keep_plan(const B200SdpaPlan& plan) {
   g_plan_fresh = true;
 }
 
-// A plain strided CUDA tensor with nothing between it and the kernels.
+// A plain strided CUDA tensor with nothing between it and the kernels; a dual tensor of forward-mode differentiation
+// has the same keys but carries a tangent, which only the dispatcher's formulas see (and refuse).
 bool plain(PyObject* o) {
   if (!THPVariable_CheckExact(o)) return false;
   const at::Tensor& t = THPVariable_Unpack(o);
   static const uint64_t expected = c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA,
                                                         c10::DispatchKey::ADInplaceOrView, c10::DispatchKey::AutocastCUDA})
                                        .raw_repr();
-  return t.is_cuda() && (t.key_set().raw_repr() & ~expected) == 0;
+  return t.is_cuda() && (t.key_set().raw_repr() & ~expected) == 0 && !t._fw_grad(/*level=*/0).defined();
 }
+// Nothing on this thread stands between a call and the CUDA kernels.  The modes written in Python have stacks of their
+// own; whatever else wants to see every call (the tracer, functorch's transforms, functionalization) includes a
+// dispatch key.  Those included by default and autocast's, which these operations do not listen to, may be there.
 bool no_modes() {
-  return !at::impl::torch_function_mode_enabled() && !c10::impl::TorchDispatchModeTLS::any_modes_set();
+  static const c10::DispatchKeySet harmless = c10::default_included_set | c10::autocast_dispatch_keyset;
+  return !at::impl::torch_function_mode_enabled() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+         (c10::impl::tls_local_dispatch_key_set().included_ - harmless).empty();
 }
 bool wants_grad(const at::Tensor& t) { return t.requires_grad(); }
 
