@@ -505,6 +505,11 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           const bool has_next = j + 1 < n_iter;
           alive = wait_full(pos_v);
           if (!alive) break;
+          if (PAD && !has_next && it.kv_limit < p.S) {   // as in prefill_sm100.cu
+            const int key0 = (BIAS && it.tiles != 0 ? 63 - __clzll(static_cast<long long>(it.tiles)) : j) * kBlockN;
+            if (key0 + kBlockN > it.kv_limit)
+              zero_tile_rows<C::kBoxes, kBlockN>(kv_smem + stage_of(pos_v) * C::kTileBytes, it.kv_limit - key0, lane);
+          }
           // one tile: P_t(j) V(j) in two halves as the halves of P arrive, then Q_t K(j+1)^T
           auto serve = [&](auto tile_const) {
             constexpr int t = decltype(tile_const)::value;

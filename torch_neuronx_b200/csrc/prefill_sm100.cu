@@ -446,6 +446,9 @@ prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const bool has_next = j + 1 < n_iter;
         alive = wait_full(item_v);
         if (!alive) break;
+        // (these shapes came from a kernel that never reads a key beyond kv_lens)
+        if (PAD && !has_next && kv_limit < p.S && (j + 1) * kBlockN > kv_limit)
+          zero_tile_rows<C::kBoxes, kBlockN>(kv_smem + stage_addr(item_v) * C::kTileBytes, kv_limit - j * kBlockN, lane);
         // one tile: P_t(j) V(j) in two halves as the halves of P arrive, then Q_t K(j+1)^T
         auto serve = [&](auto tile_const) {
           constexpr int t = decltype(tile_const)::value;

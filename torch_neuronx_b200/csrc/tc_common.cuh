@@ -193,6 +193,19 @@ inline bool strides_ok(const void* base, const int64_t* s, int rows, int heads, 
   return true;
 }
 
+// Rows [row0, kRows) of a tile in shared memory (boxes of kRows rows of 128 bytes; the swizzle stays inside a row) become
+// zeros, ready for the tensor cores.  For keys at or beyond kv_lens, whose weight is exactly 0 but whose bytes may be a
+// NaN: 0 x NaN is NaN.  The tile's copy has landed; the whole warp calls.
+template <int kBoxes, int kRows>
+__device__ __forceinline__ void zero_tile_rows(uint32_t tile, int row0, int lane) {
+#pragma unroll
+  for (int bx = 0; bx < kBoxes; ++bx)
+    for (int off = row0 * 128 + lane * 16; off < kRows * 128; off += 32 * 16)
+      asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(tile + bx * (kRows * 128) + off), "r"(0) : "memory");
+  fence_proxy_async_smem();
+  __syncwarp();
+}
+
 // What rounding (x0, x1) to the 16-bit pair `hi` left over, rounded to 16 bits itself.  Where a shape was served with
 // fp32 probabilities before, the second product takes both parts, hi + lo, as two operands: 2^-16 (bf16) or 2^-22
 // (fp16) of the value is lost, far below the rounding of the result.
