@@ -385,6 +385,9 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         return false;
       }
       tc_fence_after_sync();
+      // (PAD: these shapes came from kernels that leave out what lies beyond kv_lens, and dS = 0 times a NaN row of K is NaN)
+      if (PAD && kv_limit < p.S && (j + 1) * kT > kv_limit)
+        zero_tile_rows<C::kBoxes, kT>(k_ring + ks * C::kTileBytes, kv_limit - j * kT, lane);
       const uint64_t qd = kmajor_desc(q_tile), kd = kmajor_desc(k_ring + ks * C::kTileBytes);
       const uint64_t od = kmajor_desc(do_tile), vd = kmajor_desc(v_ring + vs * C::kTileBytes);
       if (elect_one()) {
@@ -512,12 +515,16 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         f2_unpack(f2_fma(f2_pack(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2_2, f2_pack(off0, off1)), a0, a1);
         float p0 = ex2(a0);
         float p1 = ex2(a1);
-        if (need_mask) {
+        if (!PAD && need_mask) {
           p0 = (col0 + i < lim) ? p0 : 0.f;
           p1 = (col0 + i + 1 < lim) ? p1 : 0.f;
         }
         float d0, d1;
         f2_unpack(f2_mul(f2_pack(p0, p1), f2_add(f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])), neg_dl2)), d0, d1);
+        if (PAD && need_mask) {   // after the product: dP of a hidden key may be NaN
+          d0 = (col0 + i < lim) ? d0 : 0.f;
+          d1 = (col0 + i + 1 < lim) ? d1 : 0.f;
+        }
         pk[i >> 1] = pack2<BF16>(d0, d1);
         if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(d0, d1, pk[i >> 1]);
       }
@@ -878,6 +885,10 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           f2_unpack(f2_mul(f2_pack(pr[i], pr[i + 1]), f2_add(f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])),
                                                               f2_pack(nd[e], nd[e + 1]))),
                     d0, d1);
+          if (PAD && need_mask) {
+            d0 = (qrow0 + i >= i_min) ? d0 : 0.f;
+            d1 = (qrow0 + i + 1 >= i_min) ? d1 : 0.f;
+          }
           pk[i >> 1] = pack2<BF16>(d0, d1);
           if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(d0, d1, pk[i >> 1]);
         }
