@@ -366,10 +366,11 @@ __global__ void __launch_bounds__(kThreads) fp32_bwd_dq_kernel(const BwdProblem 
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int64_t lim64 = p.causal ? static_cast<int64_t>(row0 + f0 + i) + p.causal_shift + 1 : n_keys;
-      const int lim = lse[i] == -CUDART_INF_F ? 0 : (lim64 < n_keys ? static_cast<int>(lim64 < 0 ? 0 : lim64) : n_keys);
+      const int lim = lim64 < n_keys ? static_cast<int>(lim64 < 0 ? 0 : lim64) : n_keys;
+      const bool dead = lse[i] == -CUDART_INF_F;   // no key seen, or nothing but NaN: then delta is NaN and so is dS
 #pragma unroll
       for (int j = 0; j < J; ++j)
-        s[i][j] = j0 + tx + TX * j < lim ? expf(s[i][j] * p.scale - lse[i]) * (dp[i][j] - delta[i]) : 0.f;
+        s[i][j] = j0 + tx + TX * j < lim ? (dead ? 0.f : expf(s[i][j] * p.scale - lse[i])) * (dp[i][j] - delta[i]) : 0.f;
     }
     store_transposed<TX, J>(Op, f0, tx, s);
     __syncthreads();   // the operand is here; V has been read
