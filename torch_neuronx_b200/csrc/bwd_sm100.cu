@@ -885,10 +885,6 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           f2_unpack(f2_mul(f2_pack(pr[i], pr[i + 1]), f2_add(f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])),
                                                               f2_pack(nd[e], nd[e + 1]))),
                     d0, d1);
-          if (PAD && need_mask) {
-            d0 = (qrow0 + i >= i_min) ? d0 : 0.f;
-            d1 = (qrow0 + i + 1 >= i_min) ? d1 : 0.f;
-          }
           pk[i >> 1] = pack2<BF16>(d0, d1);
           if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(d0, d1, pk[i >> 1]);
         }
@@ -913,8 +909,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       uint8_t* stage_k = smem_raw + (ring - raw_addr);
       uint8_t* stage_v = stage_k + C::kTileBytes;
       for (int c = part; c < D / 16; c += kParts) {
-        if (c < D / 32) stage_chunk<BF16>(tmem_base + lane_off + kColDK, n_items > 0, p.scale, stage_k, r, c);
-        else stage_chunk<BF16>(tmem_base + lane_off + kColDV, n_items > 0, 1.f, stage_v, r, c - D / 32);
+        if (c < D / 32) stage_chunk<BF16>(tmem_base + lane_off + kColDK, n_items > 0, p.scale, stage_k, r, c, !PAD || key_g < n_keys);
+        else stage_chunk<BF16>(tmem_base + lane_off + kColDV, n_items > 0, 1.f, stage_v, r, c - D / 32, !PAD || key_g < n_keys);
       }
       fence_proxy_async_smem();
       warp_arrive(&sync->staged, lane);

@@ -404,13 +404,17 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
           float a0, a1;
           f2_unpack(f2_fma(f2_pack(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2_2, f2_pack(nl[e], nl[e + 1])), a0, a1);
           float p0 = ex2(a0), p1 = ex2(a1);
+          if (WALK != kDQ && need_mask) {
+            p0 = col0 + i >= i_min ? p0 : 0.f;
+            p1 = col0 + i + 1 >= i_min ? p1 : 0.f;
+          }
           if constexpr (WALK != kDV) {
             f2_unpack(f2_mul(f2_pack(p0, p1), f2_add(f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])), f2_pack(nd[e], nd[e + 1]))),
                       p0, p1);
           }
-          if (need_mask) {   // after the product: dP of a hidden key may be NaN
-            p0 = (WALK == kDQ ? col0 + i < lim : col0 + i >= i_min) ? p0 : 0.f;
-            p1 = (WALK == kDQ ? col0 + i + 1 < lim : col0 + i + 1 >= i_min) ? p1 : 0.f;
+          if (WALK == kDQ && need_mask) {   // after the product: dP of a hidden key may be NaN
+            p0 = col0 + i < lim ? p0 : 0.f;
+            p1 = col0 + i + 1 < lim ? p1 : 0.f;
           }
           pk[i >> 1] = pack2<BF16>(p0, p1);
           lo[i >> 1] = remainder2<BF16>(p0, p1, pk[i >> 1]);
@@ -444,7 +448,7 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
     if (alive) {
       // the fixed operands are no longer needed: their area stages the gradient
       for (int c = quarter; c < C::kAccW / 32; c += 4)
-        stage_chunk<BF16>(acc_addr, w.n_tiles > 0, WALK == kDV ? 1.f : p.scale, smem_raw, r, c);
+        stage_chunk<BF16>(acc_addr, w.n_tiles > 0, WALK == kDV ? 1.f : p.scale, smem_raw, r, c, WALK == kDQ || row_g < w.n_keys);
       fence_proxy_async_smem();
       warp_arrive(&sync->staged, lane);
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {
