@@ -22,5 +22,9 @@ def test_nan_row(D, causal):
         res.append((out, lse) + T.sdpa_backward(go, q, k, v, out, lse, is_causal=causal, force_path=path)[:3])
     T.check_device_status()
     assert torch.isnan(res[0][0][0, 1, 70]).all() and torch.isnan(res[0][2][0, 1, 70]).all()
+    # keys that the row does not see: 0 x NaN reaches those that share a tile with it, and the kernels' tiles differ
+    seen = 71 if causal else 150
     for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), *res):
+        if name in ("dk", "dv"):
+            a, b = a[:, :, :seen], b[:, :, :seen]
         assert torch.equal(torch.isfinite(a), torch.isfinite(b)), name
