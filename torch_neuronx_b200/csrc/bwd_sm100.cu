@@ -37,6 +37,8 @@
 // Every wait is bounded (see tc_common.cuh).
 #include "bwd_common.cuh"
 
+#include <type_traits>
+
 namespace b200 {
 
 namespace {
@@ -83,15 +85,69 @@ static_assert(sizeof(BSync) <= 272, "barrier block must fit its reserve (272 byt
 
 // ------------------------------------------------------------------ prep --
 
+// (fp16) One part of the maxima that gradient_scale() combines, over dO and the visible rows of V, whose rows start on
+// 16 bytes: eight lanes a row.  Infinities and NaN are left out: what they reach is not finite at any scale.
+__device__ __forceinline__ void range_part(const BwdProblem& bp, float2* range, int n_parts, int unit) {
+  const Problem& p = bp.f;
+  __shared__ uint32_t sm[2][8];
+  const int part = unit % n_parts, stream = unit / n_parts;
+  const int hk = stream % p.Hkv, b = stream / p.Hkv;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto scan = [&](const __half* base, int64_t head_stride, int64_t row_stride, int rows, int n_rows) {   // of pairs of |x|
+    uint32_t top = 0;
+#pragma unroll 4
+    for (int r = part * 32 + static_cast<int>(threadIdx.x >> 3); r < n_rows; r += n_parts * 32) {
+      const __half* row = base + r / rows * head_stride + r % rows * row_stride;
+      for (int e = (lane & 7) * 8; e < p.Dv; e += 64) {
+        const uint4 x = *reinterpret_cast<const uint4*>(row + e);
+        for (const uint32_t w : {x.x, x.y, x.z, x.w}) {
+          const uint32_t a = w & 0x7fff7fffu;
+          top = __vmaxu2(top, a & __vcmpltu2(a, 0x7c007c00u));
+        }
+      }
+    }
+    return __vmaxu2(top, top >> 16) & 0xffffu;   // (finite halves order like their bits)
+  };
+  uint32_t go = scan(reinterpret_cast<const __half*>(bp.dout) + b * bp.dos[0] + hk * p.group * bp.dos[1], bp.dos[1], bp.dos[2], p.L,
+                     p.group * p.L);
+  uint32_t v = scan(reinterpret_cast<const __half*>(p.v) + b * p.vs[0] + hk * p.vs[1], 0, p.vs[2], p.S, valid_keys(p, b));
+  go = __reduce_max_sync(0xffffffffu, go);
+  v = __reduce_max_sync(0xffffffffu, v);
+  if (lane == 0) {
+    sm[0][warp] = go;
+    sm[1][warp] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && dbg_range(p.status, DBG_BWD_TC * 100 + 11, unit, 1, static_cast<int64_t>(p.B) * p.Hkv * n_parts)) {
+    uint32_t a = 0, c = 0;
+    for (int i = 0; i < 8; ++i) {
+      a = max(a, sm[0][i]);
+      c = max(c, sm[1][i]);
+    }
+    range[unit] = make_float2(__half2float(__ushort_as_half(static_cast<unsigned short>(a))),
+                              __half2float(__ushort_as_half(static_cast<unsigned short>(c))));
+  }
+}
+
 // Eight lanes per row (four rows per warp) when rows can be read 16 bytes at a time,
 // otherwise one warp per row with scalar loads.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) bwd_prep_kernel(const BwdProblem bp, float* __restrict__ lse2,
-                                                        float* __restrict__ delta, const int l_pad) {
+                                                        float* __restrict__ delta, const int l_pad, float2* range,
+                                                        const int n_parts, const unsigned range_blocks) {
   const Problem& p = bp.f;
+  constexpr bool kHalf = std::is_same_v<T, __half>;
+  if constexpr (kHalf) {
+    if (blockIdx.x < range_blocks) {   // (first: they take longer than the others)
+      pdl_wait();
+      pdl_launch_dependents();
+      range_part(bp, range, n_parts, static_cast<int>(blockIdx.x));
+      return;
+    }
+  }
   constexpr int kLanes = VEC ? 8 : 32;             // lanes cooperating on one row
   constexpr int kRowsPerWarp = 32 / kLanes;
-  const long long gwarp = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const long long gwarp = (static_cast<long long>(blockIdx.x - range_blocks) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int sub = lane % kLanes;
   const long long row_id = gwarp * kRowsPerWarp + lane / kLanes;
@@ -127,6 +183,7 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const BwdProblem bp, floa
   if (live && sub == 0) {
     const float l = p.lse[b * p.ls[0] + h * p.ls[1] + i * p.ls[2]];
     l2 = (l == -CUDART_INF_F) ? CUDART_INF_F : l * kLog2e;
+    if (kHalf && range != nullptr) l2 -= kPScaleLog2;
   }
   if (in_range && sub == 0 && dbg_range(p.status, DBG_BWD_TC * 100 + 1, row_id, 1, total)) {
     lse2[row_id] = l2;
@@ -245,7 +302,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                  const __grid_constant__ CUtensorMap tm_dq, const Problem p, const float* __restrict__ lse2,
                  const float* __restrict__ delta, const int l_pad, const int n_qblk, const int streams_per_wave,
-                 const long long wait_limit) {
+                 const long long wait_limit, const float2* range, const int n_parts) {
   using C = ACfg<D>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -333,6 +390,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   tc_fence_after_sync();
   const uint32_t tmem_base = sync->tmem_base;
   constexpr uint32_t kColS = 0, kColDP = 128, kColOp = 256, kColDQ = 384;
+  constexpr bool kScaled = PAD && !BF16;   // see gradient_scale
   constexpr int kBufs = PAD ? 1 : 2;   // dS operand buffers (PAD: the second one holds the remainders, see remainder2)
 
   if (warp == kProducerWarp) {
@@ -470,6 +528,8 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const float neg_l2 = stat_ok ? -lse2[stat_idx] : -CUDART_INF_F;      // -inf for rows without a visible key
     const float dl = stat_ok ? delta[stat_idx] : 0.f;
     const float sl2 = p.scale * kLog2e;
+    const float gs = kScaled ? gradient_scale(range, n_parts, kv_stream, p.Dv, lane) : 1.f;
+    const float undo = kScaled ? 1.f / (gs * kPScale) : 1.f;
     bool alive = true;
     // this row of the forward's additive bias (the query's dtype, unit stride along the keys)
     const uint4* bias_row = nullptr;
@@ -503,7 +563,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const bool need_mask = col0 + kQ > min_lim;
       uint32_t pk[kQ / 2], lo[PAD ? kQ / 2 : 1];
       // two columns per instruction (packed fp32 pairs) wherever the arithmetic allows
-      const uint64_t sl2_2 = f2_pack(sl2, sl2), neg_dl2 = f2_pack(-dl, -dl);
+      const uint64_t sl2_2 = f2_pack(sl2, sl2), neg_dl2 = f2_pack(-dl * gs, -dl * gs), gs2 = f2_pack(gs, gs);
 #pragma unroll
       for (int i = 0; i < kQ; i += 2) {
         float off0 = neg_l2, off1 = neg_l2;
@@ -520,7 +580,8 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           p1 = (col0 + i + 1 < lim) ? p1 : 0.f;
         }
         float d0, d1;
-        f2_unpack(f2_mul(f2_pack(p0, p1), f2_add(f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])), neg_dl2)), d0, d1);
+        const uint64_t dp2 = f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1]));
+        f2_unpack(f2_mul(f2_pack(p0, p1), kScaled ? f2_fma(dp2, gs2, neg_dl2) : f2_add(dp2, neg_dl2)), d0, d1);
         if (PAD && need_mask) {   // after the product: dP of a hidden key may be NaN
           d0 = (col0 + i < lim) ? d0 : 0.f;
           d1 = (col0 + i + 1 < lim) ? d1 : 0.f;
@@ -555,7 +616,7 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     if (alive) {
       uint8_t* stage = smem_raw + (q_tile - raw_addr);   // Q is no longer needed
-      for (int c = part; c < D / 32; c += kParts) stage_chunk<BF16>(dq_addr, n_tiles > 0, p.scale, stage, r, c);
+      for (int c = part; c < D / 32; c += kParts) stage_chunk<BF16>(dq_addr, n_tiles > 0, p.scale * undo, stage, r, c);
       fence_proxy_async_smem();
       warp_arrive(&sync->staged, lane);
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {
@@ -590,7 +651,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                   const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                   const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
                   const Problem p, const float* lse2, const float* delta, const int l_pad,
-                  const int n_kblk, const int streams_per_wave, const long long wait_limit) {
+                  const int n_kblk, const int streams_per_wave, const long long wait_limit, const float2* range,
+                  const int n_parts) {
   using C = BCfg<D>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -662,6 +724,7 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   tc_fence_after_sync();
   const uint32_t tmem_base = sync->tmem_base;
   constexpr uint32_t kColDV = kColAcc, kColDK = kColAcc + D;
+  constexpr bool kScaled = PAD && !BF16;   // see gradient_scale
 
   if (warp == kProducerWarp) {
     // the whole warp runs the loop: the lanes copy the query tile's row statistics into
@@ -681,6 +744,7 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         st_d = reinterpret_cast<const float4*>(delta + src)[lane];
       }
     };
+    float gs = 1.f;   // delta is kept times this
     if (n_items > 0) fetch_stats(0);
     for (int it = 0; it < n_items && alive; ++it) {
       const int stage = it % C::kStages;
@@ -696,16 +760,32 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const int h = hk * p.group + it / per_head;
       const int qrow0 = (i_first + it % per_head) * kT;
       float4* dst = reinterpret_cast<float4*>(stats + stage * 2 * kT);
+      const uint32_t bar = smem_u32(&sync->ring_full[stage]);
+      auto copy = [&]() {
+        const uint32_t q_dst = ring + stage * 2 * C::kTileBytes;
+        for (int bx = 0; bx < C::kBoxes; ++bx) {
+          tma_load_4d(q_dst + bx * kBoxBytes, &tm_q, bar, bx * 64, qrow0, h, b);
+          tma_load_4d(q_dst + C::kTileBytes + bx * kBoxBytes, &tm_do, bar, bx * 64, qrow0, h, b);
+        }
+      };
+      if constexpr (kScaled) {   // the copies go first: the maxima behind gs take a trip to L2
+        if (lane == 0) {
+          mbar_expect_tx(bar, 2 * C::kTileBytes);
+          copy();
+        }
+        __syncwarp();
+        if (it == 0) gs = gradient_scale(range, n_parts, kv_stream, p.Dv, lane);
+        st_d = make_float4(st_d.x * gs, st_d.y * gs, st_d.z * gs, st_d.w * gs);
+      }
       dst[lane] = st_l;
       dst[32 + lane] = st_d;
       __syncwarp();
       if (lane == 0) {
-        const uint32_t bar = smem_u32(&sync->ring_full[stage]);
-        const uint32_t q_dst = ring + stage * 2 * C::kTileBytes;
-        mbar_arrive_expect_tx(bar, 2 * C::kTileBytes);
-        for (int bx = 0; bx < C::kBoxes; ++bx) {
-          tma_load_4d(q_dst + bx * kBoxBytes, &tm_q, bar, bx * 64, qrow0, h, b);
-          tma_load_4d(q_dst + C::kTileBytes + bx * kBoxBytes, &tm_do, bar, bx * 64, qrow0, h, b);
+        if constexpr (kScaled) {
+          mbar_arrive(bar);
+        } else {
+          mbar_arrive_expect_tx(bar, 2 * C::kTileBytes);
+          copy();
         }
       }
       if (it + 1 < n_items) fetch_stats(it + 1);
@@ -795,6 +875,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const bool tile_has_padding = j0 + kT > n_keys;
     const float sl2 = p.scale * kLog2e;
     const uint64_t sl2_2 = f2_pack(sl2, sl2);
+    const float gs = kScaled ? gradient_scale(range, n_parts, kv_stream, p.Dv, lane) : 1.f;
+    const uint64_t gs2 = f2_pack(gs, gs);
     bool alive = true;
     int head = hk * p.group, tile = 0;         // query head and row tile (from i_first) of an item
     for (int it = 0; it < n_items; ++it) {
@@ -882,9 +964,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         for (int e = 0; e < 4; e += 2) {
           const int i = q4 * 4 + e;
           float d0, d1;
-          f2_unpack(f2_mul(f2_pack(pr[i], pr[i + 1]), f2_add(f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])),
-                                                              f2_pack(nd[e], nd[e + 1]))),
-                    d0, d1);
+          const uint64_t dp2 = f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])), nd2 = f2_pack(nd[e], nd[e + 1]);
+          f2_unpack(f2_mul(f2_pack(pr[i], pr[i + 1]), kScaled ? f2_fma(dp2, gs2, nd2) : f2_add(dp2, nd2)), d0, d1);
           pk[i >> 1] = pack2<BF16>(d0, d1);
           if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(d0, d1, pk[i >> 1]);
         }
@@ -909,8 +990,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       uint8_t* stage_k = smem_raw + (ring - raw_addr);
       uint8_t* stage_v = stage_k + C::kTileBytes;
       for (int c = part; c < D / 16; c += kParts) {
-        if (c < D / 32) stage_chunk<BF16>(tmem_base + lane_off + kColDK, n_items > 0, p.scale, stage_k, r, c, !PAD || key_g < n_keys);
-        else stage_chunk<BF16>(tmem_base + lane_off + kColDV, n_items > 0, 1.f, stage_v, r, c - D / 32, !PAD || key_g < n_keys);
+        if (c < D / 32) stage_chunk<BF16>(tmem_base + lane_off + kColDK, n_items > 0, p.scale * (kScaled ? 1.f / (gs * kPScale) : 1.f), stage_k, r, c, !PAD || key_g < n_keys);
+        else stage_chunk<BF16>(tmem_base + lane_off + kColDV, n_items > 0, kScaled ? 1.f / kPScale : 1.f, stage_v, r, c - D / 32, !PAD || key_g < n_keys);
       }
       fence_proxy_async_smem();
       warp_arrive(&sync->staged, lane);
@@ -937,7 +1018,7 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
 }  // namespace
 
-int launch_bwd_prep(const BwdProblem& bp, bool bf16, float* lse2, float* delta, cudaStream_t stream) {
+int launch_bwd_prep(const BwdProblem& bp, bool bf16, float* lse2, float* delta, float2* range, cudaStream_t stream) {
   const Problem& p = bp.f;
   const int l_pad = padded_rows(p);
   const long long rows = static_cast<long long>(p.B) * p.Hq * l_pad;
@@ -947,11 +1028,14 @@ int launch_bwd_prep(const BwdProblem& bp, bool bf16, float* lse2, float* delta, 
   const bool vec = p.Dv % 8 == 0 && rows_aligned(bp.dout, bp.dos) && rows_aligned(p.out, p.os);
   const long long warps = vec ? (rows + 3) / 4 : rows;
   const long long blocks = (warps * 32 + 255) / 256;
-  if (blocks > 0x7fffffffLL) return B200_SDPA_ERR_UNSUPPORTED;
-  const unsigned grid = static_cast<unsigned>(blocks);
+  const int n_parts = range_parts(p);
+  const long long extra = range != nullptr ? static_cast<long long>(p.B) * p.Hkv * n_parts : 0;
+  if (blocks + extra > 0x7fffffffLL) return B200_SDPA_ERR_UNSUPPORTED;
+  const unsigned grid = static_cast<unsigned>(blocks + extra);
   auto kern = bf16 ? (vec ? bwd_prep_kernel<__nv_bfloat16, true> : bwd_prep_kernel<__nv_bfloat16, false>)
                    : (vec ? bwd_prep_kernel<__half, true> : bwd_prep_kernel<__half, false>);
-  if (!launch_pdl(kern, dim3(grid), 256, 0, stream, bp, lse2, delta, l_pad)) return B200_SDPA_ERR_CUDA;
+  if (!launch_pdl(kern, dim3(grid), 256, 0, stream, bp, lse2, delta, l_pad, range, n_parts, static_cast<unsigned>(extra)))
+    return B200_SDPA_ERR_CUDA;
   count_launch(KID_BWD_PREP);
   return B200_SDPA_OK;
 }
@@ -959,7 +1043,7 @@ int launch_bwd_prep(const BwdProblem& bp, bool bf16, float* lse2, float* delta, 
 namespace {
 
 template <int D, bool BF16, bool BIAS, bool PAD = false>
-int launch_tc(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t stream) {
+int launch_tc(const BwdProblem& bp, float* lse2, float* delta, float2* range, cudaStream_t stream) {
   using C = BCfg<D>;
   const Problem& p = bp.f;
   CUtensorMap tq, tk, tv, tdo, tdq, tdk, tdv;
@@ -977,7 +1061,7 @@ int launch_tc(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t stre
     return B200_SDPA_ERR_CUDA;
   }
   const int l_pad = padded_rows(p);
-  const int prep = launch_bwd_prep(bp, BF16, lse2, delta, stream);
+  const int prep = launch_bwd_prep(bp, BF16, lse2, delta, range, stream);
   if (prep != B200_SDPA_OK) return prep;
   const int n_qblk = (p.L + kT - 1) / kT, n_kblk = (p.S + kT - 1) / kT;
   const long long grid_q = static_cast<long long>(n_qblk) * p.Hq * p.B;
@@ -995,12 +1079,14 @@ int launch_tc(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t stre
   // whatever follows).
   const float* c_lse2 = lse2;
   const float* c_delta = delta;
+  const float2* c_range = range;
+  const int n_parts = range_parts(p);
   if (!launch_pdl(kkv, dim3(static_cast<unsigned>(grid_kv)), kThreads, C::kSmemBytes, stream, tq, tk, tv, tdo, tdk, tdv, p, c_lse2,
-                  c_delta, l_pad, n_kblk, wave_kv, limit))
+                  c_delta, l_pad, n_kblk, wave_kv, limit, c_range, n_parts))
     return B200_SDPA_ERR_CUDA;
   count_launch(KID_BWD_DKV);
   if (!launch_pdl(kq, dim3(static_cast<unsigned>(grid_q)), kThreads, ACfg<D>::kSmemBytes, stream, tq, tk, tv, tdo, tdq, p, c_lse2,
-                  c_delta, l_pad, n_qblk, wave_q, limit))
+                  c_delta, l_pad, n_qblk, wave_q, limit, c_range, n_parts))
     return B200_SDPA_ERR_CUDA;
   count_launch(KID_BWD_DQ);
   return B200_SDPA_OK;
@@ -1049,13 +1135,25 @@ bool bwd_padded_eligible(const BwdProblem& bp, int dtype) {
   return operands_eligible(bp, dtype, nullptr);
 }
 
-uint64_t bwd_tc_workspace_bytes(const BwdProblem& bp) {
+namespace {
+
+uint64_t statistics_bytes(const BwdProblem& bp) {
   return 2ull * sizeof(float) * static_cast<uint64_t>(bp.f.B) * bp.f.Hq * padded_rows(bp.f);
+}
+// P and dS as hi + lo fp16 pairs: the shapes whose maxima the prep kernel takes
+bool scaled_gradients(const BwdProblem& bp, int dtype) {
+  return dtype == B200_SDPA_F16 && (bwd_wide_dims(bp.f) || bwd_padded_eligible(bp, dtype));
+}
+
+}  // namespace
+
+uint64_t bwd_tc_workspace_bytes(const BwdProblem& bp, int dtype) {
+  return statistics_bytes(bp) +
+         (scaled_gradients(bp, dtype) ? sizeof(float2) * static_cast<uint64_t>(bp.f.B) * bp.f.Hkv * range_parts(bp.f) : 0);
 }
 
 int plan_bwd_tc(const BwdProblem& bp, int dtype, B200SdpaPlan* plan) {
   const Problem& p = bp.f;
-  (void)dtype;
   plan->path = B200_SDPA_PATH_PREFILL;
   plan->block_m = kT;
   plan->block_n = kT;
@@ -1066,33 +1164,34 @@ int plan_bwd_tc(const BwdProblem& bp, int dtype, B200SdpaPlan* plan) {
   plan->smem_bytes = p.E == 64 && p.Dv == 64 ? BCfg<64>::kSmemBytes : BCfg<128>::kSmemBytes;
   plan->kv_splits = 1;
   plan->launches = 3;
-  plan->workspace_bytes = bwd_tc_workspace_bytes(bp);
+  plan->workspace_bytes = bwd_tc_workspace_bytes(bp, dtype);
   return B200_SDPA_OK;
 }
 
 int launch_bwd_tc(const BwdProblem& bp, int dtype, void* workspace, uint64_t workspace_bytes, cudaStream_t stream) {
   const bool padded = bwd_padded_eligible(bp, dtype);
   if (!padded && !bwd_tc_eligible(bp, dtype, nullptr)) return B200_SDPA_ERR_UNSUPPORTED;
-  const uint64_t need = bwd_tc_workspace_bytes(bp);
+  const uint64_t need = bwd_tc_workspace_bytes(bp, dtype);
   if (workspace == nullptr || workspace_bytes < need || reinterpret_cast<uintptr_t>(workspace) % 16)
     return B200_SDPA_ERR_WORKSPACE;
   float* lse2 = reinterpret_cast<float*>(workspace);
-  float* delta = lse2 + need / (2 * sizeof(float));
+  float* delta = lse2 + statistics_bytes(bp) / (2 * sizeof(float));
+  float2* range = scaled_gradients(bp, dtype) ? reinterpret_cast<float2*>(lse2 + statistics_bytes(bp) / sizeof(float)) : nullptr;
   const bool bf16 = dtype == B200_SDPA_BF16;
-  if (bwd_wide_dims(bp.f)) return launch_bwd_wide(bp, bf16, lse2, delta, stream);
+  if (bwd_wide_dims(bp.f)) return launch_bwd_wide(bp, bf16, lse2, delta, range, stream);
   if (padded) {
     if (bp.f.bias != nullptr)
-      return bf16 ? launch_tc<128, true, true, true>(bp, lse2, delta, stream) : launch_tc<128, false, true, true>(bp, lse2, delta, stream);
-    return bf16 ? launch_tc<128, true, false, true>(bp, lse2, delta, stream) : launch_tc<128, false, false, true>(bp, lse2, delta, stream);
+      return bf16 ? launch_tc<128, true, true, true>(bp, lse2, delta, range, stream) : launch_tc<128, false, true, true>(bp, lse2, delta, range, stream);
+    return bf16 ? launch_tc<128, true, false, true>(bp, lse2, delta, range, stream) : launch_tc<128, false, false, true>(bp, lse2, delta, range, stream);
   }
   if (bp.f.bias != nullptr) {
     if (bp.f.E == 128)
-      return bf16 ? launch_tc<128, true, true>(bp, lse2, delta, stream) : launch_tc<128, false, true>(bp, lse2, delta, stream);
-    return bf16 ? launch_tc<64, true, true>(bp, lse2, delta, stream) : launch_tc<64, false, true>(bp, lse2, delta, stream);
+      return bf16 ? launch_tc<128, true, true>(bp, lse2, delta, range, stream) : launch_tc<128, false, true>(bp, lse2, delta, range, stream);
+    return bf16 ? launch_tc<64, true, true>(bp, lse2, delta, range, stream) : launch_tc<64, false, true>(bp, lse2, delta, range, stream);
   }
   if (bp.f.E == 128)
-    return bf16 ? launch_tc<128, true, false>(bp, lse2, delta, stream) : launch_tc<128, false, false>(bp, lse2, delta, stream);
-  return bf16 ? launch_tc<64, true, false>(bp, lse2, delta, stream) : launch_tc<64, false, false>(bp, lse2, delta, stream);
+    return bf16 ? launch_tc<128, true, false>(bp, lse2, delta, range, stream) : launch_tc<128, false, false>(bp, lse2, delta, range, stream);
+  return bf16 ? launch_tc<64, true, false>(bp, lse2, delta, range, stream) : launch_tc<64, false, false>(bp, lse2, delta, range, stream);
 }
 
 }  // namespace b200

@@ -100,8 +100,10 @@ struct WWork {
 template <int WALK, int E, int DV, bool BF16>
 __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap* tm_fv, const CUtensorMap* tm_long,
                                      const CUtensorMap* tm_short, const CUtensorMap* tm_out, const Problem& p,
-                                     const float* lse2, const float* delta, const int l_pad, const long long wait_limit, const WWork w, uint8_t* smem_raw) {
+                                     const float* lse2, const float* delta, const int l_pad, const long long wait_limit, const float2* range,
+                                     const int n_parts, const WWork w, uint8_t* smem_raw) {
   using C = WCfg<WALK, E, DV>;
+  constexpr bool kScaled = !BF16;   // see gradient_scale
   constexpr int NT = C::kNT;
   const uint32_t tiles = smem_u32(smem_raw);
   float* stats = reinterpret_cast<float*>(smem_raw + C::kTiles);
@@ -175,6 +177,7 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
         st_d = reinterpret_cast<const float4*>(delta + src)[lane];
       }
     };
+    float gs = 1.f;   // delta is kept times this
     if (WALK != kDQ && w.n_tiles > 0) fetch_stats(0);
     bool alive = true;
     for (int j = 0; j < w.n_tiles && alive; ++j) {
@@ -188,6 +191,21 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
           break;
         }
       }
+      const uint32_t bar = smem_u32(&sync->long_full[ls]);
+      auto copy = [&]() {
+        for (int bx = 0; bx < C::kLongW / 64; ++bx)
+          tma_load_4d(long_ring + ls * C::kLongBytes + bx * C::kStreamBox, tm_long, bar, bx * 64, row, head, w.b);
+      };
+      constexpr bool kScaleDelta = kScaled && WALK == kDK;
+      if constexpr (kScaleDelta) {   // the copies go first: the maxima behind gs take a trip to L2
+        if (lane == 0) {
+          mbar_expect_tx(bar, C::kLongBytes);
+          copy();
+        }
+        __syncwarp();
+        if (j == 0) gs = gradient_scale(range, n_parts, w.b * p.Hkv + w.hk, DV, lane);
+        st_d = make_float4(st_d.x * gs, st_d.y * gs, st_d.z * gs, st_d.w * gs);
+      }
       if (WALK != kDQ) {
         if (lane < NT / 4) {
           float4* dst = reinterpret_cast<float4*>(stats + ls * 2 * NT);
@@ -197,10 +215,12 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
         __syncwarp();
       }
       if (lane == 0) {
-        const uint32_t bar = smem_u32(&sync->long_full[ls]);
-        mbar_arrive_expect_tx(bar, C::kLongBytes);
-        for (int bx = 0; bx < C::kLongW / 64; ++bx)
-          tma_load_4d(long_ring + ls * C::kLongBytes + bx * C::kStreamBox, tm_long, bar, bx * 64, row, head, w.b);
+        if constexpr (kScaleDelta) {
+          mbar_arrive(bar);
+        } else {
+          mbar_arrive_expect_tx(bar, C::kLongBytes);
+          copy();
+        }
       }
       if (WALK != kDQ && j + 1 < w.n_tiles) fetch_stats(j + 1);
       if (j >= C::kShortSlots) {
@@ -362,6 +382,9 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
     }
     const float sl2 = p.scale * kLog2e;
     const uint64_t sl2_2 = f2_pack(sl2, sl2);
+    const float gs = kScaled && WALK != kDV ? gradient_scale(range, n_parts, w.b * p.Hkv + w.hk, DV, lane) : 1.f;
+    const uint64_t gs2 = f2_pack(gs, gs);
+    const float neg_dl = -dl * gs;
     bool alive = true;
     for (int j = 0; j < w.n_tiles; ++j) {
       const int buf = j % C::kOpBufs;
@@ -389,7 +412,7 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
       uint32_t pk[HC / 2], lo[HC / 2];
 #pragma unroll
       for (int q4 = 0; q4 < HC / 4; ++q4) {
-        float nl[4] = {neg_l2, neg_l2, neg_l2, neg_l2}, nd[4] = {-dl, -dl, -dl, -dl};
+        float nl[4] = {neg_l2, neg_l2, neg_l2, neg_l2}, nd[4] = {neg_dl, neg_dl, neg_dl, neg_dl};
         if constexpr (WALK != kDQ) {
           const float4 l4 = st4[q4];
           nl[0] = -l4.x; nl[1] = -l4.y; nl[2] = -l4.z; nl[3] = -l4.w;
@@ -409,8 +432,8 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
             p1 = col0 + i + 1 >= i_min ? p1 : 0.f;
           }
           if constexpr (WALK != kDV) {
-            f2_unpack(f2_mul(f2_pack(p0, p1), f2_add(f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])), f2_pack(nd[e], nd[e + 1]))),
-                      p0, p1);
+            const uint64_t dp2 = f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])), nd2 = f2_pack(nd[e], nd[e + 1]);
+            f2_unpack(f2_mul(f2_pack(p0, p1), kScaled ? f2_fma(dp2, gs2, nd2) : f2_add(dp2, nd2)), p0, p1);
           }
           if (WALK == kDQ && need_mask) {   // after the product: dP of a hidden key may be NaN
             p0 = col0 + i < lim ? p0 : 0.f;
@@ -447,8 +470,9 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
     }
     if (alive) {
       // the fixed operands are no longer needed: their area stages the gradient
+      const float mul = (WALK == kDV ? 1.f : p.scale) * (kScaled ? 1.f / ((WALK == kDV ? 1.f : gs) * kPScale) : 1.f);
       for (int c = quarter; c < C::kAccW / 32; c += 4)
-        stage_chunk<BF16>(acc_addr, w.n_tiles > 0, WALK == kDV ? 1.f : p.scale, smem_raw, r, c, WALK == kDQ || row_g < w.n_keys);
+        stage_chunk<BF16>(acc_addr, w.n_tiles > 0, mul, smem_raw, r, c, WALK == kDQ || row_g < w.n_keys);
       fence_proxy_async_smem();
       warp_arrive(&sync->staged, lane);
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {
@@ -484,7 +508,7 @@ bwd_wide_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const __grid_constant__ CUtensorMap tm_dq, const Problem p, const float* __restrict__ lse2,
                    const float* __restrict__ delta, const int l_pad, const int n_qblk, const int streams_per_wave,
-                   const long long wait_limit) {
+                   const long long wait_limit, const float2* range, const int n_parts) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (!smem_aligned(smem_raw, p)) return;
   constexpr int NT = WCfg<kDQ, E, DV>::kNT;
@@ -518,7 +542,7 @@ bwd_wide_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
   w.min_lim = static_cast<int>(first);
   w.first_tile = 0;
   w.per_head = 1;
-  walk<kDQ, E, DV, BF16>(&tm_q, &tm_do, &tm_k, &tm_v, &tm_dq, p, lse2, delta, l_pad, wait_limit, w, smem_raw);
+  walk<kDQ, E, DV, BF16>(&tm_q, &tm_do, &tm_k, &tm_v, &tm_dq, p, lse2, delta, l_pad, wait_limit, range, n_parts, w, smem_raw);
 }
 
 template <int E, int DV, bool BF16>
@@ -527,7 +551,7 @@ bwd_wide_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                     const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
                     const Problem p, const float* lse2, const float* delta, const int l_pad,
-                    const int n_kblk, const int streams_per_wave, const long long wait_limit) {
+                    const int n_kblk, const int streams_per_wave, const long long wait_limit, const float2* range, const int n_parts) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (!smem_aligned(smem_raw, p)) return;
   constexpr int NT = WCfg<kDK, E, DV>::kNT;
@@ -558,15 +582,15 @@ bwd_wide_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
   w.n_tiles = per_head * p.group;
   w.per_head = per_head > 0 ? per_head : 1;
   if ((blockIdx.x & 1u) == 0u)
-    walk<kDK, E, DV, BF16>(&tm_k, &tm_v, &tm_q, &tm_do, &tm_dk, p, lse2, delta, l_pad, wait_limit, w, smem_raw);
+    walk<kDK, E, DV, BF16>(&tm_k, &tm_v, &tm_q, &tm_do, &tm_dk, p, lse2, delta, l_pad, wait_limit, range, n_parts, w, smem_raw);
   else
-    walk<kDV, E, DV, BF16>(&tm_k, &tm_v, &tm_do, &tm_q, &tm_dv, p, lse2, delta, l_pad, wait_limit, w, smem_raw);
+    walk<kDV, E, DV, BF16>(&tm_k, &tm_v, &tm_do, &tm_q, &tm_dv, p, lse2, delta, l_pad, wait_limit, range, n_parts, w, smem_raw);
 }
 
 // ------------------------------------------------------------------ host side --
 
 template <int E, int DV, bool BF16>
-int launch_wide(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t stream) {
+int launch_wide(const BwdProblem& bp, float* lse2, float* delta, float2* range, cudaStream_t stream) {
   const Problem& p = bp.f;
   constexpr int NT = WCfg<kDQ, E, DV>::kNT;
   constexpr int kSmemQ = WCfg<kDQ, E, DV>::kSmemBytes;
@@ -593,7 +617,7 @@ int launch_wide(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t st
   const long long grid_q = static_cast<long long>(n_qblk) * p.Hq * p.B;
   const long long grid_kv = 2LL * n_kblk * p.Hkv * p.B;
   if (grid_q > 0x7fffffffLL || grid_kv > 0x7fffffffLL) return B200_SDPA_ERR_UNSUPPORTED;
-  const int prep = launch_bwd_prep(bp, BF16, lse2, delta, stream);
+  const int prep = launch_bwd_prep(bp, BF16, lse2, delta, range, stream);
   if (prep != B200_SDPA_OK) return prep;
   const long long limit = wait_limit_cycles();
   const long long n_streams = static_cast<long long>(p.Hkv) * p.B;
@@ -601,12 +625,14 @@ int launch_wide(const BwdProblem& bp, float* lse2, float* delta, cudaStream_t st
   const int wave_kv = kv_streams_per_wave(static_cast<long long>(p.L) * p.group * ((E + DV) * 2 + 8), n_streams);
   const float* c_lse2 = lse2;
   const float* c_delta = delta;
+  const float2* c_range = range;
+  const int n_parts = range_parts(p);
   if (!launch_pdl(kkv, dim3(static_cast<unsigned>(grid_kv)), kThreads, kSmemKV, stream, k_f, v_f, q_s, do_s, dk, dv, p, c_lse2, c_delta,
-                  l_pad, n_kblk, wave_kv, limit))
+                  l_pad, n_kblk, wave_kv, limit, c_range, n_parts))
     return B200_SDPA_ERR_CUDA;
   count_launch(KID_BWD_DKV);
   if (!launch_pdl(kq, dim3(static_cast<unsigned>(grid_q)), kThreads, kSmemQ, stream, q_f, do_f, k_s, v_s, dq, p, c_lse2, c_delta, l_pad,
-                  n_qblk, wave_q, limit))
+                  n_qblk, wave_q, limit, c_range, n_parts))
     return B200_SDPA_ERR_CUDA;
   count_launch(KID_BWD_DQ);
   return B200_SDPA_OK;
@@ -619,10 +645,10 @@ bool bwd_wide_dims(const Problem& p) {
   return ((p.E == 192 && p.Dv == 128) || (p.E == 256 && p.Dv == 256)) && p.bias == nullptr;
 }
 
-int launch_bwd_wide(const BwdProblem& bp, bool bf16, float* lse2, float* delta, cudaStream_t stream) {
+int launch_bwd_wide(const BwdProblem& bp, bool bf16, float* lse2, float* delta, float2* range, cudaStream_t stream) {
   if (bp.f.E == 192)
-    return bf16 ? launch_wide<192, 128, true>(bp, lse2, delta, stream) : launch_wide<192, 128, false>(bp, lse2, delta, stream);
-  return bf16 ? launch_wide<256, 256, true>(bp, lse2, delta, stream) : launch_wide<256, 256, false>(bp, lse2, delta, stream);
+    return bf16 ? launch_wide<192, 128, true>(bp, lse2, delta, range, stream) : launch_wide<192, 128, false>(bp, lse2, delta, range, stream);
+  return bf16 ? launch_wide<256, 256, true>(bp, lse2, delta, range, stream) : launch_wide<256, 256, false>(bp, lse2, delta, range, stream);
 }
 
 }  // namespace b200

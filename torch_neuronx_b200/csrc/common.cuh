@@ -135,9 +135,9 @@ int plan_bwd_generic(const BwdProblem& bp, int dtype, B200SdpaPlan* plan);
 bool bwd_tc_eligible(const BwdProblem& bp, int dtype, bool* alignment_only_failure);
 // head dimensions 192/128 and 256 (bwd_wide_sm100.cu)
 bool bwd_wide_dims(const Problem& p);
-int launch_bwd_wide(const BwdProblem& bp, bool bf16, float* lse2, float* delta, cudaStream_t stream);
+int launch_bwd_wide(const BwdProblem& bp, bool bf16, float* lse2, float* delta, float2* range, cudaStream_t stream);
 bool bwd_padded_eligible(const BwdProblem& bp, int dtype);
-uint64_t bwd_tc_workspace_bytes(const BwdProblem& bp);
+uint64_t bwd_tc_workspace_bytes(const BwdProblem& bp, int dtype);
 int plan_bwd_tc(const BwdProblem& bp, int dtype, B200SdpaPlan* plan);
 int launch_bwd_tc(const BwdProblem& bp, int dtype, void* workspace, uint64_t workspace_bytes, cudaStream_t stream);
 

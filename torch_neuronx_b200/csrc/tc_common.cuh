@@ -208,7 +208,9 @@ __device__ __forceinline__ void zero_tile_rows(uint32_t tile, int row0, int lane
 
 // What rounding (x0, x1) to the 16-bit pair `hi` left over, rounded to 16 bits itself.  Where a shape was served with
 // fp32 probabilities before, the second product takes both parts, hi + lo, as two operands: 2^-16 (bf16) or 2^-22
-// (fp16) of the value is lost, far below the rounding of the result.
+// (fp16) of the value is lost, far below the rounding of the result.  In fp16 that holds above 2^-3; below, lo is
+// subnormal and what is lost is 2^-25 -- of a row whose largest probability is 1 in the forward; the backward brings its
+// operands into range first (gradient_scale).
 template <bool BF16>
 __device__ __forceinline__ uint32_t remainder2(float x0, float x1, uint32_t hi) {
   float h0, h1;
