@@ -443,9 +443,11 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         return false;
       }
       tc_fence_after_sync();
-      // (PAD: these shapes came from kernels that leave out what lies beyond kv_lens, and dS = 0 times a NaN row of K is NaN)
-      if (PAD && kv_limit < p.S && (j + 1) * kT > kv_limit)
+      // (PAD: these shapes came from kernels that leave out what lies beyond kv_lens; P = 0 times a NaN of V or K is NaN)
+      if (PAD && kv_limit < p.S && (j + 1) * kT > kv_limit) {
         zero_tile_rows<C::kBoxes, kT>(k_ring + ks * C::kTileBytes, kv_limit - j * kT, lane);
+        zero_tile_rows<C::kBoxes, kT>(v_ring + vs * C::kTileBytes, kv_limit - j * kT, lane);
+      }
       const uint64_t qd = kmajor_desc(q_tile), kd = kmajor_desc(k_ring + ks * C::kTileBytes);
       const uint64_t od = kmajor_desc(do_tile), vd = kmajor_desc(v_ring + vs * C::kTileBytes);
       if (elect_one()) {
@@ -575,17 +577,13 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         f2_unpack(f2_fma(f2_pack(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2_2, f2_pack(off0, off1)), a0, a1);
         float p0 = ex2(a0);
         float p1 = ex2(a1);
-        if (!PAD && need_mask) {
+        if (need_mask) {
           p0 = (col0 + i < lim) ? p0 : 0.f;
           p1 = (col0 + i + 1 < lim) ? p1 : 0.f;
         }
         float d0, d1;
         const uint64_t dp2 = f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1]));
         f2_unpack(f2_mul(f2_pack(p0, p1), kScaled ? f2_fma(dp2, gs2, neg_dl2) : f2_add(dp2, neg_dl2)), d0, d1);
-        if (PAD && need_mask) {   // after the product: dP of a hidden key may be NaN
-          d0 = (col0 + i < lim) ? d0 : 0.f;
-          d1 = (col0 + i + 1 < lim) ? d1 : 0.f;
-        }
         pk[i >> 1] = pack2<BF16>(d0, d1);
         if constexpr (PAD) lo[i >> 1] = remainder2<BF16>(d0, d1, pk[i >> 1]);
       }

@@ -269,7 +269,7 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
       tc_fence_after_sync();
       const uint32_t e_tile = WALK == kDV ? short_ring + (j % C::kShortSlots) * C::kShortBytes
                                           : long_ring + (j % C::kLongSlots) * C::kLongBytes;
-      // (as in bwd_sm100.cu: keys beyond kv_lens, which the product dS K reads with dS = 0)
+      // (as in bwd_sm100.cu: keys beyond kv_lens, here and in dP)
       if (WALK == kDQ && w.n_keys < p.S && (j + 1) * NT > w.n_keys) zero_tile_rows<E / 64, NT>(e_tile, w.n_keys - j * NT, lane);
       const uint64_t fd = kmajor_desc(fe_tile), gd = kmajor_desc(e_tile);
       if (elect_one()) {
@@ -283,6 +283,8 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
       if (!(WALK == kDV ? wait_long(j) : wait_short(j))) return false;
       tc_fence_after_sync();
       const int ss = j % C::kShortSlots;
+      if (WALK == kDQ && w.n_keys < p.S && (j + 1) * NT > w.n_keys)
+        zero_tile_rows<DV / 64, NT>(short_ring + ss * C::kShortBytes, w.n_keys - j * NT, lane);
       const uint64_t fvd = kmajor_desc(fv_tile), gvd = kmajor_desc(short_ring + ss * C::kShortBytes);
       if (elect_one()) {
         if (WALK != kDV) {
@@ -427,17 +429,13 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
           float a0, a1;
           f2_unpack(f2_fma(f2_pack(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2_2, f2_pack(nl[e], nl[e + 1])), a0, a1);
           float p0 = ex2(a0), p1 = ex2(a1);
-          if (WALK != kDQ && need_mask) {
-            p0 = col0 + i >= i_min ? p0 : 0.f;
-            p1 = col0 + i + 1 >= i_min ? p1 : 0.f;
+          if (need_mask) {
+            p0 = (WALK == kDQ ? col0 + i < lim : col0 + i >= i_min) ? p0 : 0.f;
+            p1 = (WALK == kDQ ? col0 + i + 1 < lim : col0 + i + 1 >= i_min) ? p1 : 0.f;
           }
           if constexpr (WALK != kDV) {
             const uint64_t dp2 = f2_pack(__uint_as_float(dv[i]), __uint_as_float(dv[i + 1])), nd2 = f2_pack(nd[e], nd[e + 1]);
             f2_unpack(f2_mul(f2_pack(p0, p1), kScaled ? f2_fma(dp2, gs2, nd2) : f2_add(dp2, nd2)), p0, p1);
-          }
-          if (WALK == kDQ && need_mask) {   // after the product: dP of a hidden key may be NaN
-            p0 = col0 + i < lim ? p0 : 0.f;
-            p1 = col0 + i + 1 < lim ? p1 : 0.f;
           }
           pk[i >> 1] = pack2<BF16>(p0, p1);
           lo[i >> 1] = remainder2<BF16>(p0, p1, pk[i >> 1]);
