@@ -132,7 +132,9 @@ typedef struct B200SdpaParams {
   int32_t kv_chunk;       /* decode: keys per split, 0 = library default               */
   int64_t bias_stride[4]; /* 0 for broadcast dimensions                                */
 
-  void* workspace;        /* scratch, b200_sdpa_query_plan() says how much             */
+  void* workspace;        /* scratch, b200_sdpa_query_plan() says how much; on 4 bytes
+                             for the decode path (16 are faster), other paths do
+                             without one that is not on 16                             */
   uint64_t workspace_bytes;
   int32_t* status;        /* optional device int32[4]: [0] = first error code seen by
                              a kernel (0 = none), [1..3] = where; caller zeroes it     */

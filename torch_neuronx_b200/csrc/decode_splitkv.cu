@@ -223,10 +223,11 @@ __global__ void __launch_bounds__(kThreads) decode_partial_kernel(const Problem 
 
 // Merge of the partials: one CTA of four warps per (batch, query head).  Every warp takes every fourth split (the
 // (max, sum) pairs of all splits are read once, 32 at a time), then the four states meet in shared memory.  Bound by
-// latency: two dependent rounds of loads, whatever the number of splits up to 128.
+// latency: two dependent rounds of loads, whatever the number of splits up to 128.  WIDE: the scratch starts on 16 bytes
+// and is read in vectors; a caller's scratch need not (the partial kernels store single floats).
 constexpr int kCombineWarps = 4;
 
-template <typename T, int D>
+template <typename T, int D, bool WIDE>
 __global__ void __launch_bounds__(kCombineWarps * 32) decode_combine_kernel(const Problem p, const int chunk, const int nsplit,
                                                                             const float* __restrict__ part_o,
                                                                             const float* __restrict__ part_ml) {
@@ -257,11 +258,19 @@ __global__ void __launch_bounds__(kCombineWarps * 32) decode_combine_kernel(cons
   for (int c = 0; c < C; ++c) acc[c] = 0.f;
 #pragma unroll 4
   for (int s = warp; s < used; s += kCombineWarps) {
-    const float2 ml = *reinterpret_cast<const float2*>(part_ml + (slot0 + s) * 2);
+    const float* pair = part_ml + (slot0 + s) * 2;
     const float* src = part_o + (slot0 + s) * D + lane * C;
+    float2 ml;
     float v[C];
-    if constexpr (C == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src);
-    else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(src);
+    if constexpr (WIDE) {
+      ml = *reinterpret_cast<const float2*>(pair);
+      if constexpr (C == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src);
+      else *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(src);
+    } else {
+      ml = make_float2(pair[0], pair[1]);
+#pragma unroll
+      for (int c = 0; c < C; ++c) v[c] = src[c];
+    }
     const float w = exp2f(ml.x - ms);
     lsum = fmaf(ml.y, w, lsum);
 #pragma unroll
@@ -342,8 +351,8 @@ DecodeGeom geometry(const Problem& p, int kv_chunk) {
 
 template <typename T, int D>
 int launch_combine(const Problem& p, const DecodeGeom& gm, float* po, float* pml, cudaStream_t stream) {
-  if (!launch_pdl(decode_combine_kernel<T, D>, dim3(p.B * p.Hq), kCombineWarps * 32, 0, stream, p, gm.chunk, gm.nsplit, po, pml))
-    return B200_SDPA_ERR_CUDA;
+  auto kern = reinterpret_cast<uintptr_t>(po) % 16 == 0 ? decode_combine_kernel<T, D, true> : decode_combine_kernel<T, D, false>;
+  if (!launch_pdl(kern, dim3(p.B * p.Hq), kCombineWarps * 32, 0, stream, p, gm.chunk, gm.nsplit, po, pml)) return B200_SDPA_ERR_CUDA;
   count_launch(KID_COMBINE);
   return B200_SDPA_OK;
 }
