@@ -356,7 +356,8 @@ int b200_sdpa_decode(const B200SdpaParams* params, void* stream);
  * memory to their own pool at start-up, or that run where allocator calls are not
  * allowed; the call itself performs no allocation of any kind.
  *   - a request whose partials need more than the capacity (see `workspace_bytes`
- *     of b200_sdpa_query_plan) returns B200_SDPA_ERR_TOO_LARGE and launches nothing;
+ *     of b200_sdpa_query_plan) returns B200_SDPA_ERR_TOO_LARGE and launches nothing; with
+ *     kv_chunk = 0 the library first lengthens its chunks, up to 2048 keys;
  *   - the first call on each device resolves the array's device address; make that
  *     first call outside any stream capture;
  *   - all calls share the one array, which keeps the previous call's contents; the

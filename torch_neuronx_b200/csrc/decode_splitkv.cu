@@ -296,6 +296,8 @@ __global__ void __launch_bounds__(kCombineWarps * 32) decode_combine_kernel(cons
 
 int pick_group(int group) { return group >= 8 ? 8 : group > 2 ? 4 : group; }
 
+constexpr int kMaxChunk = 2048;
+
 // Keys per CTA.  A model of the launch, fitted to measurements (bf16, head dimension 128, 1 to 128 sequences of 512 to
 // 32768 keys, within a tenth of the best chunk everywhere): up to kSlots CTAs run at a time; a CTA needs kFixed for its
 // start and end and, per block of 64 keys, kBlock alone (the latency of its two-stage ring) and kShared more when all
@@ -319,7 +321,7 @@ int default_chunk(const Problem& p) {
   };
   int best = 256;
   double best_us = 1e30;
-  for (int chunk = 64; chunk <= 2048; chunk += chunk < 512 ? 64 : 256) {
+  for (int chunk = 64; chunk <= kMaxChunk; chunk += chunk < 512 ? 64 : 256) {
     const int n = (p.S + chunk - 1) / chunk;
     double t = launch_us(units * n, chunk, false);
     if (p.kv_lens != nullptr) t += 2 * launch_us(units * (n + 1) / 2, chunk, true);
@@ -489,7 +491,12 @@ void* g_scratch_ptr[kMaxDevices] = {};
 
 int launch_decode_static(const Problem& p, int dtype, int kv_chunk, cudaStream_t stream) {
   if (!decode_eligible(p, dtype)) return B200_SDPA_ERR_UNSUPPORTED;
-  const DecodeGeom gm = geometry(p, kv_chunk);
+  DecodeGeom gm = geometry(p, kv_chunk);
+  // the library's own choice of chunk, which is made for speed with scratch of any size, gives way to longer ones
+  for (int chunk = gm.chunk; kv_chunk <= 0 && gm.ws_bytes > kStaticScratchBytes && chunk < kMaxChunk;) {
+    chunk = chunk + 256 < kMaxChunk ? chunk + 256 : kMaxChunk;
+    gm = geometry(p, chunk);
+  }
   if (gm.ws_bytes > kStaticScratchBytes) return B200_SDPA_ERR_TOO_LARGE;
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
@@ -509,7 +516,7 @@ int launch_decode_static(const Problem& p, int dtype, int kv_chunk, cudaStream_t
     }
     ptr = g_scratch_ptr[dev];
   }
-  return launch_decode(p, dtype, kv_chunk, ptr, kStaticScratchBytes, stream);
+  return launch_decode(p, dtype, gm.chunk, ptr, kStaticScratchBytes, stream);
 }
 
 
