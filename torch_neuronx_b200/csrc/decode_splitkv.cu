@@ -299,7 +299,7 @@ int pick_group(int group) { return group >= 8 ? 8 : group > 2 ? 4 : group; }
 constexpr int kMaxChunk = 2048;
 
 // Keys per CTA.  A model of the launch, fitted to measurements (bf16, head dimension 128, 1 to 128 sequences of 512 to
-// 32768 keys, within a tenth of the best chunk everywhere): up to kSlots CTAs run at a time; a CTA needs kFixed for its
+// 32768 keys, within a tenth of the best chunk everywhere): up to `slots` CTAs run at a time; a CTA needs kFixed for its
 // start and end and, per block of 64 keys, kBlock alone (the latency of its two-stage ring) and kShared more when all
 // slots are taken (its share of the HBM rate).  Short chunks pay kFixed too often, long ones leave SMs without work.
 // More CTAs than slots cost, on average, a third of a round for the last, partly filled one -- less when their lengths
@@ -307,14 +307,20 @@ constexpr int kMaxChunk = 2048;
 // evenly up to S are added, else full caches are assumed.  A paged cache's block costs more alone (table and address
 // arithmetic).  16 sequences of 128..4000 keys, 4096 cached, 32/8 heads: 34.9 us at the 256 keys taken before, 32.3 at
 // the 1024 taken now (paged, with append: 41.1 -> 33.5 at 768); one sequence of 30000 keys 41.2 -> 31.8.
+// At head dimension 64 four CTAs fit on an SM (128 registers), a block's share of the HBM rate halves, and every
+// partial of a (batch, head) adds `merge` to the second kernel, which is then no longer small.  242 dense and 242 paged problems
+// (1 to 100 sequences of 512 to 32768 keys, 1 to 12 kv heads; device time): 3 % faster on the geometric mean than with
+// the constants of 128, 5 % than with 256..2048 keys by S and the number of units alone; more than 5 % slower than
+// that older rule in 42 of them (90 with the constants of 128), at worst 8 x 4096 keys ragged, 11.8 us against 14.0.
 int default_chunk(const Problem& p) {
-  constexpr double kSlots = 444, kFixed = 3.5;        // us
+  constexpr double kFixed = 3.5;        // us
+  const double slots = p.E == 64 ? 592 : 444, merge = p.E == 64 ? 0.1 : 0.0;
   const double block = p.block_table != nullptr ? 1.12 : 0.71;
   const int sub = (p.group + 15) / 16;
   const double shared = 1.6 * (p.E + p.Dv) / 256.0;
   const double units = static_cast<double>(p.B) * p.Hkv * sub;
   auto launch_us = [&](double ctas, int chunk, bool ragged) {
-    const double blocks = chunk / 64.0, fill = ctas / kSlots;
+    const double blocks = chunk / 64.0, fill = ctas / slots;
     if (fill <= 1.0) return kFixed + blocks * (block + shared * fill);
     const double over = ragged && fill < 4.0 / 3.0 ? 3.0 * (fill - 1.0) : 1.0;
     return (fill + 0.35 * over) * (kFixed + blocks * (block + shared));
@@ -324,7 +330,8 @@ int default_chunk(const Problem& p) {
   for (int chunk = 64; chunk <= kMaxChunk; chunk += chunk < 512 ? 64 : 256) {
     const int n = (p.S + chunk - 1) / chunk;
     double t = launch_us(units * n, chunk, false);
-    if (p.kv_lens != nullptr) t += 2 * launch_us(units * (n + 1) / 2, chunk, true);
+    t += merge * n;
+    if (p.kv_lens != nullptr) t += 2 * launch_us(units * (n + 1) / 2, chunk, true) + merge * (n + 1);
     t *= 1.0 + 0.002 * n;   // equal: fewer partials
     if (t < best_us) {
       best_us = t;
