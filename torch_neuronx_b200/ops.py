@@ -141,6 +141,16 @@ def _workspace(dev: int, nbytes: int) -> torch.Tensor:
     return w
 
 
+def _bias_scratch(dev: int, nbytes: int) -> Optional[torch.Tensor]:
+    """Scratch for one forward call with a bias, which may be a copy of that bias: too large to keep.  The block goes
+    back to the (stream-ordered) caching allocator when the call has been queued.  None where it cannot be had: every
+    such request has a kernel that needs no scratch."""
+    try:
+        return torch.empty(nbytes, dtype=torch.uint8, device=torch.device("cuda", dev))
+    except torch.OutOfMemoryError:
+        return None
+
+
 def release_workspaces() -> None:
     """Drop every cached scratch buffer (also the retired ones).  Only safe when no CUDA graph
     that was captured through this module will be replayed again."""
@@ -325,7 +335,8 @@ def sdpa_forward(
         raise RuntimeError(f"b200_sdpa_query_plan: {_lib.strerror(rc)}")
     ws = None
     if plan.workspace_bytes:
-        ws = _workspace(dev, int(plan.workspace_bytes))
+        ws = _workspace(dev, int(plan.workspace_bytes)) if attn_bias is None else _bias_scratch(dev, int(plan.workspace_bytes))
+    if ws is not None:
         p.workspace = ws.data_ptr()
         p.workspace_bytes = ws.numel()
     stream = torch.cuda.current_stream(dev).cuda_stream
