@@ -250,6 +250,7 @@ def load():
 
 _ops_loaded = None
 native = None   # the extension module with the direct entry points (csrc_ops/py_calls.cpp), once loaded
+last_plan: dict = {}   # the plan of the last forward call (ops.last_plan), filled by whichever layer made the call
 
 
 def load_ops() -> bool:
@@ -273,8 +274,9 @@ def load_ops() -> bool:
                     if os.path.exists(NATIVE_PATH):
                         from . import _native as module
 
+                        module.set_plan_record(last_plan)
                         native = module
-                except (OSError, ImportError) as exc:
+                except (OSError, ImportError, AttributeError) as exc:
                     # a library from an interrupted or outdated build: importing the package must still work
                     # (the build itself runs as a module of it); any compute call will report the real problem
                     import warnings

@@ -22,7 +22,6 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
-#include <mutex>
 
 #include "ops_common.h"
 
@@ -35,14 +34,33 @@ struct NoGil {   // the interpreter lock is released for the lifetime of the obj
   ~NoGil() { PyEval_RestoreThread(state); }
 };
 
-std::mutex g_plan_mutex;
-B200SdpaPlan g_plan{};       // the last plan made here, until Python takes it
-bool g_plan_fresh = false;
+// The record of the last forward's plan: the dict of the Python layer, filled under the interpreter lock.
+PyObject* g_plan_record = nullptr;
 
-void keep_plan(const B200SdpaPlan& plan) {
-  std::lock_guard<std::mutex> lock(g_plan_mutex);
-  g_plan = plan;
-  g_plan_fresh = true;
+bool record_plan(const B200SdpaPlan& plan) {
+  if (g_plan_record == nullptr) return true;
+  static PyObject* const names[] = {
+      PyUnicode_InternFromString("path"),      PyUnicode_InternFromString("block_m"),    PyUnicode_InternFromString("block_n"),
+      PyUnicode_InternFromString("grid"),      PyUnicode_InternFromString("threads"),    PyUnicode_InternFromString("smem_bytes"),
+      PyUnicode_InternFromString("kv_splits"), PyUnicode_InternFromString("launches"),   PyUnicode_InternFromString("workspace_bytes")};
+  static PyObject* const paths[] = {PyUnicode_InternFromString("auto"), PyUnicode_InternFromString("generic"),
+                                    PyUnicode_InternFromString("prefill"), PyUnicode_InternFromString("decode")};
+  PyObject* const values[] = {Py_NewRef(paths[plan.path & 3]),
+                              PyLong_FromLong(plan.block_m),
+                              PyLong_FromLong(plan.block_n),
+                              Py_BuildValue("(iii)", plan.grid_x, plan.grid_y, plan.grid_z),
+                              PyLong_FromLong(plan.threads),
+                              PyLong_FromLong(plan.smem_bytes),
+                              PyLong_FromLong(plan.kv_splits),
+                              PyLong_FromLong(plan.launches),
+                              PyLong_FromUnsignedLongLong(plan.workspace_bytes)};
+  PyDict_Clear(g_plan_record);
+  bool ok = true;
+  for (int i = 0; i < 9; ++i) {
+    ok = ok && values[i] != nullptr && PyDict_SetItem(g_plan_record, names[i], values[i]) == 0;
+    Py_XDECREF(values[i]);
+  }
+  return ok;
 }
 
 // A plain strided CUDA tensor with nothing between it and the kernels; a dual tensor of forward-mode differentiation
@@ -126,10 +144,9 @@ void fill_common(B200SdpaParams& p, const at::Tensor& q, const at::Tensor& out, 
 }
 
 // Plan, scratch, launch; the interpreter lock is not held.
-void launch(B200SdpaParams& p, int dev, bool decode_only) {
+void launch(B200SdpaParams& p, int dev, bool decode_only, B200SdpaPlan& plan) {
   at::Tensor ws;   // freed (stream-ordered) when the launch has been queued
   NoGil nogil;
-  B200SdpaPlan plan{};
   plan.struct_size = sizeof(B200SdpaPlan);
   int rc = b200_sdpa_query_plan(&p, &plan);
   TORCH_CHECK(rc == B200_SDPA_OK, "b200_sdpa_query_plan: ", b200_sdpa_strerror(rc));
@@ -141,7 +158,6 @@ void launch(B200SdpaParams& p, int dev, bool decode_only) {
   const auto stream = c10::cuda::getCurrentCUDAStream(dev).stream();
   rc = decode_only ? b200_sdpa_decode(&p, stream) : b200_sdpa_fwd(&p, stream);
   TORCH_CHECK(rc == B200_SDPA_OK, decode_only ? "b200_sdpa_decode: " : "b200_sdpa_fwd: ", b200_sdpa_strerror(rc));
-  if (!decode_only) keep_plan(plan);
 }
 
 struct ForwardArgs {
@@ -151,7 +167,8 @@ struct ForwardArgs {
   at::Tensor lens;
 };
 
-void forward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const ForwardArgs& a, const at::Tensor& out,
+// False: a Python error is set.
+bool forward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const ForwardArgs& a, const at::Tensor& out,
              const at::Tensor& lse) {
   const int dev = q.device().index();
   B200SdpaParams p{};
@@ -170,7 +187,9 @@ void forward(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, cons
   p.k_offset = a.k_offset;
   p.kv_chunk = static_cast<int32_t>(a.kv_chunk);
   if (a.lens.defined()) p.kv_lens = a.lens.data_ptr<int32_t>();
-  launch(p, dev, false);
+  B200SdpaPlan plan{};
+  launch(p, dev, false, plan);
+  return record_plan(plan);
 }
 
 #define NOT_SERVED() do { if (PyErr_Occurred()) PyErr_Clear(); Py_RETURN_NONE; } while (0)
@@ -199,7 +218,7 @@ PyObject* py_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
   } else {
     const c10::cuda::CUDAGuard guard(q.device());
     out = alloc_like_query(q, {q.size(0), q.size(1), q.size(2), v.size(3)});
-    forward(q, k, v, a, out, at::Tensor());
+    if (!forward(q, k, v, a, out, at::Tensor())) return nullptr;
   }
   return THPVariable_Wrap(out);
   END_HANDLE_TH_ERRORS
@@ -232,7 +251,7 @@ PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const c10::cuda::CUDAGuard guard(q.device());
   if (!out.defined()) out = alloc_like_query(q, {B, H, L, Dv});
   if (!lse.defined() && need_lse) lse = at::empty({B, H, L}, q.options().dtype(at::kFloat));
-  forward(q, k, v, a, out, lse);
+  if (!forward(q, k, v, a, out, lse)) return nullptr;
   PyObject* po = THPVariable_Wrap(out);
   PyObject* pl = lse.defined() ? THPVariable_Wrap(lse) : Py_NewRef(Py_None);
   return Py_BuildValue("(NN)", po, pl);
@@ -333,7 +352,8 @@ PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
     new_lens = at::empty_like(lens);
     p.kv_lens_out = new_lens.data_ptr<int32_t>();
   }
-  launch(p, dev, true);
+  B200SdpaPlan plan{};
+  launch(p, dev, true, plan);
   PyObject* po = THPVariable_Wrap(out);
   PyObject* pl = lse.defined() ? THPVariable_Wrap(lse) : Py_NewRef(Py_None);
   PyObject* pn = new_lens.defined() ? THPVariable_Wrap(new_lens) : Py_NewRef(Py_None);
@@ -341,25 +361,23 @@ PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// take_plan() -> the plan of the last forward made here as a tuple, once; None if there is none since
-PyObject* py_take_plan(PyObject*, PyObject*) {
-  B200SdpaPlan plan;
-  {
-    std::lock_guard<std::mutex> lock(g_plan_mutex);
-    if (!g_plan_fresh) Py_RETURN_NONE;
-    plan = g_plan;
-    g_plan_fresh = false;
+// set_plan_record(dict): where every forward made here leaves its plan
+PyObject* py_set_plan_record(PyObject*, PyObject* record) {
+  if (!PyDict_CheckExact(record)) {
+    PyErr_SetString(PyExc_TypeError, "set_plan_record: a dict");
+    return nullptr;
   }
-  return Py_BuildValue("(iiiiiiiiiiK)", plan.path, plan.block_m, plan.block_n, plan.grid_x, plan.grid_y, plan.grid_z,
-                       plan.threads, plan.smem_bytes, plan.kv_splits, plan.launches,
-                       static_cast<unsigned long long>(plan.workspace_bytes));
+  PyObject* old = g_plan_record;
+  g_plan_record = Py_NewRef(record);
+  Py_XDECREF(old);
+  Py_RETURN_NONE;
 }
 
 PyMethodDef kMethods[] = {
     {"attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attention)), METH_FASTCALL, nullptr},
     {"forward", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_forward)), METH_FASTCALL, nullptr},
     {"decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_decode)), METH_FASTCALL, nullptr},
-    {"take_plan", py_take_plan, METH_NOARGS, nullptr},
+    {"set_plan_record", py_set_plan_record, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

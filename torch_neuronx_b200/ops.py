@@ -26,7 +26,6 @@ fallback: non-CUDA tensors are rejected and a missing library raises.
 
 from __future__ import annotations
 
-import collections.abc
 import ctypes as C
 import math
 from typing import Optional
@@ -46,51 +45,8 @@ _status_words: dict[int, torch.Tensor] = {}
 _zero_scalars: dict[int, tuple] = {}
 _workspaces: dict[tuple[int, int], torch.Tensor] = {}
 _retired_workspaces: list = []
+last_plan = _lib.last_plan
 last_bwd_plan: dict = {}
-
-
-class _LastPlan(collections.abc.MutableMapping):
-    """The plan of the last forward call.  A call made by the direct native entry points leaves its plan there
-    and it is turned into a dict only when somebody looks."""
-
-    def __init__(self):
-        self._d: dict = {}
-
-    def _now(self) -> dict:
-        t = _lib.native.take_plan() if _lib.native is not None else None
-        if t is not None:
-            path, block_m, block_n, gx, gy, gz, threads, smem, splits, launches, workspace = t
-            self._d = dict(
-                path=_lib.PATH_NAMES.get(path, str(path)), block_m=block_m, block_n=block_n, grid=(gx, gy, gz),
-                threads=threads, smem_bytes=smem, kv_splits=splits, launches=launches, workspace_bytes=workspace,
-            )
-        return self._d
-
-    def __getitem__(self, key):
-        return self._now()[key]
-
-    def __setitem__(self, key, value):
-        self._now()[key] = value
-
-    def __delitem__(self, key):
-        del self._now()[key]
-
-    def __iter__(self):
-        return iter(self._now())
-
-    def __len__(self):
-        return len(self._now())
-
-    def clear(self):
-        if _lib.native is not None:
-            _lib.native.take_plan()
-        self._d = {}
-
-    def __repr__(self):
-        return repr(self._now())
-
-
-last_plan = _LastPlan()
 
 
 def _device_index(t: torch.Tensor) -> int:
