@@ -300,8 +300,8 @@ template <int D, bool BF16, bool BIAS, bool PAD>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                 const __grid_constant__ CUtensorMap tm_dq, const Problem p, const float* __restrict__ lse2,
-                 const float* __restrict__ delta, const int l_pad, const int n_qblk, const int streams_per_wave,
+                 const __grid_constant__ CUtensorMap tm_dq, const Problem p, const float* lse2,
+                 const float* delta, const int l_pad, const int n_qblk, const int streams_per_wave,
                  const long long wait_limit, const float2* range, const int n_parts) {
   using C = ACfg<D>;
   extern __shared__ uint8_t smem_raw[];
@@ -527,8 +527,11 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     const long long stat_idx = (static_cast<long long>(b) * p.Hq + h) * l_pad + row_g;
     const bool stat_ok = dbg_range(p.status, DBG_BWD_TC * 100 + 6, stat_idx, 1, static_cast<long long>(p.B) * p.Hq * l_pad);
-    const float neg_l2 = stat_ok ? -lse2[stat_idx] : -CUDART_INF_F;      // -inf for rows without a visible key
-    const float dl = stat_ok ? delta[stat_idx] : 0.f;
+    // Read past L1.  This grid starts when every CTA of the dK/dV grid is past its wait for the prep kernel, so the
+    // statistics are in L2; but no wait of its own orders them before these reads, and they lie at the address where
+    // the last call's lay, which an L1 may still hold.
+    const float neg_l2 = stat_ok ? -__ldcg(lse2 + stat_idx) : -CUDART_INF_F;   // -inf for rows without a visible key
+    const float dl = stat_ok ? __ldcg(delta + stat_idx) : 0.f;
     const float sl2 = p.scale * kLog2e;
     const float gs = kScaled ? gradient_scale(range, n_parts, kv_stream, p.Dv, lane) : 1.f;
     const float undo = kScaled ? 1.f / (gs * kPScale) : 1.f;
@@ -675,6 +678,10 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int hk = kv_stream % p.Hkv;
   const int b = kv_stream / p.Hkv;
   const int j0 = kblk * kT;
+  // A programmatic dependent of the prep kernel: its launch overlaps that kernel, nothing of global memory is touched
+  // before the wait.  (The dQ kernel, which follows without a wait of its own: see there.)
+  pdl_wait();
+  pdl_launch_dependents();
   const int n_keys = valid_keys(p, b);
   const int n_qt = (p.L + kT - 1) / kT;
   int i_first = 0;
@@ -711,12 +718,6 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     tmem_alloc(smem_u32(&sync->tmem_base), kTmemCols);
     tmem_relinquish();
   }
-  // A programmatic dependent of the prep kernel.  Everything above, the copies of K and V too, may run before that
-  // grid is done: it writes the row statistics only, and its own wait was over before this grid could start.  The
-  // dQ kernel reads the statistics without a wait of its own and nothing that this kernel writes, so it may start
-  // once every CTA of this grid is past the wait.
-  pdl_wait();
-  pdl_launch_dependents();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();

@@ -152,10 +152,6 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
     tmem_alloc(smem_u32(&sync->tmem_base), kTmemCols);
     tmem_relinquish();
   }
-  if (WALK != kDQ) {   // as in bwd_sm100.cu: the row statistics are not read before the prep kernel is done
-    pdl_wait();
-    pdl_launch_dependents();
-  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -379,8 +375,8 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
     if (WALK == kDQ) {
       const long long idx = (static_cast<long long>(w.b) * p.Hq + w.h) * l_pad + row_g;
       const bool ok = dbg_range(p.status, DBG_BWD_WIDE * 100 + 6, idx, 1, static_cast<long long>(p.B) * p.Hq * l_pad);
-      neg_l2 = ok ? -lse2[idx] : -CUDART_INF_F;   // -inf for rows without a visible key
-      dl = ok ? delta[idx] : 0.f;
+      neg_l2 = ok ? -__ldcg(lse2 + idx) : -CUDART_INF_F;   // -inf for rows without a visible key (past L1: as in bwd_sm100.cu)
+      dl = ok ? __ldcg(delta + idx) : 0.f;
     }
     const float sl2 = p.scale * kLog2e;
     const uint64_t sl2_2 = f2_pack(sl2, sl2);
@@ -504,8 +500,8 @@ template <int E, int DV, bool BF16>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd_wide_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                   const __grid_constant__ CUtensorMap tm_dq, const Problem p, const float* __restrict__ lse2,
-                   const float* __restrict__ delta, const int l_pad, const int n_qblk, const int streams_per_wave,
+                   const __grid_constant__ CUtensorMap tm_dq, const Problem p, const float* lse2,
+                   const float* delta, const int l_pad, const int n_qblk, const int streams_per_wave,
                    const long long wait_limit, const float2* range, const int n_parts) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   if (!smem_aligned(smem_raw, p)) return;
@@ -551,6 +547,8 @@ bwd_wide_dkv_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_const
                     const Problem p, const float* lse2, const float* delta, const int l_pad,
                     const int n_kblk, const int streams_per_wave, const long long wait_limit, const float2* range, const int n_parts) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  pdl_wait();   // as in bwd_sm100.cu
+  pdl_launch_dependents();
   if (!smem_aligned(smem_raw, p)) return;
   constexpr int NT = WCfg<kDK, E, DV>::kNT;
   // Earliest key blocks (seen by the most query tiles under a causal mask) first, within waves of groups whose
