@@ -62,10 +62,9 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
 }
 
 // 32 columns (chunk c) of one thread's accumulator row (TMEM lane) -> 16-bit -> the 128-byte-swizzled staging tile a
-// TMA store expects; zeros for a row that is not to be kept (a key beyond kv_lens, whose own dP may be NaN).
+// TMA store expects.
 template <bool BF16>
-__device__ __forceinline__ void stage_chunk(uint32_t acc_addr, bool have_acc, float mul, uint8_t* stage, int r, int c,
-                                            bool keep = true) {
+__device__ __forceinline__ void stage_chunk(uint32_t acc_addr, bool have_acc, float mul, uint8_t* stage, int r, int c) {
   uint32_t v[32];
   if (have_acc) {
     tmem_ld_32x32(acc_addr + c * 32, v);
@@ -77,7 +76,7 @@ __device__ __forceinline__ void stage_chunk(uint32_t acc_addr, bool have_acc, fl
   uint32_t pk[16];
 #pragma unroll
   for (int i = 0; i < 32; i += 2)
-    pk[i >> 1] = keep ? pack2<BF16>(__uint_as_float(v[i]) * mul, __uint_as_float(v[i + 1]) * mul) : 0u;
+    pk[i >> 1] = pack2<BF16>(__uint_as_float(v[i]) * mul, __uint_as_float(v[i + 1]) * mul);
   uint8_t* box = stage + (c >> 1) * kBoxBytes + r * 128;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {

@@ -802,6 +802,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     if (alive) {
       alive = wait_clocked(smem_u32(&sync->fixed_full), 0, abort_flag, wait_limit);
       if (!alive && lane == 0) report(p.status, 22, -1, 0);
+      // (as in the dQ kernel: the keys' own gradients would be 0 x NaN)
+      if (PAD && alive && n_keys < p.S && j0 + kT > n_keys) zero_tile_rows<C::kBoxes, kT>(v_tile, n_keys - j0, lane);
     }
     auto q_tile = [&](int it) { return ring + (it % C::kStages) * 2 * C::kTileBytes; };   // dO right behind it
     // S^T_i = K Q_i^T (waits for the query tile); the MMA pipe executes in issue order, so it may be issued right
@@ -989,8 +991,8 @@ bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       uint8_t* stage_k = smem_raw + (ring - raw_addr);
       uint8_t* stage_v = stage_k + C::kTileBytes;
       for (int c = part; c < D / 16; c += kParts) {
-        if (c < D / 32) stage_chunk<BF16>(tmem_base + lane_off + kColDK, n_items > 0, p.scale * (kScaled ? 1.f / (gs * kPScale) : 1.f), stage_k, r, c, !PAD || key_g < n_keys);
-        else stage_chunk<BF16>(tmem_base + lane_off + kColDV, n_items > 0, kScaled ? 1.f / kPScale : 1.f, stage_v, r, c - D / 32, !PAD || key_g < n_keys);
+        if (c < D / 32) stage_chunk<BF16>(tmem_base + lane_off + kColDK, n_items > 0, p.scale * (kScaled ? 1.f / (gs * kPScale) : 1.f), stage_k, r, c);
+        else stage_chunk<BF16>(tmem_base + lane_off + kColDV, n_items > 0, kScaled ? 1.f / kPScale : 1.f, stage_v, r, c - D / 32);
       }
       fence_proxy_async_smem();
       warp_arrive(&sync->staged, lane);

@@ -245,6 +245,7 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
     if (alive) {
       alive = wait_clocked(smem_u32(&sync->fixed_full), 0, abort_flag, wait_limit);
       if (!alive && lane == 0) report(p.status, 32, -1, 0);
+      if (WALK == kDK && alive && w.n_keys < p.S && w.row0 + kT > w.n_keys) zero_tile_rows<DV / 64, kT>(fv_tile, w.n_keys - w.row0, lane);
     }
     // k-step kk (16 elements of the head dimension) of a K-major streamed tile
     auto stream_step = [](int kk) { return static_cast<uint64_t>(((kk >> 2) * C::kStreamBox + (kk & 3) * 32) >> 4); };
@@ -466,7 +467,7 @@ __device__ __forceinline__ void walk(const CUtensorMap* tm_fe, const CUtensorMap
       // the fixed operands are no longer needed: their area stages the gradient
       const float mul = (WALK == kDV ? 1.f : p.scale) * (kScaled ? 1.f / ((WALK == kDV ? 1.f : gs) * kPScale) : 1.f);
       for (int c = quarter; c < C::kAccW / 32; c += 4)
-        stage_chunk<BF16>(acc_addr, w.n_tiles > 0, mul, smem_raw, r, c, WALK == kDQ || row_g < w.n_keys);
+        stage_chunk<BF16>(acc_addr, w.n_tiles > 0, mul, smem_raw, r, c);
       fence_proxy_async_smem();
       warp_arrive(&sync->staged, lane);
       if (tid == 0 && wait_clocked(smem_u32(&sync->staged), 0, abort_flag, wait_limit)) {

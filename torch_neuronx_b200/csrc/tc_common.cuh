@@ -198,8 +198,9 @@ inline bool strides_ok(const void* base, const int64_t* s, int rows, int heads, 
 // NaN: 0 x NaN is NaN.  The tile's copy has landed; the whole warp calls.
 template <int kBoxes, int kRows>
 __device__ __forceinline__ void zero_tile_rows(uint32_t tile, int row0, int lane) {
-#pragma unroll
+#pragma unroll 1
   for (int bx = 0; bx < kBoxes; ++bx)
+#pragma unroll 1
     for (int off = row0 * 128 + lane * 16; off < kRows * 128; off += 32 * 16)
       asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(tile + bx * (kRows * 128) + off), "r"(0) : "memory");
   fence_proxy_async_smem();
