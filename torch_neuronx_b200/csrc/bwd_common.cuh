@@ -34,9 +34,13 @@ __device__ __forceinline__ uint64_t mnmajor_step(int kk) { return static_cast<ui
 // between 4 and 8.  What is lost of dS then is 2^-22 of its value or 2^-40 of the bound, whichever is larger.
 constexpr float kPScale = 4096.f, kPScaleLog2 = 12.f;
 
-// Partial maxima of a (batch, kv head): one CTA of the prep kernel per 128 rows of dO and V, at most 128.
+// Partial maxima of a (batch, kv head): one CTA of the prep kernel for 1024 16-byte pieces of dO and V (four loads a
+// thread), for more where that gives more than about eight CTAs to an SM, and at most 128 parts.
 inline int range_parts(const Problem& p) {
-  const int64_t n = (static_cast<int64_t>(p.group) * p.L + p.S + 127) / 128;
+  const int64_t pieces = (static_cast<int64_t>(p.group) * p.L + p.S) * (p.Dv / 8), streams = static_cast<int64_t>(p.B) * p.Hkv;
+  int64_t n = (pieces + 1023) / 1024;
+  const int64_t most = (8 * 148 + streams - 1) / streams;
+  n = n > most ? most : n;
   return n < 1 ? 1 : (n > 128 ? 128 : static_cast<int>(n));
 }
 

@@ -86,36 +86,48 @@ static_assert(sizeof(BSync) <= 272, "barrier block must fit its reserve (272 byt
 // ------------------------------------------------------------------ prep --
 
 // (fp16) One part of the maxima that gradient_scale() combines, over dO and the visible rows of V, whose rows start on
-// 16 bytes: eight lanes a row.  Infinities and NaN are left out: what they reach is not finite at any scale.
+// 16 bytes.  Infinities and NaN are left out: what they reach is not finite at any scale.
 __device__ __forceinline__ void range_part(const BwdProblem& bp, float2* range, int n_parts, int unit) {
   const Problem& p = bp.f;
   __shared__ uint32_t sm[2][8];
   const int part = unit % n_parts, stream = unit / n_parts;
   const int hk = stream % p.Hkv, b = stream / p.Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  auto scan = [&](const __half* base, int64_t head_stride, int64_t row_stride, int rows, int n_rows) {   // of pairs of |x|
-    uint32_t top = 0;
-#pragma unroll 4
-    for (int r = part * 32 + static_cast<int>(threadIdx.x >> 3); r < n_rows; r += n_parts * 32) {
-      const __half* row = base + r / rows * head_stride + r % rows * row_stride;
-      for (int e = (lane & 7) * 8; e < p.Dv; e += 64) {
-        const uint4 x = *reinterpret_cast<const uint4*>(row + e);
-        for (const uint32_t w : {x.x, x.y, x.z, x.w}) {
-          const uint32_t a = w & 0x7fff7fffu;
-          top = __vmaxu2(top, a & __vcmpltu2(a, 0x7c007c00u));
-        }
+  const __half* go = reinterpret_cast<const __half*>(bp.dout) + b * bp.dos[0] + hk * p.group * bp.dos[1];
+  const __half* vb = reinterpret_cast<const __half*>(p.v) + b * p.vs[0] + hk * p.vs[1];
+  // 16-byte pieces of a row and in all (31 bits would end at 32 GB of dO in a kv head; 32 go beyond what a device holds)
+  const uint32_t pieces = p.Dv / 8, n_l = p.L, step = n_parts * 256;
+  const uint32_t go_pieces = p.group * n_l * pieces, all = go_pieces + valid_keys(p, b) * pieces;
+  uint32_t top_go = 0, top_v = 0;   // of pairs of |x|; finite halves order like their bits
+  for (uint32_t i0 = part * 256 + threadIdx.x; i0 < all; i0 += 4 * step) {
+    uint4 x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {   // four loads in flight
+      const uint32_t i = i0 + u * step;
+      x[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (i < go_pieces) {
+        const uint32_t row = i / pieces;
+        x[u] = *reinterpret_cast<const uint4*>(go + row / n_l * bp.dos[1] + row % n_l * bp.dos[2] + i % pieces * 8);
+      } else if (i < all) {
+        x[u] = *reinterpret_cast<const uint4*>(vb + (i - go_pieces) / pieces * p.vs[2] + (i - go_pieces) % pieces * 8);
       }
     }
-    return __vmaxu2(top, top >> 16) & 0xffffu;   // (finite halves order like their bits)
-  };
-  uint32_t go = scan(reinterpret_cast<const __half*>(bp.dout) + b * bp.dos[0] + hk * p.group * bp.dos[1], bp.dos[1], bp.dos[2], p.L,
-                     p.group * p.L);
-  uint32_t v = scan(reinterpret_cast<const __half*>(p.v) + b * p.vs[0] + hk * p.vs[1], 0, p.vs[2], p.S, valid_keys(p, b));
-  go = __reduce_max_sync(0xffffffffu, go);
-  v = __reduce_max_sync(0xffffffffu, v);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      uint32_t top = 0;
+      for (const uint32_t w : {x[u].x, x[u].y, x[u].z, x[u].w}) {
+        const uint32_t a = w & 0x7fff7fffu;
+        top = __vmaxu2(top, a & __vcmpltu2(a, 0x7c007c00u));
+      }
+      if (i0 + u * step < go_pieces) top_go = __vmaxu2(top_go, top);
+      else top_v = __vmaxu2(top_v, top);
+    }
+  }
+  top_go = __reduce_max_sync(0xffffffffu, __vmaxu2(top_go, top_go >> 16) & 0xffffu);
+  top_v = __reduce_max_sync(0xffffffffu, __vmaxu2(top_v, top_v >> 16) & 0xffffu);
   if (lane == 0) {
-    sm[0][warp] = go;
-    sm[1][warp] = v;
+    sm[0][warp] = top_go;
+    sm[1][warp] = top_v;
   }
   __syncthreads();
   if (threadIdx.x == 0 && dbg_range(p.status, DBG_BWD_TC * 100 + 11, unit, 1, static_cast<int64_t>(p.B) * p.Hkv * n_parts)) {
