@@ -68,8 +68,12 @@ typedef enum b200_sdpa_dtype {
 /* Which kernel family served (or must serve) a request. */
 typedef enum b200_sdpa_path {
   B200_SDPA_PATH_AUTO = 0,
-  B200_SDPA_PATH_GENERIC = 1,  /* CUDA-core fp32-accumulate flash kernel: any dtype,
-                                  any strides, additive bias, head dim <= 512        */
+  B200_SDPA_PATH_GENERIC = 1,  /* everything else: any dtype, any strides, additive
+                                  bias, head dim <= 512.  Where this is AUTO's choice,
+                                  tensor-core tiles serve the 16-bit head dimensions
+                                  72..128 (multiples of 8) and copied biases, tiled fp32
+                                  kernels the fp32 ones of 64 and 128, the CUDA-core
+                                  kernel the rest and every forced request             */
   B200_SDPA_PATH_PREFILL = 2,  /* TMA + tcgen05/TMEM warp-specialised kernels:
                                   f16/bf16, E == Dv in {64,128,256} or E = 192
                                   with Dv = 128, unit inner stride; also with an
@@ -127,7 +131,9 @@ typedef struct B200SdpaParams {
   const void* bias;       /* optional additive bias broadcastable to (B,Hq,L,S), or
                              NULL.  The tensor-core kernels read it when it has the
                              query's dtype, unit stride along the keys, S % 8 == 0 and
-                             16-byte aligned rows; any other bias runs the generic path */
+                             16-byte aligned rows; any other bias runs the generic
+                             path, on a copy in the workspace when it has the query's
+                             16-bit dtype and the workspace is given                   */
   int32_t bias_dtype;     /* b200_sdpa_dtype of bias                                   */
   int32_t kv_chunk;       /* decode: keys per split, 0 = library default               */
   int64_t bias_stride[4]; /* 0 for broadcast dimensions                                */
@@ -372,9 +378,11 @@ int b200_sdpa_decode_static(const B200SdpaParams* params, void* stream);
  * Kernel family, launch geometry (grid_x: grad_q kernel, grid_y: grad_k/grad_v kernel)
  * and scratch size of a backward request, without launching.  Host-only.
  * `path` is B200_SDPA_PATH_PREFILL for the tcgen05 kernels (f16/bf16, E == Dv in
- * {64,128}, no grad_bias, a bias only under the forward's rules for that path, unit
- * inner strides, 16-byte aligned bases and outer strides of q, k, v, grad_out and the
- * three gradients) and B200_SDPA_PATH_GENERIC otherwise.
+ * {64,128,256} or E = 192 with Dv = 128, no grad_bias, a bias at 64 and 128 only and under
+ * the forward's rules for that path, unit inner strides, 16-byte aligned bases and outer
+ * strides of q, k, v, grad_out and the three gradients) and B200_SDPA_PATH_GENERIC
+ * otherwise, also where tcgen05 kernels serve the head dimensions 72..128 and tiled fp32
+ * kernels those of 64 and 128.
  */
 int b200_sdpa_bwd_query_plan(const B200SdpaBwdParams* params, B200SdpaPlan* plan);
 

@@ -1173,8 +1173,9 @@ int plan_bwd_tc(const BwdProblem& bp, int dtype, B200SdpaPlan* plan) {
   plan->grid_x = static_cast<int32_t>(static_cast<long long>((p.L + kT - 1) / kT) * p.Hq * p.B);
   plan->grid_y = static_cast<int32_t>(static_cast<long long>((p.S + kT - 1) / kT) * p.Hkv * p.B);
   plan->grid_z = 1;
-  plan->threads = bwd_wide_dims(p) ? 576 : kThreads;
+  plan->threads = kThreads;
   plan->smem_bytes = p.E == 64 && p.Dv == 64 ? BCfg<64>::kSmemBytes : BCfg<128>::kSmemBytes;
+  if (bwd_wide_dims(p)) plan_bwd_wide(p, plan);
   plan->kv_splits = 1;
   plan->launches = 3;
   plan->workspace_bytes = bwd_tc_workspace_bytes(bp, dtype);

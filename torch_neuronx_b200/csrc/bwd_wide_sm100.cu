@@ -642,6 +642,12 @@ bool bwd_wide_dims(const Problem& p) {
   return ((p.E == 192 && p.Dv == 128) || (p.E == 256 && p.Dv == 256)) && p.bias == nullptr;
 }
 
+void plan_bwd_wide(const Problem& p, B200SdpaPlan* plan) {
+  plan->threads = kThreads;
+  plan->grid_y *= 2;   // dK and dV are CTAs of their own
+  plan->smem_bytes = p.E == 192 ? WCfg<kDQ, 192, 128>::kSmemBytes : WCfg<kDQ, 256, 256>::kSmemBytes;
+}
+
 int launch_bwd_wide(const BwdProblem& bp, bool bf16, float* lse2, float* delta, float2* range, cudaStream_t stream) {
   if (bp.f.E == 192)
     return bf16 ? launch_wide<192, 128, true>(bp, lse2, delta, range, stream) : launch_wide<192, 128, false>(bp, lse2, delta, range, stream);

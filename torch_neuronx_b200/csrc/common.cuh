@@ -135,6 +135,7 @@ int plan_bwd_generic(const BwdProblem& bp, int dtype, B200SdpaPlan* plan);
 bool bwd_tc_eligible(const BwdProblem& bp, int dtype, bool* alignment_only_failure);
 // head dimensions 192/128 and 256 (bwd_wide_sm100.cu)
 bool bwd_wide_dims(const Problem& p);
+void plan_bwd_wide(const Problem& p, B200SdpaPlan* plan);   // what differs from the kernels up to 128
 int launch_bwd_wide(const BwdProblem& bp, bool bf16, float* lse2, float* delta, float2* range, cudaStream_t stream);
 bool bwd_padded_eligible(const BwdProblem& bp, int dtype);
 uint64_t bwd_tc_workspace_bytes(const BwdProblem& bp, int dtype);
