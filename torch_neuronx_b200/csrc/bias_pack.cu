@@ -12,7 +12,7 @@ namespace {
 
 constexpr uint64_t kMaxPackedBytes = 4ull << 30;   // more than this stays where it is
 
-// One CTA per row and 2048 columns; a thread writes four pairs of neighbouring columns, a warp 128 bytes at a time.
+// One CTA per row, 2048 columns at a time; a thread writes four pairs of neighbouring columns, a warp 128 bytes at a time.
 __global__ void __launch_bounds__(256) bias_pack_kernel(const uint16_t* src, uint16_t* dst, const int S, const int sp, const int n_rows,
                                                         const int n_heads, const int64_t s0, const int64_t s1, const int64_t s2,
                                                         const int64_t s3, const uint32_t hidden) {

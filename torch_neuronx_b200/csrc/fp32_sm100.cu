@@ -333,9 +333,11 @@ __global__ void __launch_bounds__(kThreads) fp32_bwd_dq_kernel(const BwdProblem 
     for (int i = 0; i < R; ++i) {
       const int row = row0 + f0 + i;
       float d = 0.f;
-      lse[i] = -CUDART_INF_F;
+      lse[i] = CUDART_INF_F;
       if (row < p.L) {
-        lse[i] = p.lse[b * p.ls[0] + h * p.ls[1] + row * p.ls[2]];
+        const float l = p.lse[b * p.ls[0] + h * p.ls[1] + row * p.ls[2]];
+        // -inf: no key seen, or nothing but NaN.  With +inf finite scores give 0 and NaN stays NaN, as it is in delta
+        lse[i] = l == -CUDART_INF_F ? CUDART_INF_F : l;
 #pragma unroll
         for (int c = 0; c < D / (4 * TX); ++c) {
           const float4 x = *reinterpret_cast<const float4*>(go + row * bp.dos[2] + c * 4 * TX + tx * 4);
@@ -367,10 +369,9 @@ __global__ void __launch_bounds__(kThreads) fp32_bwd_dq_kernel(const BwdProblem 
     for (int i = 0; i < R; ++i) {
       const int64_t lim64 = p.causal ? static_cast<int64_t>(row0 + f0 + i) + p.causal_shift + 1 : n_keys;
       const int lim = lim64 < n_keys ? static_cast<int>(lim64 < 0 ? 0 : lim64) : n_keys;
-      const bool dead = lse[i] == -CUDART_INF_F;   // no key seen, or nothing but NaN: then delta is NaN and so is dS
 #pragma unroll
       for (int j = 0; j < J; ++j)
-        s[i][j] = j0 + tx + TX * j < lim ? (dead ? 0.f : expf(s[i][j] * p.scale - lse[i])) * (dp[i][j] - delta[i]) : 0.f;
+        s[i][j] = j0 + tx + TX * j < lim ? expf(s[i][j] * p.scale - lse[i]) * (dp[i][j] - delta[i]) : 0.f;
     }
     store_transposed<TX, J>(Op, f0, tx, s);
     __syncthreads();   // the operand is here; V has been read
