@@ -87,7 +87,7 @@ template <int D> struct Cfg {
   // the softmax loop) shrinks from 60 KB to 28 KB and every spill turns into an L2 round trip.  That is
   // why there is no slack for rounding the tile area up to 1024 bytes: the dynamic shared memory is
   // declared with that alignment and the kernel checks it.
-  static constexpr int kSmemBytes = kSmemTiles + kStatBytes + 640 /*barriers, items*/;
+  static constexpr int kSmemBytes = kSmemTiles + kStatBytes + 896 /*barriers, items, tile lists*/;
   static_assert(kSmemBytes + 1024 <= 196 * 1024, "must fit the 196 KB shared-memory configuration");
   // With D = 64 the two O accumulators leave 128 tensor-memory columns free: P_t gets columns of its
   // own ([384,448) / [448,512)) instead of overwriting S_t, so Q_t K(j+1)^T no longer has to wait for
@@ -134,9 +134,10 @@ struct Sync {
   uint32_t tmem_base;
   int abort_flag;
   ItemRec item[kItemSlots];
+  uint8_t list[kItemSlots][64];     // (bias) the item's key tiles in order, where it.tiles names them
 };
 
-static_assert(sizeof(Sync) <= 640, "barrier block must fit its reserve");
+static_assert(sizeof(Sync) <= 896, "barrier block must fit its reserve");
 
 template <int N> __device__ __forceinline__ void setmaxnreg_inc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
@@ -229,6 +230,12 @@ __device__ __forceinline__ ItemRec decode_item(const Problem& p, int idx, int n_
   return it;
 }
 
+__device__ __forceinline__ int ld_shared_u8(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return static_cast<int>(v);
+}
+
 // The key tile after `j`: the lowest bit of `rest`, which it loses, or j + 1 where there is no list.
 template <bool BIAS>
 __device__ __forceinline__ int next_tile(int j, uint64_t& rest) {
@@ -314,14 +321,15 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   int q_loads[2] = {0, 0};       // Q_t copies issued so far
 
   // every consumer role reads the next item from the scheduler's ring
-  auto next_item_rec = [&](int k, bool* ok) -> ItemRec {
+  auto release_item = [&](int k) { mbar_arrive(smem_u32(&sync->item_empty[k % kItemSlots])); };
+  auto next_item_rec = [&](int k, bool* ok, bool hold = false) -> ItemRec {
     const int slot = k % kItemSlots;
     ItemRec rec;
     rec.idx = -1;
     *ok = wait_clocked(smem_u32(&sync->item_full[slot]), (k / kItemSlots) & 1, abort_flag, wait_limit);
     if (!*ok) return rec;
     rec = sync->item[slot];
-    mbar_arrive(smem_u32(&sync->item_empty[slot]));
+    if (!hold) release_item(k);
     return rec;
   };
 
@@ -356,6 +364,10 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           it.idx = -1;
           if (idx >= 0) it = decode_item(p, idx, n_qblk, pair_heads, streams_per_wave, BIAS ? lists : TileLists{});
           sync->item[slot] = it;
+          if constexpr (BIAS) {
+            uint8_t* list = sync->list[slot];
+            for (uint64_t rest = it.tiles; rest != 0; rest &= rest - 1) *list++ = static_cast<uint8_t>(__ffsll(static_cast<long long>(rest)) - 1);
+          }
           mbar_arrive(smem_u32(&sync->item_full[slot]));
           if (idx < 0) break;
           const int n_iter = it.nt0 > it.nt1 ? it.nt0 : it.nt1;
@@ -711,14 +723,17 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     int n_done = 0;     // items (with keys) of this tile finished so far
 
     for (int k = 0; alive; ++k) {
-      const ItemRec it = next_item_rec(k, &alive);
+      const ItemRec it = next_item_rec(k, &alive, BIAS);   // (with a bias the slot is kept until its tile list has been read)
       if (!alive) {
         if (lane == 0) report(p.status, 4 + t, -3, k);
         break;
       }
       if (it.idx < 0) break;
       const int n_tiles = t == 0 ? it.nt0 : it.nt1;
-      if (n_tiles == 0) continue;
+      if (n_tiles == 0) {
+        if (BIAS) release_item(k);
+        continue;
+      }
       const int min_lim = t == 0 ? it.lim0 : it.lim1;
       const int head = t == 0 ? it.head0 : it.head1;
       const int b = it.b;
@@ -747,10 +762,9 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
                                                     static_cast<long long>(row_g) * p.bs[2]);
       }
 
-      uint64_t rest = it.tiles;
-      int key_tile = -1;
+      const uint8_t* list = BIAS && it.tiles != 0 ? sync->list[k % kItemSlots] : nullptr;
       for (int j = 0; j < n_tiles; ++j) {
-        key_tile = next_tile<BIAS>(key_tile, rest);
+        const int key_tile = BIAS && list != nullptr ? list[j] : j;
         uint4 bv[BIAS ? kBlockN / 8 : 1];
         if constexpr (BIAS) {
           // the bias of this key tile travels while the scores are awaited
@@ -921,6 +935,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         mbar_arrive(smem_u32(&sync->p_ready[t][1]));
         ++n_s;
       }
+      if (BIAS) release_item(k);
     }
   }
 
@@ -1043,9 +1058,18 @@ __global__ void __launch_bounds__(kListThreads) bias_tiles_kernel(const Problem 
   }
 }
 
-// Where the bias is looked over first: up to the 64 key tiles that a word holds, and where a CTA has at least eight
-// tile steps (2 us each) in front of it, against the launch's 5-8 (1 x 8 x 512, four steps: 23.4 us without, 31.7 with;
-// 4 x 12 x 1024, head dimension 64, a causal bias, 16 steps: 69.6 / 50.2; 2 x 32/8 x 2048 with a window of 512, 64 steps: 259 / 120).
+// Where the bias is looked over first: up to the 64 key tiles that a word holds, and where a CTA has at least sixteen
+// tile steps in front of it.  What a bias hides is not known to the host, so both kinds count; device time in us, this
+// form with the look-over against the per-CTA kernel without, for a bias that hides nothing, all above the diagonal, or
+// all but a quarter below it:
+//   head dimension 128   1 x 8 x 1024 (8 steps)     36 / 31     37 / 31     26 / 31
+//                        4 x 12 x 1024 (16)         64 / 62     42 / 62     39 / 62
+//                        2 x 32/8 x 2048 (64)      207 / 223   130 / 223    91 / 223    (203 here without the look-over)
+//   head dimension 64    1 x 8 x 1024               36 / 30     37 / 30     25 / 30
+//                        4 x 12 x 1024              66 / 60     42 / 60     37 / 60
+//                        2 x 32/8 x 2048           219 / 211   131 / 210    89 / 210
+//                        1 x 16 x 4096 (64)        223 / 204   132 / 204    95 / 204
+// So a dense bias loses 2 to 4 % at 128 and 4 to 10 % at 64 where half a bias of -inf gains 30 to 40 %.
 // Counter and words share the scratch.
 struct ListGeom {
   int n_batches, n_heads, n_row_tiles;
@@ -1057,7 +1081,7 @@ ListGeom list_geometry(const Problem& p) {
   if (p.bias == nullptr || n_tiles > 64) return g;
   const char* mode = getenv("B200_SDPA_PREFILL");
   const bool forced = mode != nullptr && strncmp(mode, "pers", 4) == 0;
-  if (!forced && (prefill_geometry(p).n_items + kAssumedSms - 1) / kAssumedSms * n_tiles < 8) return g;
+  if (!forced && (prefill_geometry(p).n_items + kAssumedSms - 1) / kAssumedSms * n_tiles < 16) return g;
   if (p.bs[0] != 0) g.n_batches = p.B;
   if (p.bs[1] != 0) g.n_heads = p.Hq;
   if (p.bs[2] != 0) g.n_row_tiles = (p.L + kBlockM - 1) / kBlockM;
@@ -1137,8 +1161,8 @@ bool prefill_accumulate_eligible(const Problem& p) {
 // tiles per item, or more than one item per SM and at most 8 key tiles (2 x 32/8 x 1024 causal, 256 items: 37.8 us
 // per CTA, 36.8 here; 8 x 32 x 256, 256 items: 33.7 / 29.6; at 64 key tiles 146.4 / 148.6).  Padded head dimensions
 // follow the same rule (fp16 16 x 16 x 577, head dimension 80: 92.2 / 80.0).  At head dimension 64 the exponentials
-// bound the loop and this form measured up to 15 % slower; it serves those shapes only with a bias whose hidden key
-// tiles it can leave out.  B200_SDPA_PREFILL = "persistent" or "per_cta" overrides the
+// bound the loop and this form measured up to 15 % slower; it serves those shapes only with a bias that is looked over
+// for hidden key tiles (list_geometry has the figures).  B200_SDPA_PREFILL = "persistent" or "per_cta" overrides the
 // choice where both kernels can serve the request (for tests and measurements).
 bool prefill_persistent_wanted(const Problem& p) {
   const int hi = p.E > p.Dv ? p.E : p.Dv;
