@@ -1003,7 +1003,7 @@ PrefillGeom prefill_geometry(const Problem& p) {
 // With few items to a CTA the order hardly matters and the counter does: the memset that clears it is an operation of its
 // own in the stream and keeps the launch from being a programmatic dependent of the kernel before.  Measured (fixed
 // order / counter, us, head dimension 128 unless said): 2 x 32/8 x 1024 causal, 256 items, 36.8 / 39.0; 8 x 16 x 577, 384 items,
-// 50.0 / 51.2; but 16 x 16 x 577 at head dimension 80, 768 items, 84.9 / 80.0 and 4 x 32/8 x 4096, 2048 items, 609 / 496.
+// 50.0 / 51.2; but 4 x 32/8 x 4096, 2048 items, 609 / 496.
 bool items_in_fixed_order(const PrefillGeom& g) { return g.n_items < 3LL * kAssumedSms; }
 
 // One CTA per 128 bias rows: which of its key tiles (at most 64) hold an element other than -inf.  The warps share the
@@ -1160,7 +1160,7 @@ bool prefill_accumulate_eligible(const Problem& p) {
 // over 131072) the per-CTA kernel is 5 % faster either way.  So: at least three items per SM and at most 64 key
 // tiles per item, or more than one item per SM and at most 8 key tiles (2 x 32/8 x 1024 causal, 256 items: 37.8 us
 // per CTA, 36.8 here; 8 x 32 x 256, 256 items: 33.7 / 29.6; at 64 key tiles 146.4 / 148.6).  Padded head dimensions
-// follow the same rule (fp16 16 x 16 x 577, head dimension 80: 92.2 / 80.0).  At head dimension 64 the exponentials
+// follow the same rule (fp16 16 x 16 x 577, head dimension 80: 92 us per CTA, 90 here).  At head dimension 64 the exponentials
 // bound the loop and this form measured up to 15 % slower; it serves those shapes only with a bias that is looked over
 // for hidden key tiles (list_geometry has the figures).  B200_SDPA_PREFILL = "persistent" or "per_cta" overrides the
 // choice where both kernels can serve the request (for tests and measurements).
